@@ -150,15 +150,13 @@ int nspt_twist_boundary(nspt_ctx *ctx);
  * NSPT_UPDATE_ONTHEFLY, whose rectangles reach two sites), else
  * NSPT_ERR_ARG. */
 int nspt_set_gf_grid(nspt_ctx *ctx, const int grid[4]);
-/* Which kernels run the work ordered by the thread grid -- the local gauge
- * fixing and the on-the-fly sweep; both forms visit the sites in the grid's
- * order and give the same links.  NSPT_LGF_GROUP: one 9-lane link group per
- * reference thread.  NSPT_LGF_TEAM: a warp of three groups per thread (the
- * gauge fixing's stagings and link products, or the sweep's three planes of
- * staples, spread over them: shorter latency for grids with few threads;
- * the on-the-fly team form needs one site per thread and barrier step).
- * NSPT_LGF_AUTO (the default): the team form when all the barrier step's
- * teams fit on the GPU at once.  Anything else: NSPT_ERR_ARG. */
+/* Which form of the kernels runs the work ordered by the thread grid -- the
+ * local gauge fixing and the on-the-fly sweep; both visit the sites in the
+ * grid's order and give the same links to rounding.  NSPT_LGF_GROUP: 9 lanes
+ * per reference thread (orders below 18; above, as TEAM).  NSPT_LGF_TEAM: a
+ * warp per thread, a third of the instructions in a row: shorter latency for
+ * grids with few threads.  NSPT_LGF_AUTO (the default): by the number of
+ * threads and the order.  Anything else: NSPT_ERR_ARG. */
 #define NSPT_LGF_AUTO 0
 #define NSPT_LGF_GROUP 1
 #define NSPT_LGF_TEAM 2
@@ -270,14 +268,14 @@ int nspt_batch_step(nspt_batch *b, int nsteps, int gf_every);
 double nspt_batch_last_step_ms(const nspt_batch *b);
 /* Plaquette series of every replica's last sweep: plaq[nrep][(N+1)*2]. */
 int nspt_batch_observables(nspt_batch *b, double *plaq);
-/* Autotuner over the tile shape of the series kernels: orders per lane and
- * pass (8, or 4 where N <= 12; in the paired-run product the run length is
- * half of it) and the sweep's warps per CTA (3 links each).  Every candidate
- * is timed on the batch step itself and the fastest kept: *warps_out,
- * *mo_out (orders per lane and pass); ms_table (may be NULL) gets [2][8]
- * times, row 0 for 8 orders per lane, row 1 for 4, column w-1 for w warps,
- * 0 where a candidate does not exist.  The trial steps are undone (every
- * replica back to a cold start with its seed).  Call before stepping. */
+/* Autotuner over the launch shape of the series kernels: warps per CTA (1 to
+ * 4, or as many as shared memory holds; more run as 4).  Every candidate is
+ * timed on the batch step itself and the fastest kept: *warps_out, *mo_out;
+ * ms_table (may be NULL) gets [2][8] times, column w-1 for w warps, 0 where a
+ * candidate does not exist.  The two rows (*mo_out 8, or 4 where N <= 12) are
+ * two timings of the same kernels, which accumulate 8 orders per lane whatever
+ * the row.  The trial steps are undone (every replica back to a cold start with
+ * its seed).  Call before stepping. */
 int nspt_batch_tune_shape(nspt_batch *b, int gf_every, int *warps_out, int *mo_out,
                           float *ms_table);
 /* nspt_batch_tune_shape reporting the warps only. */

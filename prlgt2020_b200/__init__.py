@@ -286,10 +286,10 @@ class NsptEngine:
         self._check(load_library().nspt_set_gf_grid(self._h, g), "nspt_set_gf_grid")
 
     def set_local_gf_form(self, form: str):
-        """Kernel of the local gauge fixing: "group" (one 9-lane link group
-        per reference thread), "team" (a warp of three groups per thread) or
-        "auto" (the team form when the barrier step's teams all fit on the
-        GPU at once).  Both forms give the same links."""
+        """Form of the kernels that follow the thread grid: "group" (9 lanes
+        per reference thread), "team" (a warp per thread) or "auto" (by the
+        number of threads and the order).  Both give the same links to
+        rounding."""
         code = {"auto": 0, "group": 1, "team": 2}.get(form)
         if code is None:
             raise ValueError(f"local gauge fixing form {form!r}: auto, group or team")
@@ -428,8 +428,9 @@ class NsptBatch:
         return w.value
 
     def tune_shape(self, gf_every: int = 1):
-        """Autotune the tile shape: (warps per CTA, orders per lane and pass,
-        table of step times in ms [orders 8 / 4][warps 1..8], 0 = not tried)."""
+        """Autotune the launch shape: (warps per CTA, 8 or 4, table of step
+        times in ms [rows 8 / 4][warps 1..8], 0 = not tried); the rows are two
+        timings of the same kernels."""
         w, mo = ctypes.c_int(), ctypes.c_int()
         table = (ctypes.c_float * 16)()
         check(load_library().nspt_batch_tune_shape(self._h, int(gf_every), ctypes.byref(w),

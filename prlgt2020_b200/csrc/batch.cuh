@@ -218,10 +218,9 @@ extern "C" int nspt_batch_observables(nspt_batch *b, double *plaq) {
   return NSPT_OK;
 }
 
-// Autotuner over the tile shape of the series kernels: orders per lane and
-// pass (MO, or MO_LOW where N <= 3 MO_LOW; in the paired-run product this
-// is the run length, MO/2) and, for the sweep, warps per CTA (3 links per
-// warp: the links, i.e. sites x directions, per block).  Every candidate is
+// Autotuner over the tile shape of the series kernels: orders a lane
+// accumulates per pass (MO: the block chosen by N, or MO_LOW where N <= 3
+// MO_LOW) and warps per CTA (one link per warp).  Every candidate is
 // captured and timed on the batch itself; the fastest is kept.  The trial
 // steps change the fields, so every replica is put back to a cold start
 // with its seed (counter 0) afterwards.  ms_table (may be NULL) receives
@@ -238,7 +237,7 @@ extern "C" int nspt_batch_tune_shape(nspt_batch *b, int gf_every, int *warps_out
   for (int row = 0; row < 2; row++) {
     const int mo = row == 0 ? MO : MO_LOW;
     if (mo == MO_LOW && b->N > 3 * MO_LOW) continue;
-    const int wmax = (mo == MO ? SWEEP_THREADS : SWEEP_THREADS_LOW) / 32;
+    const int wmax = mo == MO ? 8 : 6;
     for (int w = 1; w <= wmax; w++) {
       for (nspt_ctx *c : b->ctx) {
         c->sweep_warps = w;

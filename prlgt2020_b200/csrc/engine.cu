@@ -14,7 +14,10 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
+#include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/nspt_b200.h"
@@ -23,11 +26,6 @@
 #include "loops.cuh"
 
 using namespace nspt;
-
-struct KernelShape {
-  int warps;  // warps per CTA (3 link groups of 9 lanes each)
-  int slots;  // shared series slots per group
-};
 
 struct nspt_ctx {
   int L[4];
@@ -47,29 +45,31 @@ struct nspt_ctx {
   double last_kernel_ms;  // average sweep-kernel launch of the last call
   Geo geo;
   int SS;  // slot stride (double2)
-  double2 *U, *Uf, *F, *Ff;
+  double2 *U, *F;    // link records (kernels.cuh)
+  bool unit_flags;   // every link's flag is 1 (false after an upload that says otherwise)
+  double2 *plaq[2];  // plaquette records of two slabs of the Jacobi sweep
+  int slab;          // planes of direction 0 per slab
   double2 *Lg;       // per-link logs (zero modes, FA)
   bool snap_valid;   // on the fly, twisted: F holds the step's start field, which reads
                      // across a twisted face see until twist_boundary
   bool lg_current;   // Lg holds log U of the current field (after a sweep with
                      // zero modes and after the zero-mode subtraction)
-  double2 *Wg, *Gx;  // FA work planes
-  double2 *obs_tr, *obs_tru;
-  double *obs_norm;
-  double2 *red2;  // [(N+1) + 4N + 4*9N] reduced sums
-  double *red1;   // [N]
+  double2 *Wg, *Gx;  // FA work planes, gauge transformation records
+  double *obs, *obs_tr;  // SweepArgs
+  // column sums: obs [12N], obs_tr [<= 8(N+1)], obs_tr2 [8(N+1)], Lg [8(1+9N)]
+  double *red;
+  double *red_part;  // [COLSUM_CHUNKS][widest row]
+  int tr_rows;       // rows of the last sweep's traces per site: 6 (plaquettes) or 4 (links)
+  double2 *meas;     // plaquette_measure: per-CTA rows
   double *p2;     // lattice momenta p2hat[4][128] of this context's extents
   double2 *ftw;   // FFT twiddles exp(-2 pi i t / L_d), [4][128] (FA only)
   int gf_grid[4]; // local gauge fixing: the reference's thread grid (ntt, ntx, nty, ntz)
-  int gf_form;    // local gauge fixing kernel: NSPT_LGF_AUTO, NSPT_LGF_GROUP or NSPT_LGF_TEAM
+  int gf_form;    // form of the grid-ordered kernels: NSPT_LGF_AUTO, _GROUP or _TEAM
   unsigned long long *dcounter;  // Philox step counter on the device (advanced by k_inc)
   int sweep_warps;               // warps per CTA of the sweep, 0 = as many as fit
-  // orders per lane and pass of the series kernels: 0 = by N (the low-order
-  // shape, MO_LOW, for N <= 3 MO_LOW), MO = the 24-order shape everywhere,
-  // MO_LOW = the low-order shape (only where N <= 3 MO_LOW)
-  int shape_mo;
+  int shape_mo;                  // the tuner's row: see nspt_batch_tune_shape
   double c1;                     // improved action weight (0: Wilson), c0 = 1 - 8 c1
-  double2 *obs_tr2;              // [(N+1)][4V] rectangle traces (improved actions)
+  double *obs_tr2;               // rectangle traces (improved actions)
   int *ff_e;                     // float-float scale exponent used by the sweep (device)
   unsigned long long *ff_mx;     // [N] per-order max |U_k| (bit patterns)
   bool ff_auto;                  // fit the exponent each sweep
@@ -120,115 +120,97 @@ extern "C" const char *nspt_last_error(nspt_ctx *ctx) {
 
 // ---------------- kernel shapes ----------------
 
-// per-group shared memory: `slots` series slots plus `extra` double2
-static size_t group_bytes(const nspt_ctx *ctx, int slots, int extra) {
-  return ((size_t)slots * ctx->SS + extra) * sizeof(double2);
+// CTAs (partial rows) of plaquette_measure
+constexpr int MEASURE_CTAS = 592;
+// sites per slab of the Jacobi sweep at least: 24 k plaquettes, ten rounds of
+// the 2368 warps that the GPU holds
+constexpr long SLAB_SITES = 4096;
+
+constexpr int MO = 8, MO_LOW = 4;
+
+// Lanes of a link's group (wseries.cuh) in a launch of `units` groups: 9 where
+// the SMs then have enough warps, 32 where they have not -- because shared
+// memory holds few links (sweep of 16 x 16 x 16 x 8, ms with 9 / 32 lanes: 2.2 /
+// 2.9 at 8 orders, 5.3 / 5.6 at 14, 6.7 / 6.1 at 16, 13.7 / 11.2 at 24) or
+// because the launch is small (1296 links of an on-the-fly step of 12^4 x 8: 5.1
+// / 4.0 ms per sweep; 1024 links of 4^4: 67 / 51 us).
+static int form_lanes(const nspt_ctx *ctx, long units) {
+  return ctx->N > 14 || units < 24L * ctx->nsm ? 32 : 9;
+}
+// Runs with logarithms (zero modes, Fourier-accelerated gauge fixing) at high
+// order keep the order of every sum (wseries.cuh, ORDERED).  The difference of
+// two orders of summation is 1e-10 of the field's largest entries after 40 steps
+// at 13 orders and 4e-7 after 20 steps at 20.
+static bool ordered(const nspt_ctx *ctx) {
+  return ctx->N > 14 && (ctx->flags & (NSPT_ZEROMODE | NSPT_GF_FA));
+}
+// Run fn with the form as a constant: for what enters the field, and for
+// measurements, which have no order to keep.
+template <class Fn>
+static void measure_form(const nspt_ctx *ctx, long units, Fn fn) {
+  if (form_lanes(ctx, units) == 9)
+    fn(std::integral_constant<int, 9>());
+  else
+    fn(std::integral_constant<int, 32>());
+}
+template <class Fn>
+static void with_form(const nspt_ctx *ctx, long units, Fn fn) {
+  if (ordered(ctx))
+    fn(std::integral_constant<int, ORDERED>());
+  else
+    measure_form(ctx, units, fn);
+}
+// The kernels that follow the thread grid: as set by nspt_set_local_gf_form
+// (9 lanes serve orders below 18, see ser_exp).
+template <class Fn>
+static void with_grid_form(const nspt_ctx *ctx, long units, Fn fn) {
+  if (ordered(ctx) || ctx->gf_form == NSPT_LGF_AUTO)
+    with_form(ctx, units, fn);
+  else if (ctx->gf_form == NSPT_LGF_GROUP && ctx->N < 9 * EXP_LANE)
+    fn(std::integral_constant<int, 9>());
+  else
+    fn(std::integral_constant<int, 32>());
 }
 
-// the low-order kernel shape (MO_LOW orders per lane and pass, 6-warp CTAs,
-// two per SM) for this context's series kernels
-static bool use_low(const nspt_ctx *ctx) {
-  if (ctx->N > 3 * MO_LOW) return false;
-  return ctx->shape_mo != MO;
-}
-
-static KernelShape choose_shape(const nspt_ctx *ctx, int slots, long units, int extra = 0,
-                                int max_warps = 8, int ctas_per_sm = 1) {
-  KernelShape k;
-  k.slots = slots;
-  const size_t per_warp = (size_t)LPW * group_bytes(ctx, slots, extra);
-  // shared memory per SM: 228 KB, of which up to smem_optin for one CTA
-  const size_t budget = ctas_per_sm > 1 ? (size_t)228 * 1024 / ctas_per_sm - 1024 : ctx->smem_optin;
-  int wmax = (int)std::min<size_t>(max_warps, std::min(budget, ctx->smem_optin) / per_warp);
-  if (wmax < 1) wmax = 1;
-  // spread small lattices over the SMs: about two CTAs per SM if possible
-  const long want = (units + (long)LPW * 2 * ctx->nsm - 1) / ((long)LPW * 2 * ctx->nsm);
-  k.warps = (int)std::max<long>(1, std::min<long>(wmax, want));
+// Groups per CTA: as many as give an SM the most groups, with 228 KB of shared
+// memory per SM, 1 KB of it taken by each CTA, at most ctas_max CTAs per SM
+// (registers) of CTA_WARPS warps of 32 / lanes groups; among equals the
+// larger CTA.  cap: warps per CTA at most.  gpc 0 when not even one group fits.
+struct Shape {
+  int warps, gpc;
+  size_t smem;
+};
+static Shape group_shape(int lanes, int ctas_max, int slots, int SS, size_t smem_optin, int cap = CTA_WARPS) {
+  const size_t lead = LEAD * sizeof(double2);
+  const size_t per = group_stride(slots, SS) * sizeof(double2);
+  cap = std::min(cap, CTA_WARPS);
+  Shape k = {0, 0, 0};
+  long most = 0;
+  for (int ctas = 1; ctas <= ctas_max; ctas++) {
+    const size_t room = std::min<size_t>(smem_optin, (size_t)228 * 1024 / ctas - 1024);
+    const long g = std::min<long>(32L / lanes * cap, room > lead ? (long)((room - lead) / per) : 0);
+    if (g * ctas > most) most = g * ctas, k.gpc = (int)g;
+  }
+  k.warps = std::min(cap, k.gpc);
+  k.smem = lead + k.gpc * per;
   return k;
 }
 
-template <bool MEASURE, bool FF, bool LOW = false>
-static void sweep_kernel(dim3 grid, dim3 blk, size_t smem, cudaStream_t st, const SweepArgs &a) {
-  cudaFuncSetAttribute(k_sweep<MEASURE, FF, LOW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
-  k_sweep<MEASURE, FF, LOW><<<grid, blk, smem, st>>>(a);
-}
-
-static int launch_sweep(nspt_ctx *ctx, const SweepArgs &a0, bool measure) {
-  const long nl = 4 * ctx->V;
-  const bool ff = (ctx->flags & NSPT_PRECISION_FF) != 0;
-  // low orders: the lighter variant, two CTAs per SM
-  const bool low = !measure && !ff && use_low(ctx);
-  const int max_warps = (low ? SWEEP_THREADS_LOW : SWEEP_THREADS) / 32;
-  KernelShape k = choose_shape(ctx, SWEEP_SLOTS, nl, 0,
-                               ctx->sweep_warps > 0 ? std::min(ctx->sweep_warps, max_warps)
-                                                    : max_warps,
-                               low ? 2 : 1);
-  int warps = k.warps, gpc = k.warps * LPW;
-  if (!low && ctx->sweep_warps == 0 && k.warps < max_warps) {
-    // shared memory, not the lattice, limits the CTA: as many link groups
-    // as it holds, over all max_warps warps (sweep_group), where that keeps
-    // at least 2.5 groups per warp.  Measured at 32^4 x 24: 22 groups as 8
-    // warps 511 ms, 21 as 7 full warps 538 ms; at 24^4 x 40, 13 groups as 8
-    // warps 732 ms, 12 as 4 full warps 671 ms.
-    const size_t per_group = group_bytes(ctx, SWEEP_SLOTS, 0);
-    const long fit = std::min<long>((long)(ctx->smem_optin / per_group), (long)max_warps * LPW);
-    const long want = (nl + 2L * ctx->nsm - 1) / (2L * ctx->nsm);  // about two CTAs per SM
-    if (fit > gpc && want >= fit && 2 * fit >= 5L * max_warps) {
-      gpc = (int)fit;
-      warps = max_warps;
-    }
-  }
-  SweepArgs a = a0;
-  a.gpc = gpc;
-  const size_t smem = (size_t)gpc * group_bytes(ctx, SWEEP_SLOTS, 0);
-  const unsigned grid = (unsigned)((nl + gpc - 1) / gpc);
-  const dim3 blk(32 * warps);
-  if (measure)
-    sweep_kernel<true, false>(grid, blk, smem, ctx->st, a);
-  else if (ff)
-    sweep_kernel<false, true>(grid, blk, smem, ctx->st, a);
-  else if (low)
-    sweep_kernel<false, false, true>(grid, blk, smem, ctx->st, a);
-  else
-    sweep_kernel<false, false>(grid, blk, smem, ctx->st, a);
-  CK(cudaGetLastError());
-  return NSPT_OK;
-}
-
-static int launch_sweep_imp(nspt_ctx *ctx, const SweepArgs &a) {
-  const long nl = 4 * ctx->V;
-  const bool low = use_low(ctx);
-  KernelShape k = low ? choose_shape(ctx, IMP_SLOTS, nl, 0, SWEEP_THREADS_LOW / 32, 2)
-                      : choose_shape(ctx, IMP_SLOTS, nl, 0);
-  const size_t smem = (size_t)k.warps * LPW * group_bytes(ctx, IMP_SLOTS, 0);
-  const long per_cta = (long)k.warps * LPW;
-  const unsigned grid = (unsigned)((nl + per_cta - 1) / per_cta);
-  if (low) {
-    cudaFuncSetAttribute(k_sweep_imp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_sweep_imp<true><<<grid, 32 * k.warps, smem, ctx->st>>>(a);
-  } else {
-    cudaFuncSetAttribute(k_sweep_imp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_sweep_imp<false><<<grid, 32 * k.warps, smem, ctx->st>>>(a);
-  }
-  CK(cudaGetLastError());
-  return NSPT_OK;
-}
-
-// Launch a per-link (or per-site) group kernel with `slots` series per group.
-// low: the kernel's low-order instantiation (N <= 3 MO_LOW; 6-warp CTAs,
-// two per SM).
-template <class Fn>
-static int launch_groups(nspt_ctx *ctx, const void *fn, int slots, long units, Fn launch,
-                         const char *what, int extra = 0, bool low = false) {
-  KernelShape k = low ? choose_shape(ctx, slots, units, extra, SWEEP_THREADS_LOW / 32, 2)
-                      : choose_shape(ctx, slots, units, extra);
-  const size_t smem = (size_t)k.warps * LPW * group_bytes(ctx, slots, extra);
-  const long per_cta = (long)k.warps * LPW;
-  const unsigned grid = (unsigned)((units + per_cta - 1) / per_cta);
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  launch(grid, dim3(32 * k.warps), smem);
-  cudaError_t e = cudaGetLastError();
+// Launch a kernel of a group per unit with `slots` series per group; units too
+// few to fill the GPU are spread over the SMs.
+template <int G, class... P, class... A>
+static int wlaunch(nspt_ctx *ctx, std::integral_constant<int, G>, void (*kernel)(P...), int slots,
+                   long units, const char *what, A... args) {
+  Shape k = group_shape(glanes<G>(), sm_ctas<G>(), slots, ctx->SS, ctx->smem_optin,
+                        ctx->sweep_warps > 0 ? ctx->sweep_warps : CTA_WARPS);
+  if (k.gpc < 1) return NSPT_ERR_ORDER;
+  k.gpc = (int)std::max<long>(1, std::min<long>(k.gpc, (units + ctx->nsm - 1) / ctx->nsm));
+  k.warps = std::min(k.warps, k.gpc);
+  k.smem = (LEAD + (size_t)k.gpc * group_stride(slots, ctx->SS)) * sizeof(double2);
+  cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)ctx->smem_optin);
+  kernel<<<(unsigned)((units + k.gpc - 1) / k.gpc), 32 * k.warps, k.smem, ctx->st>>>(args..., k.gpc);
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     ctx->err = std::string(what) + ": " + cudaGetErrorString(e);
     return NSPT_ERR_CUDA;
@@ -238,21 +220,33 @@ static int launch_groups(nspt_ctx *ctx, const void *fn, int slots, long units, F
 
 // ---------------- reductions ----------------
 
-// rectangle traces of the improved actions sit after the MM area of red2
-static size_t w2_offset(int N) { return (size_t)(N + 1) + 4 * N + 36 * N; }
+// Column sums (k_colsum) in a fixed order that depends on the sizes alone.
+constexpr int COLSUM_CHUNKS = 296;
+
+static int colsum(nspt_ctx *ctx, const double *in, long rows, int width, double *out) {
+  const long chunk = std::max<long>(32, (rows + COLSUM_CHUNKS - 1) / COLSUM_CHUNKS);
+  const long n = (rows + chunk - 1) / chunk;
+  const unsigned cols = (unsigned)((width + 31) / 32);
+  k_colsum<<<dim3(cols, (unsigned)n), 256, 0, ctx->st>>>(in, rows, width, chunk, ctx->red_part);
+  k_colsum<<<cols, 256, 0, ctx->st>>>(ctx->red_part, n, width, n, out);
+  CK(cudaGetLastError());
+  return NSPT_OK;
+}
+
+// the areas of red
+static size_t red_tr(const nspt_ctx *ctx) { return 12 * (size_t)ctx->N; }
+static size_t red_tr2(const nspt_ctx *ctx) { return red_tr(ctx) + 8 * (size_t)(ctx->N + 1); }
+static size_t red_mm(const nspt_ctx *ctx) { return red_tr2(ctx) + 8 * (size_t)(ctx->N + 1); }
+static size_t red_size(const nspt_ctx *ctx) { return red_mm(ctx) + 8 * link_rec(ctx->N); }
 
 static int reduce_sweep_obs(nspt_ctx *ctx) {
   const int N = ctx->N;
-  const long nl = 4 * ctx->V;
-  if (ctx->c1 != 0.0)
-    k_rowsum<double2><<<N + 1, 256, 0, ctx->st>>>(ctx->obs_tr2, (size_t)nl, nl,
-                                                   ctx->red2 + w2_offset(N));
-  k_rowsum<double2><<<N + 1, 256, 0, ctx->st>>>(ctx->obs_tr, (size_t)nl, nl, ctx->red2);
-  k_rowsum<double2><<<4 * N, 256, 0, ctx->st>>>(ctx->obs_tru, (size_t)ctx->V, ctx->V,
-                                                   ctx->red2 + (N + 1));
-  k_rowsum<double><<<N, 256, 0, ctx->st>>>(ctx->obs_norm, (size_t)nl, nl, ctx->red1);
-  CK(cudaGetLastError());
-  return NSPT_OK;
+  int rc = colsum(ctx, ctx->obs, ctx->V, 12 * N, ctx->red);
+  const int w = ctx->tr_rows == 6 ? 6 * (N + 1) : 8 * (N + 1);
+  if (!rc) rc = colsum(ctx, ctx->obs_tr, ctx->V, w, ctx->red + red_tr(ctx));
+  if (!rc && ctx->c1 != 0.0)
+    rc = colsum(ctx, ctx->obs_tr2, ctx->V, 8 * (N + 1), ctx->red + red_tr2(ctx));
+  return rc;
 }
 
 // The reference's OpenMP thread grid (the context's gf_grid) as the kernels
@@ -280,125 +274,82 @@ static LgfGrid thread_grid(const nspt_ctx *ctx, long &steps) {
 
 // gauge_wilson on the fly (UPDATE_ONTHEFLY, nspt.cc:355-460): one launch per
 // barrier step of the thread grid, one group per reference thread.
-static int launch_sweep_otf(nspt_ctx *ctx, const SweepArgs &a0) {
+static int launch_sweep_otf(nspt_ctx *ctx, const SweepArgs &a) {
   long steps;
   const LgfGrid gr = thread_grid(ctx, steps);
-  const bool low = use_low(ctx);
-  const int max_warps = (low ? SWEEP_THREADS_LOW : SWEEP_THREADS) / 32;
-  const KernelShape k = choose_shape(ctx, SWEEP_SLOTS, gr.nthr, 0, max_warps, low ? 2 : 1);
-  int warps = k.warps;
-  SweepArgs a = a0;
-  a.gpc = k.warps * LPW;
-  if (!low && k.warps < max_warps) {
-    // as the Jacobi sweep: as many groups as shared memory holds, dealt over
-    // all max_warps warps (sweep_group), where that keeps >= 2.5 per warp
-    const long fit = std::min<long>((long)(ctx->smem_optin / group_bytes(ctx, SWEEP_SLOTS, 0)),
-                                    (long)max_warps * LPW);
-    const long want = (gr.nthr + 2L * ctx->nsm - 1) / (2L * ctx->nsm);
-    if (fit > a.gpc && want >= fit && 2 * fit >= 5L * max_warps) {
-      a.gpc = (int)fit;
-      warps = max_warps;
-    }
-  }
-  const size_t smem = (size_t)a.gpc * group_bytes(ctx, SWEEP_SLOTS, 0);
-  const unsigned grid = (unsigned)((gr.nthr + a.gpc - 1) / a.gpc);
-  // a warp of three groups per reference thread (the three planes' staples
-  // side by side) where every team of a barrier step fits on the GPU at once
-  const size_t team_bytes = (size_t)LPW * SWEEP_SLOTS * ctx->SS * sizeof(double2);
-  int team_warps = 4;
-  while (team_warps > 1 && (size_t)team_warps * team_bytes > ctx->smem_optin) team_warps /= 2;
-  bool team = gr.seg == 1 && team_bytes <= ctx->smem_optin && ctx->gf_form != NSPT_LGF_GROUP;
-  if (team && ctx->gf_form == NSPT_LGF_AUTO) {
-    const long per_sm = std::min<long>((long)((size_t)228 * 1024 / team_bytes), low ? 12 : 8);
-    team = gr.nthr <= per_sm * ctx->nsm;
-  }
-  if (team) {
-    const size_t tsmem = (size_t)team_warps * team_bytes;
-    const void *fn =
-        low ? (const void *)k_sweep_otf1_team<true> : (const void *)k_sweep_otf1_team<false>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
-    const unsigned tgrid = (unsigned)((gr.nthr + team_warps - 1) / team_warps);
-    for (long p = 0; p < steps; p++)
-      for (int mu = 0; mu < 4; mu++) {
-        if (low)
-          k_sweep_otf1_team<true><<<tgrid, 32 * team_warps, tsmem, ctx->st>>>(a, gr, p, mu);
-        else
-          k_sweep_otf1_team<false><<<tgrid, 32 * team_warps, tsmem, ctx->st>>>(a, gr, p, mu);
-      }
-  } else if (gr.seg == 1) {
-    // one site per thread and barrier step: a launch per (step, mu), the
-    // link update inline without a loop around it
-    const void *fn = low ? (const void *)k_sweep_otf1<true> : (const void *)k_sweep_otf1<false>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    for (long p = 0; p < steps; p++)
-      for (int mu = 0; mu < 4; mu++) {
-        if (low)
-          k_sweep_otf1<true><<<grid, 32 * warps, smem, ctx->st>>>(a, gr, p, mu);
-        else
-          k_sweep_otf1<false><<<grid, 32 * warps, smem, ctx->st>>>(a, gr, p, mu);
-      }
-  } else {
-    const void *fn = low ? (const void *)k_sweep_otf<true> : (const void *)k_sweep_otf<false>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    for (long p = 0; p < steps; p++) {
-      if (low)
-        k_sweep_otf<true><<<grid, 32 * warps, smem, ctx->st>>>(a, gr, p);
-      else
-        k_sweep_otf<false><<<grid, 32 * warps, smem, ctx->st>>>(a, gr, p);
-    }
-  }
-  CK(cudaGetLastError());
-  return NSPT_OK;
+  int rc = NSPT_OK;
+  with_grid_form(ctx, gr.nthr, [&](auto G) {
+    for (long p = 0; p < steps && !rc; p++)
+      rc = ctx->c1 != 0.0 ? wlaunch(ctx, G, k_sweep_imp_otf<G.value>, IMP_SLOTS, gr.nthr,
+                                    "on-the-fly sweep", a, gr, p)
+                          : wlaunch(ctx, G, k_sweep_otf<G.value>, LINK_SLOTS, gr.nthr,
+                                    "on-the-fly sweep", a, gr, p);
+  });
+  return rc;
 }
 
-// The improved-action sweep on the fly (periodic boundaries only): one
-// launch per barrier step, or per (barrier step, mu) where every thread owns
-// one site per barrier step.
-static int launch_sweep_imp_otf(nspt_ctx *ctx, const SweepArgs &a) {
-  long steps;
-  const LgfGrid gr = thread_grid(ctx, steps);
-  const bool low = use_low(ctx);
-  const int max_warps = low ? SWEEP_THREADS_LOW / 32 : 8;
-  const KernelShape k = choose_shape(ctx, IMP_SLOTS, gr.nthr, 0, max_warps, low ? 2 : 1);
-  const size_t smem = (size_t)k.warps * LPW * group_bytes(ctx, IMP_SLOTS, 0);
-  const long per_cta = (long)k.warps * LPW;
-  const unsigned grid = (unsigned)((gr.nthr + per_cta - 1) / per_cta);
-  if (gr.seg == 1) {
-    const void *fn =
-        low ? (const void *)k_sweep_imp_otf1<true> : (const void *)k_sweep_imp_otf1<false>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    for (long p = 0; p < steps; p++)
-      for (int mu = 0; mu < 4; mu++) {
-        if (low)
-          k_sweep_imp_otf1<true><<<grid, 32 * k.warps, smem, ctx->st>>>(a, gr, p, mu);
-        else
-          k_sweep_imp_otf1<false><<<grid, 32 * k.warps, smem, ctx->st>>>(a, gr, p, mu);
-      }
-  } else {
-    const void *fn =
-        low ? (const void *)k_sweep_imp_otf<true> : (const void *)k_sweep_imp_otf<false>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    for (long p = 0; p < steps; p++) {
-      if (low)
-        k_sweep_imp_otf<true><<<grid, 32 * k.warps, smem, ctx->st>>>(a, gr, p, 0, 4);
-      else
-        k_sweep_imp_otf<false><<<grid, 32 * k.warps, smem, ctx->st>>>(a, gr, p, 0, 4);
-    }
+// The Jacobi sweep plaquette by plaquette, slab by slab of direction 0: the
+// plaquettes of a slab, then its links.  A slab's links also need the
+// plaquettes of the plane before it, kept in the other buffer; the first slab
+// takes them from the last plane, whose plaquettes are formed ahead for it.
+template <bool FF, int G>
+static int launch_sweep_plaq(nspt_ctx *ctx, SweepArgs a) {
+  const std::integral_constant<int, G> g;
+  const int L0 = ctx->L[0], s0 = ctx->geo.s0;
+  auto plaq = [&](int x, int n, int buf) {
+    a.site0 = x * s0;
+    a.nsite = n * s0;
+    a.plaq = ctx->plaq[buf];
+    return wlaunch(ctx, g, k_plaq<FF, G>, PLAQ_SLOTS, 6L * a.nsite, "sweep, plaquettes", a);
+  };
+  int cur = 0, rc = NSPT_OK;
+  a.prev = ctx->plaq[0];
+  a.prev0 = 0;
+  if (ctx->slab < L0) {
+    rc = plaq(L0 - 1, 1, 1);
+    a.prev = ctx->plaq[1];
+    a.prev0 = a.site0;
   }
-  CK(cudaGetLastError());
-  return NSPT_OK;
+  for (int x = 0; x < L0 && !rc; x += ctx->slab) {
+    rc = plaq(x, std::min(ctx->slab, L0 - x), cur);
+    if (!rc)
+      rc = wlaunch(ctx, g, k_update<FF, G>, UPDATE_SLOTS, 4L * a.nsite, "sweep, links", a);
+    a.prev = a.plaq;
+    a.prev0 = a.site0;
+    cur ^= 1;
+  }
+  return rc;
+}
+
+static int launch_sweep(nspt_ctx *ctx, const SweepArgs &a) {
+  const bool ff = (ctx->flags & NSPT_PRECISION_FF) != 0;
+  const long nl = 4 * ctx->V;
+  int rc = NSPT_OK;
+  with_form(ctx, nl, [&](auto G) {
+    constexpr int g = G.value;
+    if constexpr (g != ORDERED) {
+      if (ctx->tr_rows == 6) {
+        rc = ff ? launch_sweep_plaq<true, g>(ctx, a) : launch_sweep_plaq<false, g>(ctx, a);
+        return;
+      }
+    }
+    if (ctx->c1 != 0.0)
+      rc = wlaunch(ctx, G, k_sweep_imp<g>, IMP_SLOTS, nl, "sweep", a);
+    else
+      rc = ff ? wlaunch(ctx, G, k_sweep_link<true, g>, LINK_SLOTS, nl, "sweep", a)
+              : wlaunch(ctx, G, k_sweep_link<false, g>, LINK_SLOTS, nl, "sweep", a);
+  });
+  return rc;
 }
 
 static int do_sweep(nspt_ctx *ctx, double dt, bool use_noise) {
   SweepArgs a;
+  memset(&a, 0, sizeof(a));
   a.U = ctx->U;
-  a.Uf = ctx->Uf;
   a.F = ctx->F;
-  a.Ff = ctx->Ff;
   a.Lg = (ctx->flags & NSPT_ZEROMODE) ? ctx->Lg : nullptr;
+  a.obs = ctx->obs;
   a.obs_tr = ctx->obs_tr;
-  a.obs_norm = ctx->obs_norm;
-  a.obs_tru = ctx->obs_tru;
   a.noise = use_noise ? ctx->noise : nullptr;
   a.seed = ctx->seed;
   a.step = ctx->counter;
@@ -416,23 +367,25 @@ static int do_sweep(nspt_ctx *ctx, double dt, bool use_noise) {
   a.SS = ctx->SS;
   a.g = ctx->geo;
   a.Ut = ctx->U;
-  a.Utf = ctx->Uf;
   const bool otf = (ctx->flags & NSPT_UPDATE_ONTHEFLY) != 0;
+  // plaquette by plaquette unless the order of the links is fixed, the action
+  // has rectangles, the sums have an order to keep, the records found no
+  // memory, or a flag other than 1 meets
+  // a twisted face (where each link's staples see flags of their own)
+  ctx->tr_rows = !otf && ctx->c1 == 0.0 && ctx->plaq[0] && !ordered(ctx) &&
+                         (ctx->unit_flags || !ctx->geo.twist)
+                     ? 6 : 4;
   if (otf) {
     // in place; with twisted boundaries F keeps the step's start field for
     // the reads across a twisted face (the reference's copy sites)
     a.F = ctx->U;
-    a.Ff = ctx->Uf;
     if (ctx->geo.twist) {
       if (!ctx->snap_valid) {
-        const size_t nb = (size_t)4 * 9 * ctx->N * ctx->V * sizeof(double2);
+        const size_t nb = (size_t)4 * ctx->V * link_rec(ctx->N) * sizeof(double2);
         CK(cudaMemcpyAsync(ctx->F, ctx->U, nb, cudaMemcpyDeviceToDevice, ctx->st));
-        CK(cudaMemcpyAsync(ctx->Ff, ctx->Uf, (size_t)4 * ctx->V * sizeof(double2),
-                           cudaMemcpyDeviceToDevice, ctx->st));
         ctx->snap_valid = true;
       }
       a.Ut = ctx->F;
-      a.Utf = ctx->Ff;
     }
   }
   if ((ctx->flags & NSPT_PRECISION_FF) && ctx->ff_auto) {
@@ -445,10 +398,7 @@ static int do_sweep(nspt_ctx *ctx, double dt, bool use_noise) {
   }
   const bool timed = ctx->kcount < nspt_ctx::KEV;
   if (timed) CK(cudaEventRecord(ctx->kev[2 * ctx->kcount], ctx->st));
-  int rc = otf && ctx->c1 != 0.0 ? launch_sweep_imp_otf(ctx, a)
-           : otf                 ? launch_sweep_otf(ctx, a)
-           : ctx->c1 != 0.0      ? launch_sweep_imp(ctx, a)
-                                 : launch_sweep(ctx, a, false);
+  int rc = otf ? launch_sweep_otf(ctx, a) : launch_sweep(ctx, a);
   if (rc) return rc;
   if (timed) {
     CK(cudaEventRecord(ctx->kev[2 * ctx->kcount + 1], ctx->st));
@@ -460,7 +410,6 @@ static int do_sweep(nspt_ctx *ctx, double dt, bool use_noise) {
   CK(cudaGetLastError());
   if (!otf) {
     std::swap(ctx->U, ctx->F);
-    std::swap(ctx->Uf, ctx->Ff);
   }
   ctx->counter++;
   ctx->have_obs = true;
@@ -470,26 +419,20 @@ static int do_sweep(nspt_ctx *ctx, double dt, bool use_noise) {
 
 static int do_zero_modes(nspt_ctx *ctx) {
   const int N = ctx->N;
-  double2 *MM = ctx->red2 + (N + 1) + 4 * N;
-  k_rowsum<double2><<<4 * 9 * N, 256, 0, ctx->st>>>(ctx->Lg, (size_t)ctx->V, ctx->V, MM);
-  k_scale_mm<<<(36 * N + 127) / 128, 128, 0, ctx->st>>>(MM, 36 * N, 1.0 / (double)ctx->V);
-  CK(cudaGetLastError());
-  const long nl = 4 * ctx->V;
-  double2 *U = ctx->U, *Uf = ctx->Uf;
-  double2 *Lg = ctx->Lg;
-  const int SS = ctx->SS;
-  const Geo geo = ctx->geo;
-  cudaStream_t st = ctx->st;
-  const bool low = use_low(ctx);
-  const int rc = launch_groups(
-      ctx, low ? (const void *)k_zero_modes<true> : (const void *)k_zero_modes<false>, 3, nl,
-      [&](unsigned g, dim3 b, size_t sm) {
-        if (low)
-          k_zero_modes<true><<<g, b, sm, st>>>(U, Uf, Lg, MM, N, SS, geo);
-        else
-          k_zero_modes<false><<<g, b, sm, st>>>(U, Uf, Lg, MM, N, SS, geo);
-      },
-      "zero modes", 0, low);
+  double *mm = ctx->red + red_mm(ctx);
+  int rc = NSPT_OK;
+  const int width = 4 * (int)link_rec(N);
+  if (ordered(ctx)) {
+    k_logsum<<<(width + LOGSUM_COLS - 1) / LOGSUM_COLS, 256, 0, ctx->st>>>(ctx->Lg, ctx->V, width,
+                                                                           (double2 *)mm);
+    CK(cudaGetLastError());
+  } else if ((rc = colsum(ctx, (const double *)ctx->Lg, ctx->V, 2 * width, mm))) {
+    return rc;
+  }
+  with_form(ctx, 4 * ctx->V, [&](auto G) {
+    rc = wlaunch(ctx, G, k_zero_modes<G.value>, SERIES_SLOTS, 4 * ctx->V, "zero modes", ctx->U,
+                 ctx->Lg, (const double2 *)mm, 1.0 / (double)ctx->V, N, ctx->SS, ctx->geo);
+  });
   if (rc == NSPT_OK) ctx->lg_current = true;  // Lg = the new field's log
   return rc;
 }
@@ -528,19 +471,12 @@ static bool fft_planned(int n) {
 }
 
 template <int n>
-static void fft_t_launch(nspt_ctx *ctx, double2 *data, const double2 *Lg, bool div, int inv) {
+static void fft_t_launch(nspt_ctx *ctx, double2 *data, int inv) {
   const long nlines = (long)9 * ctx->N * (ctx->V / n);
   const unsigned grid = (unsigned)((nlines + 127) / 128);
   const size_t smem = (size_t)128 * (n | 1) * sizeof(double2);
-  if (div) {
-    cudaFuncSetAttribute(k_fft_t<n, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fft_t<n, true><<<grid, 128, smem, ctx->st>>>(data, Lg, nlines, 9 * ctx->N, ctx->geo,
-                                                   ctx->ftw + 3 * 128, inv);
-  } else {
-    cudaFuncSetAttribute(k_fft_t<n, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fft_t<n, false><<<grid, 128, smem, ctx->st>>>(data, Lg, nlines, 9 * ctx->N, ctx->geo,
-                                                    ctx->ftw + 3 * 128, inv);
-  }
+  cudaFuncSetAttribute(k_fft_t<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_fft_t<n><<<grid, 128, smem, ctx->st>>>(data, nlines, ctx->ftw + 3 * 128, inv);
 }
 
 template <int n>
@@ -558,16 +494,15 @@ static void fft_x_launch(nspt_ctx *ctx, double2 *data, double alpha) {
       data, nlines, ctx->geo, ctx->ftw, alpha, ctx->p2);
 }
 
-// Wg = iFFT(-alpha / p^2 FFT(div log U)) in seven passes (fft.cuh), or
+// Wg = iFFT(-alpha / p^2 FFT(Wg)) in seven passes (fft.cuh), or
 // NSPT_ERR_ARG when an extent has no compile-time plan.
 static int fa_fft_fused(nspt_ctx *ctx, double alpha) {
   for (int d = 0; d < 4; d++)
     if (!fft_planned(ctx->L[d])) return NSPT_ERR_ARG;
   double2 *Wg = ctx->Wg;
-  const double2 *Lg = ctx->Lg;
-  auto t_pass = [&](bool div, int inv) {
+  auto t_pass = [&](int inv) {
     switch (ctx->L[3]) {
-#define NSPT_FFT_CASE(n_) case n_: fft_t_launch<n_>(ctx, Wg, Lg, div, inv); break;
+#define NSPT_FFT_CASE(n_) case n_: fft_t_launch<n_>(ctx, Wg, inv); break;
       NSPT_FFT_SIZES(NSPT_FFT_CASE)
 #undef NSPT_FFT_CASE
     }
@@ -579,7 +514,7 @@ static int fa_fft_fused(nspt_ctx *ctx, double alpha) {
 #undef NSPT_FFT_CASE
     }
   };
-  t_pass(true, 0);  // divergence + forward t
+  t_pass(0);
   s_pass(2, 0);
   s_pass(1, 0);
   switch (ctx->L[0]) {  // forward x, -alpha / p^2, backward x
@@ -589,7 +524,7 @@ static int fa_fft_fused(nspt_ctx *ctx, double alpha) {
   }
   s_pass(1, 1);
   s_pass(2, 1);
-  t_pass(false, 1);
+  t_pass(1);
   CK(cudaGetLastError());
   return NSPT_OK;
 }
@@ -599,59 +534,41 @@ static int do_fa(nspt_ctx *ctx, double alpha) {
   const long nl = 4 * ctx->V;
   const Geo geo = ctx->geo;
   cudaStream_t st = ctx->st;
-  double2 *U = ctx->U, *Uf = ctx->Uf, *F = ctx->F, *Ff = ctx->Ff, *Lg = ctx->Lg, *Wg = ctx->Wg,
-          *Gx = ctx->Gx;
-  const bool low = use_low(ctx);
   // log U per link (nspt.cc:874-875); after the zero-mode subtraction Lg
   // already holds it (k_zero_modes)
   int rc = NSPT_OK;
   if (!ctx->lg_current) {
-    rc = launch_groups(
-      ctx, low ? (const void *)k_log_links<true> : (const void *)k_log_links<false>, 3, nl,
-      [&](unsigned g, dim3 b, size_t sm) {
-        if (low)
-          k_log_links<true><<<g, b, sm, st>>>(U, Uf, Lg, N, SS, geo);
-        else
-          k_log_links<false><<<g, b, sm, st>>>(U, Uf, Lg, N, SS, geo);
-      },
-      "FA logs", 0, low);
+    with_form(ctx, nl, [&](auto G) {
+      rc = wlaunch(ctx, G, k_log_links<G.value>, SERIES_SLOTS, nl, "FA logs",
+                   (const double2 *)ctx->U, ctx->Lg, N, SS, geo);
+    });
     if (rc) return rc;
   }
+  k_fa_div<<<dim3((unsigned)((ctx->V + 31) / 32), (unsigned)((9 * N + 31) / 32)), 256, 0, st>>>(
+      ctx->Lg, ctx->Wg, N, geo);
+  CK(cudaGetLastError());
   rc = fa_fft_fused(ctx, alpha);
   if (rc == NSPT_ERR_ARG) {  // an extent without a compile-time FFT plan
     const size_t tot = (size_t)9 * N * ctx->V;
     const unsigned eg = (unsigned)std::min<size_t>((tot + 255) / 256, (size_t)ctx->nsm * 32);
-    k_fa_div<<<eg, 256, 0, st>>>(Lg, Wg, N, geo);
+    if ((rc = fft4d(ctx, ctx->Wg, -1))) return rc;
+    k_fa_scale<<<eg, 256, 0, st>>>(ctx->Wg, N, geo, alpha, ctx->p2);
     CK(cudaGetLastError());
-    if ((rc = fft4d(ctx, Wg, -1))) return rc;
-    k_fa_scale<<<eg, 256, 0, st>>>(Wg, N, geo, alpha, ctx->p2);
-    CK(cudaGetLastError());
-    if ((rc = fft4d(ctx, Wg, +1))) return rc;
+    if ((rc = fft4d(ctx, ctx->Wg, +1))) return rc;
   } else if (rc) {
     return rc;
   }
-  rc = launch_groups(
-      ctx, low ? (const void *)k_fa_gt<true> : (const void *)k_fa_gt<false>, 3, ctx->V,
-      [&](unsigned g, dim3 b, size_t sm) {
-        if (low)
-          k_fa_gt<true><<<g, b, sm, st>>>(Wg, Gx, N, SS, geo);
-        else
-          k_fa_gt<false><<<g, b, sm, st>>>(Wg, Gx, N, SS, geo);
-      },
-      "FA gauge transform", 0, low);
+  with_form(ctx, ctx->V, [&](auto G) {
+    rc = wlaunch(ctx, G, k_fa_gt<G.value>, SERIES_SLOTS, ctx->V, "FA gauge transform",
+                 (const double2 *)ctx->Wg, ctx->Gx, N, SS, geo);
+  });
   if (rc) return rc;
-  rc = launch_groups(
-      ctx, low ? (const void *)k_fa_apply<true> : (const void *)k_fa_apply<false>, 2, nl,
-      [&](unsigned g, dim3 b, size_t sm) {
-        if (low)
-          k_fa_apply<true><<<g, b, sm, st>>>(U, Uf, Gx, F, Ff, N, SS, geo);
-        else
-          k_fa_apply<false><<<g, b, sm, st>>>(U, Uf, Gx, F, Ff, N, SS, geo);
-      },
-      "FA apply", 0, low);
+  with_form(ctx, nl, [&](auto G) {
+    rc = wlaunch(ctx, G, k_fa_apply<G.value>, APPLY_SLOTS, nl, "FA apply", (const double2 *)ctx->U,
+                 (const double2 *)ctx->Gx, ctx->F, N, SS, geo);
+  });
   if (rc) return rc;
   std::swap(ctx->U, ctx->F);
-  std::swap(ctx->Uf, ctx->Ff);
   ctx->lg_current = false;
   return NSPT_OK;
 }
@@ -661,59 +578,17 @@ static int do_fa(nspt_ctx *ctx, double alpha) {
 static int do_local_gf(nspt_ctx *ctx, double alpha) {
   long steps;
   const LgfGrid gr = thread_grid(ctx, steps);
-  const int N = ctx->N, SS = ctx->SS;
-  const Geo geo = ctx->geo;
-  cudaStream_t st = ctx->st;
-  double2 *U = ctx->U, *Uf = ctx->Uf;
   // reads across a twisted face: the step's start field after an on-the-fly
   // sweep (the reference's copy sites before twist_boundary)
-  const double2 *Ut = ctx->snap_valid ? ctx->F : U, *Utf = ctx->snap_valid ? ctx->Ff : Uf;
-  const bool low = use_low(ctx);
+  const double2 *Ut = ctx->snap_valid ? ctx->F : ctx->U;
   ctx->lg_current = false;
-  // The team form (a warp of three groups per reference thread) shortens
-  // each thread's chain of dependent stagings and products about threefold
-  // but keeps a third of its lanes idle in the exps: automatic choice takes
-  // it when every team of the barrier step is resident at once.
-  const size_t team_bytes = (size_t)LGF_TEAM_SLOTS * SS * sizeof(double2);
-  const int team_warps = 2 * team_bytes <= ctx->smem_optin ? 2 : 1;
-  bool team = team_bytes <= ctx->smem_optin && ctx->gf_form != NSPT_LGF_GROUP;
-  if (team && ctx->gf_form == NSPT_LGF_AUTO) {
-    const long per_sm = std::min<long>((long)((size_t)228 * 1024 / team_bytes), low ? 12 : 8);
-    team = gr.nthr <= per_sm * ctx->nsm;
-  }
-  if (team) {
-    const size_t smem = (size_t)team_warps * team_bytes;
-    const void *fn = low ? (const void *)k_local_gf_team<true> : (const void *)k_local_gf_team<false>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const unsigned grid = (unsigned)((gr.nthr + team_warps - 1) / team_warps);
-    for (long p = 0; p < steps; p++) {
-      if (low)
-        k_local_gf_team<true><<<grid, 32 * team_warps, smem, st>>>(U, Uf, Ut, Utf, N, SS, geo,
-                                                                    alpha, gr, p);
-      else
-        k_local_gf_team<false><<<grid, 32 * team_warps, smem, st>>>(U, Uf, Ut, Utf, N, SS, geo,
-                                                                     alpha, gr, p);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      ctx->err = std::string("local gauge fixing: ") + cudaGetErrorString(e);
-      return NSPT_ERR_CUDA;
-    }
-    return NSPT_OK;
-  }
-  for (long p = 0; p < steps; p++) {
-    int rc = launch_groups(
-        ctx, low ? (const void *)k_local_gf<true> : (const void *)k_local_gf<false>, 4, gr.nthr,
-        [&](unsigned g, dim3 b, size_t sm) {
-          if (low)
-            k_local_gf<true><<<g, b, sm, st>>>(U, Uf, Ut, Utf, N, SS, geo, alpha, gr, p);
-          else
-            k_local_gf<false><<<g, b, sm, st>>>(U, Uf, Ut, Utf, N, SS, geo, alpha, gr, p);
-        },
-        "local gauge fixing", 0, low);
-    if (rc) return rc;
-  }
-  return NSPT_OK;
+  int rc = NSPT_OK;
+  with_grid_form(ctx, gr.nthr, [&](auto G) {
+    for (long p = 0; p < steps && !rc; p++)
+      rc = wlaunch(ctx, G, k_local_gf<G.value>, lgf_slots<G.value>(), gr.nthr, "local gauge fixing", ctx->U, Ut,
+                   ctx->N, ctx->SS, ctx->geo, alpha, gr, p);
+  });
+  return rc;
 }
 
 // minb: the smallest block along a split direction.  The reference needs 2
@@ -782,10 +657,9 @@ static int upload_constants(nspt_ctx *ctx) {
 }
 
 static void free_all(nspt_ctx *ctx) {
-  void *ptrs[] = {ctx->U, ctx->Uf, ctx->F, ctx->Ff, ctx->Lg, ctx->Wg, ctx->Gx, ctx->p2, ctx->ftw,
-                  ctx->dcounter,
-                  ctx->loop_part, ctx->obs_tr2, ctx->ff_e, ctx->ff_mx,
-                  ctx->obs_tr, ctx->obs_tru, ctx->obs_norm, ctx->red2, ctx->red1, ctx->noise};
+  void *ptrs[] = {ctx->U, ctx->F, ctx->Lg, ctx->Wg, ctx->Gx, ctx->p2, ctx->ftw, ctx->dcounter,
+                  ctx->loop_part, ctx->obs_tr2, ctx->ff_e, ctx->ff_mx, ctx->plaq[0], ctx->plaq[1],
+                  ctx->obs, ctx->obs_tr, ctx->red, ctx->red_part, ctx->meas, ctx->noise};
   for (void *p : ptrs)
     if (p) cudaFree(p);
 }
@@ -826,7 +700,11 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
   ctx->flags = flags;
   ctx->alpha = alpha;
   ctx->V = V;
-  ctx->U = ctx->Uf = ctx->F = ctx->Ff = ctx->Lg = ctx->Wg = ctx->Gx = nullptr;
+  ctx->U = ctx->F = ctx->Lg = ctx->Wg = ctx->Gx = nullptr;
+  ctx->plaq[0] = ctx->plaq[1] = ctx->meas = nullptr;
+  ctx->slab = L[0];
+  ctx->unit_flags = true;
+  ctx->tr_rows = 4;
   ctx->p2 = nullptr;
   ctx->ftw = nullptr;
   ctx->dcounter = nullptr;
@@ -861,8 +739,7 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
     }
   }
   ctx->gf_form = NSPT_LGF_AUTO;
-  ctx->obs_tr = ctx->obs_tru = ctx->red2 = nullptr;
-  ctx->obs_norm = ctx->red1 = ctx->noise = nullptr;
+  ctx->obs = ctx->obs_tr = ctx->red = ctx->red_part = ctx->noise = nullptr;
   ctx->noise_pending = false;
   ctx->have_obs = false;
   ctx->seed = 0x5eed5eedULL;
@@ -886,53 +763,60 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
   g.s1 = L[2] * L[3];
   g.s0 = L[1] * L[2] * L[3];
   g.twist = 0;
-  // the sweep's site tiles (sweep_link): 4 x 4 x 4 where the extents allow
-  // (measured at 16^4 x 24: DRAM traffic 1.68x the algorithmic bytes, against
-  // 2.89x for 4 x 4 x L2 and 3.98x untiled; the same kernel time)
-  g.t0 = L[0] % 4 == 0 ? 4 : L[0] % 2 == 0 ? 2 : 1;
-  g.t1 = L[1] % 4 == 0 ? 4 : L[1] % 2 == 0 ? 2 : 1;
-  g.t2 = L[2] % 4 == 0 ? 4 : L[2] % 2 == 0 ? 2 : 1;
   if (flags & NSPT_TWIST_Y) g.twist |= 2u;
   if (flags & NSPT_TWIST_Z) g.twist |= 4u;
   if (flags & NSPT_TWIST_T) g.twist |= 8u;
-  // slot stride = 3 (mod 8) 16-byte quads: see series.cuh on bank quads
-  ctx->SS = 1 + 9 * N;
-  while (ctx->SS % 8 != 3) ctx->SS++;
-  // one warp (3 link groups of 3 slots) must fit in a CTA
-  if ((size_t)LPW * group_bytes(ctx, SWEEP_SLOTS, 0) > ctx->smem_optin) return fail(NSPT_ERR_ORDER);
-  if (ctx->c1 != 0.0 && (size_t)LPW * group_bytes(ctx, IMP_SLOTS, 0) > ctx->smem_optin)
-    return fail(NSPT_ERR_ORDER);
+  ctx->SS = (int)link_rec(N);
+  // every kernel's slots of one warp must fit in a CTA
+  if (group_shape(32, 1, 4, ctx->SS, ctx->smem_optin).gpc < 1) return fail(NSPT_ERR_ORDER);
   if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess) return fail(NSPT_ERR_CUDA);
   cudaEventCreate(&ctx->ev0);
   cudaEventCreate(&ctx->ev1);
   for (int i = 0; i < 2 * nspt_ctx::KEV; i++) cudaEventCreate(&ctx->kev[i]);
   ctx->kcount = 0;
   ctx->last_kernel_ms = 0.0;
-  const size_t field = (size_t)4 * 9 * N * V * sizeof(double2);
-  const size_t flagb = (size_t)4 * V * sizeof(double2);
+  const size_t links = (size_t)4 * V * link_rec(N) * sizeof(double2);
   const size_t nl = (size_t)4 * V;
+  const size_t width = std::max<size_t>({12 * (size_t)N, 8 * (size_t)(N + 1), 8 * link_rec(N)});
   auto alloc = [&](void **p, size_t n) {
     if (cudaMalloc(p, n) != cudaSuccess) return false;
     ctx->bytes += n;
     return true;
   };
-  bool ok = alloc((void **)&ctx->U, field) && alloc((void **)&ctx->F, field) &&
-            alloc((void **)&ctx->Uf, flagb) && alloc((void **)&ctx->Ff, flagb) &&
-            alloc((void **)&ctx->obs_tr, (N + 1) * nl * sizeof(double2)) &&
-            alloc((void **)&ctx->obs_tru, N * nl * sizeof(double2)) &&
-            alloc((void **)&ctx->obs_norm, N * nl * sizeof(double)) &&
-            alloc((void **)&ctx->red2, (2 * (N + 1) + 4 * N + 36 * N) * sizeof(double2)) &&
-            alloc((void **)&ctx->red1, N * sizeof(double)) &&
+  bool ok = alloc((void **)&ctx->U, links) && alloc((void **)&ctx->F, links) &&
+            alloc((void **)&ctx->obs, nl * 3 * N * sizeof(double)) &&
+            alloc((void **)&ctx->obs_tr, nl * 2 * (N + 1) * sizeof(double)) &&
+            alloc((void **)&ctx->red, red_size(ctx) * sizeof(double)) &&
+            alloc((void **)&ctx->red_part, COLSUM_CHUNKS * width * sizeof(double)) &&
+            alloc((void **)&ctx->meas, (size_t)MEASURE_CTAS * (N + 1) * sizeof(double2)) &&
             alloc((void **)&ctx->p2, 4 * 128 * sizeof(double)) &&
             alloc((void **)&ctx->dcounter, sizeof(unsigned long long));
-  if (ok && (flags & (NSPT_ZEROMODE | NSPT_GF_FA))) ok = alloc((void **)&ctx->Lg, field);
-  if (ok && ctx->c1 != 0.0) ok = alloc((void **)&ctx->obs_tr2, (N + 1) * nl * sizeof(double2));
+  if (ok && (flags & (NSPT_ZEROMODE | NSPT_GF_FA))) ok = alloc((void **)&ctx->Lg, links);
+  if (ok && ctx->c1 != 0.0)
+    ok = alloc((void **)&ctx->obs_tr2, nl * 2 * (N + 1) * sizeof(double));
   if (ok && (flags & NSPT_PRECISION_FF))
     ok = alloc((void **)&ctx->ff_e, sizeof(int)) &&
          alloc((void **)&ctx->ff_mx, N * sizeof(unsigned long long));
   if (ok && (flags & NSPT_GF_FA))
-    ok = alloc((void **)&ctx->Wg, field / 4) && alloc((void **)&ctx->Gx, field / 4) &&
-         alloc((void **)&ctx->ftw, 4 * 128 * sizeof(double2));
+    ok = alloc((void **)&ctx->Wg, (size_t)9 * N * V * sizeof(double2)) &&
+         alloc((void **)&ctx->Gx, links / 4) && alloc((void **)&ctx->ftw, 4 * 128 * sizeof(double2));
+  if (ok && !(flags & NSPT_UPDATE_ONTHEFLY) && ctx->c1 == 0.0 && !ordered(ctx)) {
+    // Plaquette records of two slabs of at least SLAB_SITES sites, or of the
+    // whole lattice where that is no more.  Without the memory for them the
+    // sweep goes link by link.
+    const long plane = V / L[0];
+    ctx->slab = (int)std::min<long>(L[0], (SLAB_SITES + plane - 1) / plane);
+    if (2 * ctx->slab >= L[0]) ctx->slab = L[0];
+    const size_t n = (size_t)ctx->slab * plane * 18 * link_rec(N) * sizeof(double2);
+    if (cudaMalloc(&ctx->plaq[0], n) != cudaSuccess ||
+        (ctx->slab < L[0] && cudaMalloc(&ctx->plaq[1], n) != cudaSuccess)) {
+      cudaGetLastError();
+      if (ctx->plaq[0]) cudaFree(ctx->plaq[0]);
+      ctx->plaq[0] = ctx->plaq[1] = nullptr;
+    } else {
+      ctx->bytes += ctx->slab < L[0] ? 2 * n : n;
+    }
+  }
   if (!ok) {
     cudaGetLastError();
     cudaStreamDestroy(ctx->st);
@@ -962,12 +846,17 @@ extern "C" int nspt_destroy(nspt_ctx *ctx) {
 
 extern "C" size_t nspt_device_bytes(const nspt_ctx *ctx) { return ctx ? ctx->bytes : 0; }
 
+static void set_unit_flags(nspt_ctx *ctx, bool unit) {
+  if (ctx->unit_flags != unit) ctx->launch_gen++;  // the sweep's route may change
+  ctx->unit_flags = unit;
+}
+
 extern "C" int nspt_cold_start(nspt_ctx *ctx) {
   if (!ctx) return NSPT_ERR_ARG;
   ctx->lg_current = false;
   ctx->snap_valid = false;  // a new field: no stale twisted reads
-  const size_t nU = (size_t)4 * 9 * ctx->N * ctx->V, nF = (size_t)4 * ctx->V;
-  k_cold<<<ctx->nsm * 8, 256, 0, ctx->st>>>(ctx->U, ctx->Uf, nU, nF);
+  set_unit_flags(ctx, true);
+  k_cold<<<ctx->nsm * 8, 256, 0, ctx->st>>>(ctx->U, (size_t)4 * ctx->V, ctx->N);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->st));
   return NSPT_OK;
@@ -975,11 +864,27 @@ extern "C" int nspt_cold_start(nspt_ctx *ctx) {
 
 static const size_t kChunkBytes = 64u << 20;
 
+static int field_copy(nspt_ctx *ctx, void *host, void *dev, size_t bytes, bool to_host) {
+  CK(cudaMemcpyAsync(to_host ? host : dev, to_host ? dev : host, bytes,
+                     to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  return NSPT_OK;
+}
+
 extern "C" int nspt_upload_links(nspt_ctx *ctx, const void *aos, int A) {
   if (!ctx || !aos || A < ctx->N) return NSPT_ERR_ARG;
   ctx->lg_current = false;
   ctx->snap_valid = false;  // a new field: no stale twisted reads
-  const size_t per_site = (size_t)4 * (1 + 9 * A) * sizeof(double2);
+  const size_t rec = 1 + 9 * (size_t)A, per_site = 4 * rec * sizeof(double2);
+  {
+    const double *f = (const double *)aos;
+    bool unit = true;
+    for (size_t l = 0; l < (size_t)4 * ctx->V && unit; l++)
+      unit = f[2 * rec * l] == 1.0 && f[2 * rec * l + 1] == 0.0;
+    set_unit_flags(ctx, unit);
+  }
+  if (A == ctx->N)  // the device layout
+    return field_copy(ctx, const_cast<void *>(aos), ctx->U, per_site * ctx->V, false);
   const int cs = (int)std::max<size_t>(1, std::min<size_t>(kChunkBytes / per_site, ctx->V));
   double2 *buf = nullptr;
   CK(cudaMalloc(&buf, per_site * cs));
@@ -989,8 +894,7 @@ extern "C" int nspt_upload_links(nspt_ctx *ctx, const void *aos, int A) {
     cudaError_t e = cudaMemcpyAsync(buf, (const char *)aos + per_site * s0, per_site * n,
                                     cudaMemcpyHostToDevice, ctx->st);
     if (e == cudaSuccess) {
-      k_unpack<<<ctx->nsm * 8, 256, 0, ctx->st>>>(buf, A, (int)s0, n, ctx->U, ctx->Uf, ctx->N,
-                                                  (size_t)ctx->V);
+      k_unpack<<<ctx->nsm * 8, 256, 0, ctx->st>>>(buf, A, (int)s0, n, ctx->U, ctx->N);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -1007,14 +911,15 @@ extern "C" int nspt_upload_links(nspt_ctx *ctx, const void *aos, int A) {
 extern "C" int nspt_download_links(nspt_ctx *ctx, void *aos, int A) {
   if (!ctx || !aos || A < ctx->N) return NSPT_ERR_ARG;
   const size_t per_site = (size_t)4 * (1 + 9 * A) * sizeof(double2);
+  if (A == ctx->N)  // the device layout
+    return field_copy(ctx, aos, ctx->U, per_site * ctx->V, true);
   const int cs = (int)std::max<size_t>(1, std::min<size_t>(kChunkBytes / per_site, ctx->V));
   double2 *buf = nullptr;
   CK(cudaMalloc(&buf, per_site * cs));
   int rc = NSPT_OK;
   for (long s0 = 0; s0 < ctx->V; s0 += cs) {
     const int n = (int)std::min<long>(cs, ctx->V - s0);
-    k_pack<<<ctx->nsm * 8, 256, 0, ctx->st>>>(buf, A, (int)s0, n, ctx->U, ctx->Uf, ctx->N,
-                                              (size_t)ctx->V);
+    k_pack<<<ctx->nsm * 8, 256, 0, ctx->st>>>(buf, A, (int)s0, n, ctx->U, ctx->N);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
       e = cudaMemcpyAsync((char *)aos + per_site * s0, buf, per_site * n, cudaMemcpyDeviceToHost,
@@ -1149,12 +1054,11 @@ extern "C" int nspt_fa_gauge_fixing(nspt_ctx *ctx, double alpha) {
 // h[q * (N+1) + k], un-normalised (k_loops, then its per-CTA rows summed)
 static int loop_sums(nspt_ctx *ctx, std::vector<double2> &h) {
   const int N = ctx->N, row = 4 * (N + 1);
-  const size_t gb = ((size_t)LOOP_SLOTS * ctx->SS + row) * sizeof(double2);
-  const int warps = (int)std::min<size_t>(8, ctx->smem_optin / (LPW * gb));
-  if (warps < 1) return NSPT_ERR_ORDER;
   const long units = 6L * ctx->V;
-  const long per_cta = (long)warps * LPW;
-  const int grid = (int)std::min<long>((units + per_cta - 1) / per_cta, 8L * ctx->nsm);
+  const int lanes = form_lanes(ctx, units);
+  const Shape sh = group_shape(lanes, 4, LOOP_SLOTS + LOOP_EXTRA, ctx->SS, ctx->smem_optin);
+  if (sh.gpc < 1) return NSPT_ERR_ORDER;
+  const int grid = (int)std::min<long>((units + sh.gpc - 1) / sh.gpc, 8L * ctx->nsm);
   const size_t need = (size_t)(grid + 1) * row;
   if (need > ctx->loop_part_n) {
     if (ctx->loop_part) cudaFree(ctx->loop_part);
@@ -1167,11 +1071,15 @@ static int loop_sums(nspt_ctx *ctx, std::vector<double2> &h) {
     ctx->loop_part_n = need;
   }
   double2 *part = ctx->loop_part, *res = ctx->loop_part + (size_t)grid * row;
-  const size_t smem = (size_t)warps * LPW * gb;
   int rc = timed_begin(ctx);
   if (rc) return rc;
-  CK(cudaFuncSetAttribute(k_loops, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_loops<<<grid, 32 * warps, smem, ctx->st>>>(ctx->U, ctx->Uf, N, ctx->SS, ctx->geo, part);
+  measure_form(ctx, units, [&](auto G) {
+    cudaFuncSetAttribute(k_loops<G.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)ctx->smem_optin);
+    k_loops<G.value><<<grid, 32 * sh.warps, sh.smem, ctx->st>>>(ctx->U, N, ctx->SS, ctx->geo, part,
+                                                                sh.gpc);
+  });
+  if (rc) return rc;
   CK(cudaGetLastError());
   k_rows_sum<<<(row + 127) / 128, 128, 0, ctx->st>>>(part, grid, row, res);
   CK(cudaGetLastError());
@@ -1273,27 +1181,33 @@ extern "C" int nspt_observables(nspt_ctx *ctx, double *plaq, double *norm, doubl
   if (!ctx) return NSPT_ERR_ARG;
   if (!ctx->have_obs) return NSPT_ERR_STATE;
   const int N = ctx->N;
-  std::vector<double2> r2((N + 1) + 4 * N);
-  std::vector<double> r1(N);
-  CK(cudaMemcpyAsync(r2.data(), ctx->red2, r2.size() * sizeof(double2), cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaMemcpyAsync(r1.data(), ctx->red1, r1.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
+  std::vector<double> r(red_mm(ctx));
+  CK(cudaMemcpyAsync(r.data(), ctx->red, r.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
-  const double V = (double)ctx->V;
-  (void)V;
-  if (plaq)
-    for (int k = 0; k <= N; k++) {  // nspt.cc:570-597
-      plaq[2 * k] = r2[k].x / (double)(72 * ctx->V);
-      plaq[2 * k + 1] = r2[k].y / (double)(72 * ctx->V);
-    }
-  if (norm)
-    for (int k = 0; k < N; k++) norm[k] = r1[k] / (double)(12 * ctx->V);
-  if (trU)
-    for (int k = 0; k < N; k++)
-      for (int mu = 0; mu < 4; mu++) {
-        const double2 t = r2[(N + 1) + 4 * k + mu];
-        trU[2 * (mu * N + k)] = t.x / (double)(3 * ctx->V);
-        trU[2 * (mu * N + k) + 1] = t.y / (double)(3 * ctx->V);
+  if (plaq) {  // nspt.cc:570-597
+    const double *t = r.data() + red_tr(ctx);
+    for (int k = 0; k <= N; k++) {
+      double re = 0.0, im = 0.0;
+      for (int q = 0; q < ctx->tr_rows; q++) {
+        re += ctx->tr_rows == 6 ? 4. * t[q * (N + 1) + k] : t[2 * (q * (N + 1) + k)];
+        im += ctx->tr_rows == 6 ? 0.0 : t[2 * (q * (N + 1) + k) + 1];
       }
+      plaq[2 * k] = re / (double)(72 * ctx->V);
+      plaq[2 * k + 1] = im / (double)(72 * ctx->V);
+    }
+  }
+  for (int k = 0; k < N; k++) {
+    double nrm = 0.0;
+    for (int mu = 0; mu < 4; mu++) {
+      const double *o = r.data() + 3 * (size_t)N * mu;
+      nrm += o[k];
+      if (trU) {
+        trU[2 * (mu * N + k)] = o[N + 2 * k] / (double)(3 * ctx->V);
+        trU[2 * (mu * N + k) + 1] = o[N + 2 * k + 1] / (double)(3 * ctx->V);
+      }
+    }
+    if (norm) norm[k] = nrm / (double)(12 * ctx->V);
+  }
   return NSPT_OK;
 }
 
@@ -1339,34 +1253,39 @@ extern "C" int nspt_rect_observables(nspt_ctx *ctx, double *w2) {
   if (!ctx || !w2) return NSPT_ERR_ARG;
   if (ctx->c1 == 0.0 || !ctx->have_obs) return NSPT_ERR_STATE;
   const int N = ctx->N;
-  std::vector<double2> r(N + 1);
-  CK(cudaMemcpyAsync(r.data(), ctx->red2 + w2_offset(N), r.size() * sizeof(double2),
+  std::vector<double> r(8 * (N + 1));
+  CK(cudaMemcpyAsync(r.data(), ctx->red + red_tr2(ctx), r.size() * sizeof(double),
                      cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   for (int k = 0; k <= N; k++) {  // nspt.cc:586-597
-    w2[2 * k] = r[k].x / (double)(72 * ctx->V);
-    w2[2 * k + 1] = r[k].y / (double)(72 * ctx->V);
+    double re = 0.0, im = 0.0;
+    for (int mu = 0; mu < 4; mu++) {
+      re += r[2 * (mu * (N + 1) + k)];
+      im += r[2 * (mu * (N + 1) + k) + 1];
+    }
+    w2[2 * k] = re / (double)(72 * ctx->V);
+    w2[2 * k + 1] = im / (double)(72 * ctx->V);
   }
   return NSPT_OK;
 }
 
 extern "C" int nspt_plaquette_measure(nspt_ctx *ctx, double *plaq) {
   if (!ctx || !plaq) return NSPT_ERR_ARG;
-  SweepArgs a;
-  memset(&a, 0, sizeof(a));
-  a.U = ctx->U;
-  a.Uf = ctx->Uf;
-  a.obs_tr = ctx->obs_tr;
-  a.N = ctx->N;
-  a.SS = ctx->SS;
-  a.g = ctx->geo;
-  int rc = launch_sweep(ctx, a, true);
-  if (rc) return rc;
   const int N = ctx->N;
-  const long nl = 4 * ctx->V;
-  double2 *tmp = ctx->red2 + (N + 1) + 4 * N;  // MM area, free outside zero modes
-  k_rowsum<double2><<<N + 1, 256, 0, ctx->st>>>(ctx->obs_tr, (size_t)nl, nl, tmp);
+  const long units = 6L * ctx->V;
+  const Shape sh = group_shape(form_lanes(ctx, units), 4, MEASURE_SLOTS, ctx->SS, ctx->smem_optin);
+  if (sh.gpc < 1) return NSPT_ERR_ORDER;
+  const int grid = (int)std::min<long>((units + sh.gpc - 1) / sh.gpc, MEASURE_CTAS);
+  measure_form(ctx, units, [&](auto G) {
+    cudaFuncSetAttribute(k_plaq_trace<G.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)ctx->smem_optin);
+    k_plaq_trace<G.value><<<grid, 32 * sh.warps, sh.smem, ctx->st>>>(
+        ctx->U, link_rec(N), N, ctx->SS, ctx->geo, ctx->meas, N + 1, sh.gpc);
+  });
   CK(cudaGetLastError());
+  double *tmp = ctx->red + red_mm(ctx);  // free outside zero modes
+  int rc = colsum(ctx, (const double *)ctx->meas, grid, 2 * (N + 1), tmp);
+  if (rc) return rc;
   std::vector<double2> r(N + 1);
   CK(cudaMemcpyAsync(r.data(), tmp, r.size() * sizeof(double2), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
@@ -1443,21 +1362,12 @@ extern "C" int nspt_load_lower_order(nspt_ctx *ctx, const char *path, int loword
   int rc = nspt_upload_links(ctx, host.data(), N);
   if (rc) return rc;
   // U = exp(reH(log U)) per link (QCDenvNODEpt_test.h:414-417)
-  double2 *U = ctx->U, *Uf = ctx->Uf;
-  const int SS = ctx->SS;
-  const Geo geo = ctx->geo;
-  cudaStream_t st = ctx->st;
-  const bool low = use_low(ctx);
-  rc = launch_groups(
-      ctx, low ? (const void *)k_unitarise<true> : (const void *)k_unitarise<false>, 3, 4 * ctx->V,
-      [&](unsigned g, dim3 b, size_t sm) {
-        if (low)
-          k_unitarise<true><<<g, b, sm, st>>>(U, Uf, N, SS, geo);
-        else
-          k_unitarise<false><<<g, b, sm, st>>>(U, Uf, N, SS, geo);
-      },
-      "unitarise", 0, low);
+  with_form(ctx, 4 * ctx->V, [&](auto G) {
+    rc = wlaunch(ctx, G, k_unitarise<G.value>, SERIES_SLOTS, 4 * ctx->V, "unitarise", ctx->U, N,
+                 ctx->SS, ctx->geo);
+  });
   if (rc) return rc;
+  set_unit_flags(ctx, true);
   CK(cudaStreamSynchronize(ctx->st));
   ctx->have_obs = false;
   if (plaq_trailer) std::copy(trailer.begin(), trailer.end(), plaq_trailer);

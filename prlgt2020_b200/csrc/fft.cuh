@@ -18,16 +18,14 @@
 // Passes and memory:
 //   * direction t (stride 1): the lines of a CTA are one contiguous chunk,
 //     staged through shared memory (coalesced in and out, each thread then
-//     reads its own line at a padded pitch); the first forward pass computes
-//     its input, the divergence sum_mu [log U_mu(x) - log U_mu(x - mu)]
-//     (nspt.cc:871-877), on the fly instead of reading a stored field;
+//     reads its own line at a padded pitch);
 //   * directions z, y: one thread per line, consecutive threads on
 //     consecutive sites, so every load and store is coalesced;
 //   * direction x: the last forward and the first backward transform in one
 //     kernel, with the momentum-space factor -alpha / p^2 (zero at p = 0,
 //     nspt.cc:881-894) applied between them.
-// Seven passes over the 9N planes instead of ten (divergence, four forward
-// passes, the scaling, four backward passes).
+// Seven passes over the 9N planes (four forward, four backward, the two along x
+// in one), after k_fa_div has made the planes from the logarithms' records.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -191,42 +189,20 @@ __global__ void __launch_bounds__(128) k_fft_strided(double2 *data, long nlines,
 // Direction t (stride 1): the CTA's T lines are the contiguous elements
 // [g0 n, (g0 + T) n) of the planes, staged through shared memory at pitch
 // n | 1 (odd, so that the 8 lanes of a quarter-warp reading their lines'
-// element k hit distinct 16-byte bank groups).  DIV: the input is the
-// divergence of the per-link logs Lg (planes mu*9N + e), not data.
-template <int n, bool DIV>
-__global__ void __launch_bounds__(128) k_fft_t(double2 *data, const double2 *__restrict__ Lg,
-                                               long nlines, int N9, Geo geo, const double2 *tw,
+// element k hit distinct 16-byte bank groups).
+template <int n>
+__global__ void __launch_bounds__(128) k_fft_t(double2 *data, long nlines, const double2 *tw,
                                                int inv) {
   constexpr int T = 128, PITCH = n | 1;
-  extern __shared__ double2 sh[];
+  extern __shared__ double2 sm[];
   const long g0 = (long)blockIdx.x * T;
   const int lines = (int)min((long)T, nlines - g0);
   const size_t e0 = (size_t)g0 * n;
-  const size_t V = (size_t)geo.V;
-  for (int x = threadIdx.x; x < lines * n; x += T) {
-    const size_t E = e0 + x;
-    double2 val;
-    if constexpr (DIV) {
-      const size_t e = E / V;
-      const int site = (int)(E - e * V);
-      int c[4];
-      coords(geo, site, c);
-      val = cz();
-#pragma unroll
-      for (int mu = 0; mu < 4; mu++) {
-        const Nb b = neighbour(geo, c, mu, -1, 0, 0);
-        const double2 *pl = Lg + ((size_t)mu * N9 + e) * V;
-        val = cadd(val, csub(__ldg(pl + site), __ldg(pl + b.site)));
-      }
-    } else {
-      val = data[E];
-    }
-    sh[(x / n) * PITCH + (x % n)] = val;
-  }
+  for (int x = threadIdx.x; x < lines * n; x += T) sm[(x / n) * PITCH + (x % n)] = data[e0 + x];
   __syncthreads();
   if (threadIdx.x < lines) {
     double2 v[n];
-    double2 *row = sh + threadIdx.x * PITCH;
+    double2 *row = sm + threadIdx.x * PITCH;
 #pragma unroll
     for (int i = 0; i < n; i++) v[i] = row[i];
     fft_line<n>(v, tw, inv != 0);
@@ -234,7 +210,7 @@ __global__ void __launch_bounds__(128) k_fft_t(double2 *data, const double2 *__r
     for (int i = 0; i < n; i++) row[i] = v[i];
   }
   __syncthreads();
-  for (int x = threadIdx.x; x < lines * n; x += T) data[e0 + x] = sh[(x / n) * PITCH + (x % n)];
+  for (int x = threadIdx.x; x < lines * n; x += T) data[e0 + x] = sm[(x / n) * PITCH + (x % n)];
 }
 
 // Direction x (stride V / L0): forward transform, times -alpha / p^2 of the

@@ -1,38 +1,33 @@
 // kernels.cuh -- the NSPT Langevin kernels for sm_100a (FP64).
 //
-// Device layout of a link field (structure of arrays, row major colour):
-//   U[((mu*9*N + 9*(k-1) + 3*r + c) * V + site]   double2, order k = 1..N
-//   Uf[mu*V + site]                               double2 flag (order 0)
-// site = lexicographic index with t fastest (GETINDEX, lattice.h:37).
-// Consecutive sites of one (mu, order, component) plane are contiguous.
+// Device layout of a link field: one record of 1 + 9 N double2 per link,
+//   U[(4*site + mu) * (1 + 9*N)]                          flag (order 0)
+//   U[(4*site + mu) * (1 + 9*N) + 1 + 9*(k-1) + 3*r + c]  order k = 1..N
+// the reference's own order of a field (ptGluon_fld, site then mu, row major
+// colour), site = lexicographic index with t fastest (GETINDEX, lattice.h:37).
+// A kernel takes a link whole, so a link is contiguous: staging one reads 3.4
+// KB in a row at 24 orders, where planes of one component each gave 216 pieces
+// of 16 bytes, half a 32-byte sector used.  The logarithms (Lg) and the gauge
+// transformation (Gx, one record per site) are records too; only the FFT's
+// work field is planes, Wg[e * V + site], e = 9*(k-1) + 3*r + c.
 //
-// Every link update is done by one 9-lane "link group" (series.cuh); a warp
-// holds 3 groups (lanes 0-26) working on 3 consecutive sites of one mu, each
-// group with up to 3 shared-memory series slots.  Groups are independent:
-// only group-local __syncwarp is used, never a block barrier.
+// Every link update is done by a group of 9 lanes, three to a warp, or by a warp, with a few
+// shared-memory series slots (wseries.cuh); a group's work is independent of all
+// others, no kernel of the step has a block barrier.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "series.cuh"
+#include "wseries.cuh"
 
 namespace nspt {
-
-constexpr int GROUP = 9;  // lanes per link group
-constexpr int LPW = 3;    // link groups per warp
-#ifndef NSPT_MO
-#define NSPT_MO 8
-#endif
-constexpr int MO = NSPT_MO;  // result orders per lane per pass (3*MO orders)
 
 struct Geo {
   int L[4];
   int V;
   int s0, s1, s2;  // site strides of directions 0, 1, 2 (direction 3: 1)
   unsigned twist;  // bit d: direction d twisted
-  int t0, t1, t2;  // the sweep's site tiles: t0 x t1 x t2 sites in directions 0-2 (sweep_link)
 };
-
 
 // exp(-2 pi i k / 64), k < 64, radix-2 FFT twiddles.
 __constant__ double2 c_tw64[64];
@@ -54,9 +49,9 @@ struct Nb {
 // Site of x + s1*e_d1 + s2*e_d2 (s = -1, 0, +1) with periodic wrap.
 __device__ __forceinline__ Nb neighbour(const Geo &g, const int *x, int d1, int s1, int d2 = 0,
                                         int s2 = 0) {
-  int y[4] = {x[0], x[1], x[2], x[3]};
-  y[d1] += s1;
-  y[d2] += s2;
+  int y[4];  // selects, not y[d1]: an array indexed at run time lives in memory
+#pragma unroll
+  for (int d = 0; d < 4; d++) y[d] = x[d] + (d == d1 ? s1 : 0) + (d == d2 ? s2 : 0);
   Nb n;
   n.fwd = 0;
   n.bwd = 0;
@@ -74,90 +69,53 @@ __device__ __forceinline__ Nb neighbour(const Geo &g, const int *x, int d1, int 
   return n;
 }
 
-// Copy link (mu, n.site) from the row-major planes into a column-major slot
-// (DAG: store its dagger), applying the twists of the faces the read crossed.
-// Twisted links get flag 1 (twist_* returns a default flag, nspt.cc:115-121).
-// RW: the field is being updated by the same kernel -- coherent (L2) loads
-// instead of the read-only path.
-template <bool RW>
-__device__ __forceinline__ double2 ld_link(const double2 *p) {
-  return RW ? __ldcg(p) : __ldg(p);
+// double2 in the record of one link
+__host__ __device__ __forceinline__ size_t link_rec(int N) { return 1 + 9 * (size_t)N; }
+// record of link (mu, site)
+__device__ __forceinline__ size_t link_at(int mu, int site, int N) {
+  return ((size_t)site * 4 + mu) * link_rec(N);
 }
 
-template <bool RW = false>
-__device__ __forceinline__ void stage(double2 *slot, const double2 *U, const double2 *Uf, int mu,
-                                      Nb n, const Geo &g, int N, const Lane &L, bool dag = false) {
-  const size_t V = (size_t)g.V;
-  const double2 *src = U + (size_t)mu * 9 * N * V + n.site;
+// This lane's group: its index in the grid and the offset of its slots.  A CTA
+// holds gpc groups, as many as shared memory has room for (at most 32 / G per
+// warp), dealt to its warps as evenly as possible; lanes without a group, and
+// groups past the last unit, have none of the work (ok false).
+__host__ __device__ __forceinline__ int group_stride(int slots, int SS) {
+  const int n = slots * SS;
+  return n + (4 - n % 8 + 8) % 8;
+}
+template <int G>
+struct Grp {
+  int lane, slot;
+  long id;
+  bool ok;
+  __device__ __forceinline__ Grp(int slots, int SS, int gpc, long units) {
+    const int w = threadIdx.x >> 5, nw = blockDim.x >> 5, g = (threadIdx.x & 31) / glanes<G>();
+    const int base = gpc / nw, extra = gpc - base * nw;
+    const int gi = w * base + min(w, extra) + g;
+    lane = glane<G>();
+    slot = LEAD + gi * group_stride(slots, SS);
+    id = (long)blockIdx.x * gpc + gi;
+    ok = g < base + (w < extra ? 1 : 0) && id < units;
+  }
+};
+
+// Link (mu, n.site) into a slot, twisted where its read crossed a twisted
+// face.  Two or three links are begun together and waited for once.
+template <int G>
+__device__ __forceinline__ void stage_link(int slot, const double2 *U, int mu, const Nb &n, int N) {
+  wstage<G>(slot, U + link_at(mu, n.site, N), (int)link_rec(N));
+}
+template <int G>
+__device__ __forceinline__ void twist_link(int slot, const Nb &n, const Geo &g, int N) {
   const unsigned tb = n.bwd & g.twist, tf = n.fwd & g.twist;
-  if (!(tb | tf)) {
-    // lane j copies colour component j (= 3r + c) of every order
-    const int r = L.j / 3, c = L.j - 3 * (L.j / 3);
-    const int off = dag ? 3 * r + c : 3 * c + r;
-    // every order in flight at once, global -> shared without registers
-    // (cp.async.cg reads through L2, so it is coherent for RW as well); the
-    // dagger is the transposed position plus a sign flip of the imaginary
-    // parts this lane copied, once they have landed
-    for (int k = 1; k <= N; k++) {
-      const unsigned dst = (unsigned)__cvta_generic_to_shared(slot + 1 + 9 * (k - 1) + off);
-      const double2 *gp = src + (size_t)(9 * (k - 1) + L.j) * V;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gp) : "memory");
-    }
-    cp_commit();
-    cp_wait0();
-    if (dag)
-      for (int k = 1; k <= N; k++) {
-        double *im = &slot[1 + 9 * (k - 1) + off].y;
-        *im = -*im;
-      }
-    if (L.j == 0) {
-      const double2 f = ld_link<RW>(Uf + (size_t)mu * V + n.site);
-      slot[0] = dag ? cconj(f) : f;
-    }
-  } else {
-    for (int k = 1 + L.j; k <= N; k += GROUP) {
-      double2 m[9];
-#pragma unroll
-      for (int e = 0; e < 9; e++) m[e] = ld_link<RW>(src + (size_t)(9 * (k - 1) + e) * V);
-      twist3(m, tb, tf);
-      double2 *p = slot + 1 + 9 * (k - 1);
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) p[dag ? 3 * r + c : 3 * c + r] = dag ? cconj(m[3 * r + c]) : m[3 * r + c];
-    }
-    if (L.j == 0) slot[0] = make_double2(1.0, 0.0);
-  }
-  __syncwarp(L.mask);
+  if (tb | tf) wtwist<G>(slot, tb, tf, N);
 }
-
-// Copy a per-site series (planes src[e*V + site], row major) into a slot.
-__device__ __forceinline__ void stage_site(double2 *slot, const double2 *__restrict__ src, int site,
-                                           size_t V, int N, const Lane &L, double2 flag,
-                                           bool dag = false) {
-  const int r = L.j / 3, c = L.j - 3 * (L.j / 3);
-  const int off = dag ? 3 * r + c : 3 * c + r;
-  // as stage(): all orders in flight, then the dagger's sign flip
-  for (int k = 1; k <= N; k++) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(slot + 1 + 9 * (k - 1) + off);
-    const double2 *gp = src + (size_t)(9 * (k - 1) + L.j) * V + site;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gp) : "memory");
-  }
-  cp_commit();
-  cp_wait0();
-  if (dag)
-    for (int k = 1; k <= N; k++) {
-      double *im = &slot[1 + 9 * (k - 1) + off].y;
-      *im = -*im;
-    }
-  if (L.j == 0) slot[0] = dag ? cconj(flag) : flag;
-  __syncwarp(L.mask);
-}
-
-// Flag of link (mu, n): 1 after a twist, else the stored flag.
-__device__ __forceinline__ double2 link_flag(const double2 *Uf, int mu, Nb n, const Geo &g) {
-  if ((n.bwd | n.fwd) & g.twist) return make_double2(1.0, 0.0);
-  return __ldg(Uf + (size_t)mu * g.V + n.site);
+__device__ __forceinline__ Nb nb_self(int site) {
+  Nb n;
+  n.site = site;
+  n.fwd = n.bwd = 0;
+  return n;
 }
 
 // ---------------- Philox-4x32-10 (Salmon et al., SC'11) ----------------
@@ -179,20 +137,17 @@ __device__ __forceinline__ double u53(uint32_t hi, uint32_t lo) {
   const uint64_t b = ((((uint64_t)hi) << 32) | lo) >> 11;
   return ((double)b + 1.0) * (1.0 / 9007199254740992.0);
 }
-// 8 Gaussians of variance 1/2 (the reference's convention, MyRand.cc:119-127)
-__device__ __forceinline__ void philox_gauss8(uint64_t seed, uint64_t step, uint32_t link,
-                                              double *g) {
+// 8 Gaussians of variance 1/2 (the reference's convention, MyRand.cc:119-127):
+// pair q (0..3), which lane q of the link's warp draws
+__device__ __forceinline__ double2 philox_gauss_pair(uint64_t seed, uint64_t step, uint32_t link,
+                                                     int q) {
   const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    uint4 r = philox(make_uint4(link, (uint32_t)q, (uint32_t)step, (uint32_t)(step >> 32)), key);
-    const double u1 = u53(r.x, r.y), u2 = u53(r.z, r.w);
-    const double rad = sqrt(-log(u1));
-    double sn, cs;
-    sincospi(2.0 * u2, &sn, &cs);
-    g[2 * q] = rad * cs;
-    g[2 * q + 1] = rad * sn;
-  }
+  const uint4 r = philox(make_uint4(link, (uint32_t)q, (uint32_t)step, (uint32_t)(step >> 32)), key);
+  const double u1 = u53(r.x, r.y), u2 = u53(r.z, r.w);
+  const double rad = sqrt(-log(u1));
+  double sn, cs;
+  sincospi(2.0 * u2, &sn, &cs);
+  return make_double2(rad * cs, rad * sn);
 }
 
 // SU3rand mapping of 8 Gaussians to a row-major 3x3, MyMath.cc:256-292.
@@ -213,211 +168,270 @@ __device__ __forceinline__ void su3rand(const double *g, double2 *P) {
 }
 
 struct SweepArgs {
-  const double2 *U, *Uf;
-  double2 *F, *Ff;
+  const double2 *U;
+  double2 *F;
   double2 *Lg;         // log(U') per link (zero modes) or null
-  double2 *obs_tr;     // [(N+1)][4V] Tr(U * staples) per order
-  double *obs_norm;    // [N][4V]     Re Tr(U_k U_k^dag)
-  double2 *obs_tru;    // [N][4V]     Tr U_k
+  double *obs;         // per link: norm[N], then Tr U_k[N] (re, im)
+  double *obs_tr;      // traces of U * staples: plaquette path, per (site, plane) Re Tr P of
+                       // orders 0..N; link path, per link Tr (re, im) of orders 0..N
+  double *obs_tr2;     // link path: per link Tr(U * rectangle staples), improved actions
   const double *noise; // [V][4][8] injected, or null (Philox)
   uint64_t seed, step;
   const unsigned long long *stepp;  // device step counter (Philox), or null: use step
-  double2 *obs_tr2;    // [(N+1)][4V] Tr(U * rectangle staples), improved actions
   double c0, c1;       // improved action weights (Quenched.cc:311-322)
   const int *ff_scale;  // float-float products: per-order scale exponent (device)
   double tau_g, stau;  // -dt/6, sqrt(dt)  (Quenched.cc:584-589)
   int N, SS;
-  int gpc;             // link groups per CTA of the sweep, dealt to its warps as evenly
-                       // as possible (sweep_group)
   // on-the-fly update: what a read across a twisted face sees, the field of
   // the step's start (the reference's copy sites, refreshed by
   // twist_boundary only); the Jacobi sweep reads U there too
-  const double2 *Ut, *Utf;
+  const double2 *Ut;
   Geo g;
+  // plaquette path: slab of sites [site0, site0 + nsite), its plaquette records
+  // (plaq), and those of the sites from prev0 on (prev), which hold the plane
+  // before the slab
+  double2 *plaq;
+  const double2 *prev;
+  int site0, nsite, prev0;
 };
 
-// Lane identity; lanes 27..31 of a warp have no group.
-__device__ __forceinline__ bool make_lane(Lane &L, int &g) {
-  const int lane = threadIdx.x & 31;
-  g = lane / GROUP;
-  if (g >= LPW) return false;
-  L.j = lane - g * GROUP;
-  L.c = L.j / 3;
-  L.s = L.j - 3 * L.c;
-  L.mask = ((1u << GROUP) - 1u) << (g * GROUP);
-  return true;
-}
+// ---------------- shared parts of the sweeps ----------------
 
-// The sweep's CTA holds gpc link groups, dealt to its warps as evenly as
-// possible (the first gpc mod nw warps take one more): a CTA that shared
-// memory limits to, say, 22 groups runs them as 8 warps of 3 or 2 groups,
-// so that each of the SM's four schedulers has two warps, rather than as 7
-// full warps split 2-2-2-1 over the schedulers.  gi: the group's index in
-// the CTA (its slots and unit).
-__device__ __forceinline__ bool sweep_group(Lane &L, int &gi, int gpc) {
-  int g;
-  if (!make_lane(L, g)) return false;
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int base = gpc / nw, extra = gpc - base * nw;
-  if (g >= base + (warp < extra ? 1 : 0)) return false;
-  gi = warp * base + min(warp, extra) + g;
-  return true;
-}
-
-// Unit (link or site) handled by this group; clamps to the last unit.
-__device__ __forceinline__ long group_unit(int g, long nunits, bool &valid) {
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  long u = ((long)blockIdx.x * nw + warp) * LPW + g;
-  valid = u < nunits;
-  return valid ? u : nunits - 1;
-}
-
-// Link (mu, site) of the sweep's unit u.  Units run tile by tile, a tile
-// being t0 x t1 x t2 sites in directions 0, 1, 2 times the whole lines of
-// direction 3, tiles ordered with direction 2 fastest; inside a tile, all
-// its sites for mu = 0, then mu = 1, ... .  A link's staples read links at
-// +-1 in every direction.  In a plain (mu, site) order the neighbours one
-// step away in direction 0 were last read V / L0 sites earlier, far outside
-// the 126 MB L2 at large volumes; inside a tile every neighbour was read at
-// most one tile earlier, and the other mu of the tile within the tile.  The
-// link index mu V + site, which the observables and the noise counter use,
-// does not depend on the order.
-__device__ __forceinline__ void sweep_link(const Geo &g, long u, int &mu, int &site) {
-  const int L3 = g.s2;
-  const long P = (long)g.t0 * g.t1 * g.t2 * L3;  // sites per tile
-  const long tile = u / (4 * P);
-  long r = u - tile * 4 * P;
-  mu = (int)(r / P);
-  r -= (long)mu * P;
-  const int nt2 = g.L[2] / g.t2, nt1 = g.L[1] / g.t1;
-  const int tt2 = (int)(tile % nt2);
-  const long tq = tile / nt2;
-  const int tt1 = (int)(tq % nt1), tt0 = (int)(tq / nt1);
-  const int i0 = (int)(r / ((long)g.t1 * g.t2 * L3));
-  r -= (long)i0 * g.t1 * g.t2 * L3;
-  const int i1 = (int)(r / ((long)g.t2 * L3));
-  r -= (long)i1 * g.t2 * L3;
-  const int i2 = (int)(r / L3);
-  const int x3 = (int)(r - (long)i2 * L3);
-  site = (tt0 * g.t0 + i0) * g.s0 + (tt1 * g.t1 + i1) * g.s1 + (tt2 * g.t2 + i2) * g.s2 + x3;
-}
-
-// The rest of a link update once the force (nspt.cc:392-416) is in slot T and
-// U_mu(x) in slot Y, observables written: W1 = reH(W1) tau_g - stau eta,
-// F = exp(W1) U_mu(x), and the per-link log for the zero modes.  W is a
-// free slot.  Shared by the Wilson and the improved-action sweeps.
-template <int MOx = MO, bool RW = false>
-__device__ __forceinline__ void update_link(const SweepArgs &a, double2 *T, double2 *Y, double2 *W,
-                                            long link, int mu, int site, const Nb &self,
-                                            const Lane &L) {
-  const int N = a.N, c = L.c;
-  const size_t V = (size_t)a.g.V;
-  const size_t plane_mu = (size_t)9 * N * V;
-  // ---- W1 = reH(W1) * tau_g; W1.ptU[0] -= stau * SU3rand  (nspt.cc:416-423)
-  ser_reH(T, N, L);
-  {
-    double gz[8];
-    if (L.j == 0) {
-      if (a.noise) {
+// Observables of a link in slot Y (nspt.cc:393-402): Re Tr(U_k U_k^dag), Tr U_k
+template <int G>
+__device__ __forceinline__ void link_obs(const SweepArgs &a, int Y, size_t link) {
+  const double2 *sm = wsm();
+  const int N = a.N;
+  double *o = a.obs + link * 3 * N;
+  for (int k = 1 + glane<G>(); k <= N; k += glanes<G>()) {
+    const double2 *u = sm + Y + 9 * k - 8;
+    double nrm = 0.0;
 #pragma unroll
-        for (int q = 0; q < 8; q++) gz[q] = __ldg(a.noise + ((size_t)site * 4 + mu) * 8 + q);
-      } else {
-        philox_gauss8(a.seed, a.stepp ? *a.stepp : a.step, (uint32_t)link, gz);
-      }
+    for (int i = 0; i < 3; i++) {
+      double d = 0.0;
+#pragma unroll
+      for (int l = 0; l < 3; l++) d += u[3 * i + l].x * u[3 * i + l].x + u[3 * i + l].y * u[3 * i + l].y;
+      nrm += d;
     }
-    for (int k = 1 + L.j; k <= N; k += GROUP) {
-      double2 *p = T + 1 + 9 * (k - 1);
-#pragma unroll
-      for (int e = 0; e < 9; e++) p[e] = cscale(p[e], a.tau_g);
-      if (k == 1) {
-        double2 eta[9];
-        su3rand(gz, eta);
-#pragma unroll
-        for (int r = 0; r < 3; r++)
-#pragma unroll
-          for (int q = 0; q < 3; q++) p[3 * q + r] = csub(p[3 * q + r], cscale(eta[3 * r + q], a.stau));
-      }
-    }
-    if (L.j == 0) T[0] = cscale(cz(), a.tau_g);
-    __syncwarp(L.mask);
+    o[k - 1] = nrm;
+    const double2 t = cadd(cadd(u[0], u[4]), u[8]);
+    o[N + 2 * (k - 1)] = t.x;
+    o[N + 2 * (k - 1) + 1] = t.y;
   }
-  // ---- F = exp(W1) * U  (nspt.cc:429): exp into Y (W holds the square of
-  // W1), U_mu(x) restaged into W
-  ser_exp<MOx>(T, W, Y, N, L);
-  stage<RW>(W, a.U, a.Uf, mu, self, a.g, N, L);
-  const bool zm = a.Lg != nullptr;
-  double2 *Fc = a.F + (size_t)mu * plane_mu + site;
-  product<MOx, false>(LeftS{Y}, make_double2(1.0, 0.0), W, W[0], N, L,
-                     [&](int k, int r, double2 v) {
-                       Fc[(size_t)(9 * (k - 1) + 3 * r + c) * V] = v;
-                       if (zm) W[sidx(k, r, c)] = v;
-                     });
-  if (L.j == 0) a.Ff[(size_t)mu * V + site] = W[0];
-  if (!zm) return;
-  __syncwarp(L.mask);
-  // ---- MM[mu] += log(F[link])  (nspt.cc:432-439): logs stored per link
-  double2 *Lo = a.Lg + (size_t)mu * plane_mu + site;
-  ser_log<MOx>(W, T, Y, N, L, [&](int k, int r, double2 v) {
-    Lo[(size_t)(9 * (k - 1) + 3 * r + c) * V] = v;
-  });
 }
 
-// Jacobi Langevin sweep, one link per group: gauge_wilson, nspt.cc:362-439.
-// MEASURE: only the plaquette traces (plaquette_measure, nspt.cc:1362-1383).
+// Traces of orders 0..N of a slot (ptSU3::Tr, QCDpt.cc:115-122)
+template <int G>
+__device__ __forceinline__ void link_trace(double *o, int P, int N) {
+  const double2 *sm = wsm();
+  for (int k = glane<G>(); k <= N; k += glanes<G>()) {
+    const double2 *p = sm + P + 9 * k - 8;
+    const double2 f = sm[P];
+    const double2 t = k ? cadd(cadd(p[0], p[4]), p[8]) : make_double2(3. * f.x, 3. * f.y);
+    o[2 * k] = t.x;
+    o[2 * k + 1] = t.y;
+  }
+}
+
+// The rest of a link update once the force (nspt.cc:392-416) is in slot W:
+// W = reH(W) tau_g - stau eta (nspt.cc:416-423), F = exp(W) U (nspt.cc:429)
+// and the link's log for the zero modes (nspt.cc:432-439).  All slots are
+// overwritten; link = mu V + site numbers the noise.
+template <int G, bool DAG>
+__device__ __forceinline__ void update_link(const SweepArgs &a, int T, int Y, int W, int mu,
+                                            int site) {
+  double2 *sm = wsm();
+  const int N = a.N, lane = glane<G>();
+  double gz[8];
+  {
+    double2 p = cz();
+    if (lane < 4) {
+      if (a.noise) {
+        const double *e = a.noise + ((size_t)site * 4 + mu) * 8 + 2 * lane;
+        p = make_double2(__ldg(e), __ldg(e + 1));
+      } else {
+        p = philox_gauss_pair(a.seed, a.stepp ? *a.stepp : a.step,
+                              (uint32_t)((long)mu * a.g.V + site), lane);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int src = gfirst<G>() + q;
+      gz[2 * q] = __shfl_sync(gmask<G>(), p.x, src);
+      gz[2 * q + 1] = __shfl_sync(gmask<G>(), p.y, src);
+    }
+  }
+  for (int k = 1 + lane; k <= N; k += glanes<G>()) {
+    double2 *p = sm + W + 9 * k - 8;
+    double2 m[9];
+#pragma unroll
+    for (int e = 0; e < 9; e++) m[e] = p[e];
+    reh3(m);
+#pragma unroll
+    for (int e = 0; e < 9; e++) m[e] = cscale(m[e], a.tau_g);
+    if (k == 1) {
+      double2 eta[9];
+      su3rand(gz, eta);
+#pragma unroll
+      for (int e = 0; e < 9; e++) m[e] = csub(m[e], cscale(eta[e], a.stau));
+    }
+#pragma unroll
+    for (int e = 0; e < 9; e++) p[e] = m[e];
+  }
+  if (lane == 0) sm[W] = cz();
+  gsync<G>();
+  const int E = ser_exp_to<G, DAG>(W, T, Y, N);
+  const size_t at = link_at(mu, site, N);
+  wstage<G>(T, a.U + at, (int)link_rec(N));
+  wstage_wait<G>();
+  ser_mul<G>(T, E, T, N, DAG ? MUL_DAG : 0);
+  wstore<G>(a.F + at, T, (int)link_rec(N));
+  if (a.Lg) {
+    gsync<G>();
+    ser_log<G, DAG>(T, W, Y, N);
+    wstore<G>(a.Lg + at, Y, (int)link_rec(N));
+  }
+}
+
+// ---------------- Jacobi sweep, plaquette by plaquette ----------------
 //
-// Three series slots per group (T, Y, W): W holds the staple sum, then X^2
-// of the series exp; T and Y hold staged operands, products, the force and
-// the exp.  Every operand is staged by cp.async, so no left-operand ring.
-#ifndef NSPT_SWEEP_THREADS
-#define NSPT_SWEEP_THREADS 256
-#endif
-constexpr int SWEEP_THREADS = NSPT_SWEEP_THREADS;
-constexpr int SWEEP_SLOTS = 3;
+// gauge_wilson, nspt.cc:362-439.  The six staples of a link take 12 products
+// and U times their sum one more.  A plaquette x, mu < nu has four of them in
+// common with its other links: with
+//   A = U_mu(x) U_nu(x+mu),  B = U_nu(x) U_mu(x+nu),  P = A B^dag,
+// the upper staples (QCDenvNODEpt_test.h:555) give
+//   U_mu(x) [U_nu(x+mu) B^dag] = P  and  U_nu(x) [U_mu(x+nu) A^dag] = P^dag,
+// and the lower ones (QCDenvNODEpt_test.h:556) are A^dag U_nu(x) for the link
+// (mu, x+nu) and B^dag U_mu(x) for the link (nu, x+mu).  Five products per
+// plaquette, 7.5 per link, and one more for U times the sum of the three lower
+// staples: 8.5 products per link instead of 13.  All four traces of the
+// plaquette are Tr P or its conjugate.
+//
+// The three results of a plaquette (P and the two lower staples) go through
+// global memory as records, slab by slab of direction 0 (SweepArgs): 62 KB per
+// site at 24 orders, written and read once, 0.02 us per site at the HBM's rate
+// where the sweep takes 0.3.
+constexpr int PLAQ_SLOTS = 3;
 
-// Slot products shared by the sweeps' staple chains (one copy of the
-// product code each, not one per call site).
-// T <- T Y, in place
-template <int MOx = MO>
-__device__ __noinline__ void slot_mul(double2 *T, const double2 *Y, int N, const Lane &L) {
-  const double2 a0 = T[0], b0 = Y[0];
-  const int c = L.c;
-  product<MOx, false>(LeftS{T}, a0, Y, b0, N, L,
-                     [&](int k, int r, double2 v) { T[sidx(k, r, c)] = v; });
-  if (L.j == 0) T[0] = flag_mul(a0, b0);
-  __syncwarp(L.mask);
+__device__ __forceinline__ void plane_dirs(int pl, int &mu, int &nu) {
+  mu = pl < 3 ? 0 : (pl < 5 ? 1 : 2);
+  nu = pl < 3 ? pl + 1 : (pl < 5 ? pl - 1 : 3);
+}
+__device__ __forceinline__ int plane_of(int mu, int nu) {  // mu < nu
+  return mu == 0 ? nu - 1 : mu + nu;
+}
+// record q (0: P, 1: lower staple of (mu, x+nu), 2: of (nu, x+mu)) of plane pl
+// of the s-th site of a slab
+__device__ __forceinline__ size_t plaq_at(long s, int pl, int q, int N) {
+  return ((size_t)(s * 6 + pl) * 3 + q) * link_rec(N);
 }
 
-// out <- A B, orders 1..N (out may be B: the product works in place); the
-// flag is the caller's
-template <int MOx = MO>
-__device__ __noinline__ void slot_mul_to(double2 *out, const double2 *A, const double2 *B, int N,
-                                         const Lane &L) {
-  const int c = L.c;
-  product<MOx, false>(LeftS{A}, A[0], B, B[0], N, L,
-                     [&](int k, int r, double2 v) { out[sidx(k, r, c)] = v; });
-  __syncwarp(L.mask);
+template <bool FF, int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_plaq(SweepArgs a, int gpc) {
+  const Grp<G> w(PLAQ_SLOTS, a.SS, gpc, 6L * a.nsite);
+  if (!w.ok) return;
+  const int N = a.N, S0 = w.slot, S1 = S0 + a.SS, S2 = S1 + a.SS;
+  const int ffe = FF ? *a.ff_scale : 0;
+  const int s = (int)(w.id / 6), pl = (int)(w.id - 6 * (long)s), site = a.site0 + s;
+  int mu, nu, x[4];
+  plane_dirs(pl, mu, nu);
+  coords(a.g, site, x);
+  const Nb self = nb_self(site), um = neighbour(a.g, x, mu, 1), un = neighbour(a.g, x, nu, 1);
+  stage_link<G>(S0, a.U, mu, self, N);
+  stage_link<G>(S1, a.U, nu, um, N);
+  stage_link<G>(S2, a.U, nu, self, N);
+  wstage_wait<G>();
+  twist_link<G>(S1, um, a.g, N);
+  ser_mul_x<FF, G>(S1, S0, S1, N, ffe, MUL_DAG);                                  // A
+  stage_link<G>(S0, a.U, mu, un, N);
+  cp_commit();
+  ser_mul_x<FF, G>(0, S1, S2, N, ffe, MUL_DA, a.plaq + plaq_at(s, pl, 1, N));     // A^dag U_nu
+  wstage_wait<G>();
+  twist_link<G>(S0, un, a.g, N);
+  ser_mul_x<FF, G>(S2, S2, S0, N, ffe, MUL_DAG);                                  // B
+  stage_link<G>(S0, a.U, mu, self, N);
+  cp_commit();
+  ser_mul_x<FF, G>(S1, S1, S2, N, ffe, MUL_DB);                                   // P
+  wstore<G>(a.plaq + plaq_at(s, pl, 0, N), S1, (int)link_rec(N));
+  const double2 *sm = wsm();
+  double *o = a.obs_tr + ((size_t)site * 6 + pl) * (N + 1);
+  for (int k = w.lane; k <= N; k += glanes<G>()) {
+    const double2 *p = sm + S1 + 9 * k - 8;
+    o[k] = k ? p[0].x + p[4].x + p[8].x : 3. * sm[S1].x;
+  }
+  wstage_wait<G>();
+  ser_mul_x<FF, G>(0, S2, S0, N, ffe, MUL_DA, a.plaq + plaq_at(s, pl, 2, N));     // B^dag U_mu
 }
 
-// Wacc (+)= T Y; first: Wacc = T Y.  Returns the product's flag.
-template <int MOx = MO>
-__device__ __noinline__ double2 slot_acc(double2 *Wacc, const double2 *T, const double2 *Y,
-                                        bool first, int N, const Lane &L) {
-  const double2 a0 = T[0], b0 = Y[0];
-  const int c = L.c;
-  product<MOx, false>(LeftS{T}, a0, Y, b0, N, L, [&](int k, int r, double2 v) {
-    double2 &w = Wacc[sidx(k, r, c)];
-    w = first ? v : cadd(w, v);
-  });
-  __syncwarp(L.mask);
-  return flag_mul(a0, b0);
+constexpr int UPDATE_SLOTS = 3;
+
+// Second half of the Jacobi sweep, per link (mu, x): the force from the
+// plaquette records, then the update.
+template <bool FF, int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_update(SweepArgs a, int gpc) {
+  const Grp<G> w(UPDATE_SLOTS, a.SS, gpc, 4L * a.nsite);
+  if (!w.ok) return;
+  double2 *sm = wsm();
+  const int N = a.N, T = w.slot, Y = T + a.SS, W = Y + a.SS, n = (int)link_rec(N);
+  const int site = a.site0 + (int)(w.id >> 2), mu = (int)(w.id & 3);
+  int x[4];
+  coords(a.g, site, x);
+  stage_link<G>(Y, a.U, mu, nb_self(site), N);
+  cp_commit();
+  // W = the three lower staples: of the plaquette at x - nu, twisted as a
+  // whole where x - nu is across a twisted face (the product of twisted links
+  // is the twisted product)
+  const double2 *low[3];
+  unsigned crossed = 0;
+#pragma unroll
+  for (int h = 0; h < 3; h++) {
+    const int nu = h + (h >= mu ? 1 : 0), pl = mu < nu ? plane_of(mu, nu) : plane_of(nu, mu);
+    const Nb d = neighbour(a.g, x, nu, -1);
+    const int ls = d.site - a.site0;
+    const bool here = ls >= 0 && ls < a.nsite;
+    low[h] = (here ? a.plaq : a.prev) +
+             plaq_at(here ? ls : d.site - a.prev0, pl, mu < nu ? 1 : 2, N);
+    if (d.bwd & a.g.twist) crossed |= 1u << h;
+  }
+  if (!crossed) {
+    for (int e = w.lane; e < n; e += glanes<G>())
+      sm[W + e] = cadd(cadd(__ldg(low[0] + e), __ldg(low[1] + e)), __ldg(low[2] + e));
+  } else {
+#pragma unroll
+    for (int h = 0; h < 3; h++) {
+      wstage<G>(T, low[h], n);
+      wstage_wait<G>();
+      if (crossed >> h & 1) wtwist<G>(T, 1u << (h + (h >= mu ? 1 : 0)), 0u, N);
+      for (int e = w.lane; e < n; e += glanes<G>())
+        sm[W + e] = h ? cadd(sm[W + e], sm[T + e]) : sm[T + e];
+      gsync<G>();
+    }
+  }
+  cp_wait0();
+  gsync<G>();
+  link_obs<G>(a, Y, (size_t)site * 4 + mu);
+  ser_mul_x<FF, G>(W, Y, W, N, FF ? *a.ff_scale : 0, 0);
+  // the upper staples: U_mu(x) times their sum is P of the planes where mu is
+  // the first direction and P^dag where it is the second (nu < mu: h < mu)
+  const double2 *up[3];
+#pragma unroll
+  for (int h = 0; h < 3; h++) {
+    const int nu = h + (h >= mu ? 1 : 0);
+    up[h] = a.plaq + plaq_at(w.id >> 2, mu < nu ? plane_of(mu, nu) : plane_of(nu, mu), 0, N);
+  }
+  for (int e = 1 + w.lane; e < n; e += glanes<G>()) {
+    const int k9 = (e - 1) / 9 * 9, m = e - 1 - k9, et = 1 + k9 + 3 * (m % 3) + m / 3;
+    double2 v = sm[W + e];
+#pragma unroll
+    for (int h = 0; h < 3; h++)
+      v = cadd(v, h < mu ? cconj(__ldg(up[h] + et)) : __ldg(up[h] + e));
+    sm[W + e] = v;
+  }
+  gsync<G>();
+  update_link<G, false>(a, T, Y, W, mu, site);
 }
 
-// LOW: the variant for N <= 3 * MO_LOW: products with MO_LOW orders per lane
-// and pass in CTAs of at most 6 warps, two CTAs per SM (about 168
-// registers a thread), so that an SM holds 12 warps where shared memory
-// allows.
-constexpr int MO_LOW = 4;
-constexpr int SWEEP_THREADS_LOW = 192;
+// ---------------- sweeps link by link ----------------
 
 // Thread grid of the reference's OpenMP build (choices.h:124-128): n[d]
 // threads along direction d (ntt, ntx, nty, ntz), blocks of bs[d] sites
@@ -442,16 +456,20 @@ struct LgfWalk {
     b[1] = (int)((tid / ((long)gr.n[2] * gr.n[3])) % gr.n[1]);
     b[2] = (int)((tid / gr.n[3]) % gr.n[2]);
     b[3] = (int)(tid % gr.n[3]);
-    for (int d = 0; d < 4; d++) rel[d] = 0;
     long q = step;
-    for (int d = gr.dmax; d >= 0; d--) {
-      rel[d] = (int)(q % gr.bs[d]);
-      q /= gr.bs[d];
+#pragma unroll
+    for (int d = 3; d >= 0; d--) {
+      rel[d] = 0;
+      if (d <= gr.dmax) {
+        rel[d] = (int)(q % gr.bs[d]);
+        q /= gr.bs[d];
+      }
     }
   }
   // coordinates of the r-th site of the walk
   __device__ __forceinline__ void site(const LgfGrid &gr, const Geo &geo, long r, int *x) const {
     long t = r;
+#pragma unroll
     for (int d = 3; d >= 0; d--) {
       if (d <= gr.dmax) {
         x[d] = gr.bs[d] * b[d] + rel[d];
@@ -463,547 +481,326 @@ struct LgfWalk {
   }
 };
 
-// A neighbour link of the sweep into a slot.  OTF (on-the-fly update, the
-// field changing inside the kernel): coherent loads, and a read across a
-// twisted face from the step's start field.
-template <bool OTF>
-__device__ __forceinline__ void sweep_stage(double2 *slot, const SweepArgs &a, int mu, Nb n,
-                                            int N, const Lane &L, bool dag = false) {
-  if constexpr (OTF) {
-    const bool cross = ((n.fwd | n.bwd) & a.g.twist) != 0;
-    stage<true>(slot, cross ? a.Ut : a.U, cross ? a.Utf : a.Uf, mu, n, a.g, N, L, dag);
-  } else {
-    stage(slot, a.U, a.Uf, mu, n, a.g, N, L, dag);
-  }
+// A link of a chain into a slot (not waited for).  Otf (on-the-fly update):
+// a read across a twisted face comes from the step's start field.
+template <int G>
+__device__ __forceinline__ void chain_stage(const SweepArgs &a, int slot, int d, const Nb &n) {
+  const bool cross = ((n.fwd | n.bwd) & a.g.twist) != 0;
+  stage_link<G>(slot, cross ? a.Ut : a.U, d, n, a.N);
 }
 
-// The rest of a link update once the staple sum is in slot W (flag wflag):
-// P = U W into T with U in Y, the traces, then update_link.
-template <bool MEASURE, bool FF, bool LOW, bool OTF>
-__device__ __forceinline__ void sweep_tail(const SweepArgs &a, const Lane &L, double2 *T,
-                                           double2 *Y, double2 *W, int mu, int site,
-                                           double2 wflag) {
-  constexpr int MOK = LOW ? MO_LOW : MO;
-  const int ffe = FF ? *a.ff_scale : 0;
-  const int N = a.N, c = L.c;
-  const size_t V = (size_t)a.g.V;
-  const long link = (long)mu * a.g.V + site;
-  Nb self;
-  self.site = site;
-  self.fwd = self.bwd = 0;
-  if (L.j == 0) W[0] = wflag;
-  // ---- P = U_mu(x) * staples (nspt.cc:392) into T; U_mu(x) in Y
-  sweep_stage<OTF>(Y, a, mu, self, N, L);
-  const double2 pflag = flag_mul(Y[0], wflag);
-  cprod<FF, MOK, false>(LeftS{Y}, Y[0], W, wflag, N, L, ffe,
-                     [&](int k, int r, double2 v) { T[sidx(k, r, c)] = v; });
-  if (L.j == 0) T[0] = pflag;
-  __syncwarp(L.mask);
-  // ---- traces (ptSU3::Tr, QCDpt.cc:115-122), norm and Tr U_k (nspt.cc:393-402)
-  {
-    const size_t nl4 = 4 * V;
-    if (L.j == 0) a.obs_tr[link] = make_double2(3. * pflag.x, 3. * pflag.y);
-    for (int k = 1 + L.j; k <= N; k += GROUP) {
-      a.obs_tr[(size_t)k * nl4 + link] =
-          cadd(cadd(T[sidx(k, 0, 0)], T[sidx(k, 1, 1)]), T[sidx(k, 2, 2)]);
-      if constexpr (!MEASURE) {
-        double nrm = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          double d = 0.0;
-#pragma unroll
-          for (int l = 0; l < 3; l++) {
-            const double2 u = Y[sidx(k, i, l)];
-            d += u.x * u.x + u.y * u.y;
-          }
-          nrm += d;
-        }
-        a.obs_norm[(size_t)(k - 1) * nl4 + link] = nrm;
-        a.obs_tru[(size_t)(k - 1) * nl4 + link] =
-            cadd(cadd(Y[sidx(k, 0, 0)], Y[sidx(k, 1, 1)]), Y[sidx(k, 2, 2)]);
-      }
-    }
-  }
-  if constexpr (MEASURE) return;
-  __syncwarp(L.mask);
-  update_link<MOK, OTF>(a, T, Y, W, link, mu, site, self, L);
-}
-
-// The update of link (mu, site) by one group: staples, force, observables,
-// noise, exp, the new link into a.F (a.U itself on the fly) and its log.
-template <bool MEASURE, bool FF, bool LOW, bool OTF>
-__device__ __forceinline__ void sweep_one(const SweepArgs &a, const Lane &L, double2 *T,
-                                          double2 *Y, double2 *W, int mu, int site) {
-  constexpr int MOK = LOW ? MO_LOW : MO;
-  const int ffe = FF ? *a.ff_scale : 0;
-  const int N = a.N, c = L.c;
+// Wilson update of link (mu, site) by its six staples: each as its chain of
+// links, multiplied left to right in T with the third link in Y, daggers taken
+// by the product:
+//   upper U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag          (QCDenvNODEpt_test.h:555)
+//   lower U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_nu(x-nu)    (QCDenvNODEpt_test.h:556)
+// For the on-the-fly update, whose links must be visited in order, and for
+// fields with flags other than 1 across twisted faces.
+template <bool FF, int G>
+__device__ __forceinline__ void link_one(const SweepArgs &a, int T, int Y, int W, int mu,
+                                         int site) {
+  const int N = a.N, ffe = FF ? *a.ff_scale : 0;
   int x[4];
   coords(a.g, site, x);
-
-  double2 wflag = cz();
-  bool first = true;
-  // A <- A B in place; W (+)= A B.  FP64: one out-of-line copy each;
-  // float-float: the compensated product inline.
-  auto mul = [&](double2 *A, const double2 *B) {
-    if constexpr (FF) {
-      const double2 a0 = A[0], b0 = B[0];
-      cprod<FF, MO, false>(LeftS{A}, a0, B, b0, N, L, ffe,
-                           [&](int k, int r, double2 v) { A[sidx(k, r, c)] = v; });
-      if (L.j == 0) A[0] = flag_mul(a0, b0);
-      __syncwarp(L.mask);
-    } else {
-      slot_mul<MOK>(A, B, N, L);
-    }
-  };
-  auto acc = [&](const double2 *A, const double2 *B) {
-    double2 f;
-    if constexpr (FF) {
-      const double2 a0 = A[0], b0 = B[0];
-      const bool f0 = first;
-      cprod<FF, MO, false>(LeftS{A}, a0, B, b0, N, L, ffe, [&](int k, int r, double2 v) {
-        double2 &w = W[sidx(k, r, c)];
-        w = f0 ? v : cadd(w, v);
-      });
-      __syncwarp(L.mask);
-      f = flag_mul(a0, b0);
-    } else {
-      f = slot_acc<MOK>(W, A, B, first, N, L);
-    }
-    wflag = first ? f : cadd(wflag, f);
-    first = false;
-  };
-  Nb self;
-  self.site = site;
-  self.fwd = self.bwd = 0;
-  for (int nu = 0; nu < 4; nu++) {
-    if (nu == mu) continue;
-    // Each staple as its chain of links, multiplied left to right in T with
-    // the next link staged into Y (the truncated product is associative):
-    // upper U_nu(x+mu) [U_nu(x) U_mu(x+nu)]^dag
-    //     = U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag      (QCDenvNODEpt_test.h:555),
-    // lower [U_mu(x-nu) U_nu(x-nu+mu)]^dag U_nu(x-nu)
-    //     = U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_nu(x-nu)  (QCDenvNODEpt_test.h:556).
-    // Links that cross a twisted face are staged twisted.
-    {
-      const Nb m = neighbour(a.g, x, mu, 1);
-      const Nb b = neighbour(a.g, x, nu, 1);
-      sweep_stage<OTF>(T, a, nu, m, N, L);
-      sweep_stage<OTF>(Y, a, mu, b, N, L, true);
-      mul(T, Y);
-      sweep_stage<OTF>(Y, a, nu, self, N, L, true);
-      acc(T, Y);
-    }
-    {
-      const Nb d = neighbour(a.g, x, nu, -1);
-      const Nb dm = neighbour(a.g, x, nu, -1, mu, 1);
-      sweep_stage<OTF>(T, a, nu, dm, N, L, true);
-      sweep_stage<OTF>(Y, a, mu, d, N, L, true);
-      mul(T, Y);
-      sweep_stage<OTF>(Y, a, nu, d, N, L);
-      acc(T, Y);
-    }
+  const Nb self = nb_self(site);
+#pragma unroll 1
+  for (int h = 0; h < 6; h++) {
+    const int q = h >> 1, nu = q + (q >= mu ? 1 : 0);
+    const bool up = !(h & 1);
+    const Nb l0 = up ? neighbour(a.g, x, mu, 1) : neighbour(a.g, x, nu, -1, mu, 1);
+    const Nb l1 = neighbour(a.g, x, nu, up ? 1 : -1);
+    chain_stage<G>(a, T, nu, l0);
+    chain_stage<G>(a, Y, mu, l1);
+    wstage_wait<G>();
+    twist_link<G>(T, l0, a.g, N);
+    twist_link<G>(Y, l1, a.g, N);
+    ser_mul_x<FF, G>(T, T, Y, N, ffe, up ? MUL_DB : MUL_DA | MUL_DB);
+    const Nb l2 = up ? self : l1;
+    chain_stage<G>(a, Y, nu, l2);
+    wstage_wait<G>();
+    twist_link<G>(Y, l2, a.g, N);
+    ser_mul_x<FF, G>(W, T, Y, N, ffe, (up ? MUL_DB : MUL_DAG) | (h ? MUL_ACC : 0));
   }
-  sweep_tail<MEASURE, FF, LOW, OTF>(a, L, T, Y, W, mu, site, wflag);
+  chain_stage<G>(a, Y, mu, self);
+  wstage_wait<G>();
+  const size_t link = (size_t)site * 4 + mu;
+  link_obs<G>(a, Y, link);
+  ser_mul_x<FF, G>(W, Y, W, N, ffe, MUL_DAG);
+  link_trace<G>(a.obs_tr + link * 2 * (N + 1), W, N);
+  gsync<G>();
+  update_link<G, true>(a, T, Y, W, mu, site);
 }
 
-template <bool MEASURE, bool FF = false, bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : SWEEP_THREADS, LOW ? 2 : 1)
-    k_sweep(SweepArgs a) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int gi;
-  if (!sweep_group(L, gi, a.gpc)) return;
-  const int SS = a.SS;
-  double2 *T = sm + (size_t)gi * (SWEEP_SLOTS * SS), *Y = T + SS;
-  double2 *W = Y + SS;
-  const long unit = (long)blockIdx.x * a.gpc + gi;
-  if (unit >= 4L * a.g.V) return;  // groups are independent: a group past the end has no work
-  int mu, site;
-  sweep_link(a.g, unit, mu, site);
-  sweep_one<MEASURE, FF, LOW, false>(a, L, T, Y, W, mu, site);
-}
+constexpr int LINK_SLOTS = 3;
 
-// gauge_wilson on the fly, for a thread grid whose threads own one site per
-// barrier step (every direction up to the last split one is split: the
-// default grid of blocks of 2): link mu of each thread's site for barrier
-// step `step`, one launch per (step, mu) in that order, the update inline
-// as in k_sweep.
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : SWEEP_THREADS, LOW ? 2 : 1)
-    k_sweep_otf1(SweepArgs a, LgfGrid gr, long step, int mu) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int gi;
-  if (!sweep_group(L, gi, a.gpc)) return;
-  const int SS = a.SS;
-  double2 *T = sm + (size_t)gi * (SWEEP_SLOTS * SS), *Y = T + SS;
-  double2 *W = Y + SS;
-  const long tid = (long)blockIdx.x * a.gpc + gi;
-  if (tid >= gr.nthr) return;
-  int x[4];
-  LgfWalk(gr, tid, step).site(gr, a.g, 0, x);
-  const int site = x[0] * a.g.s0 + x[1] * a.g.s1 + x[2] * a.g.s2 + x[3];
-  sweep_one<false, false, LOW, true>(a, L, T, Y, W, mu, site);
-}
-
-// k_sweep_otf1 with a warp of three groups per reference thread, for barrier
-// steps with too few threads to fill the GPU (the 12^4 lattice's 6^4
-// threads): group g forms the upper and lower staples of the g-th plane
-// (nu != mu, ascending) into its own sum, the team adds the three plane sums
-// in plane order, as the reference's W1 += staple(nu) (nspt.cc:381-388),
-// and group 0 finishes the link.  Three slots per group.
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : SWEEP_THREADS, LOW ? 2 : 1)
-    k_sweep_otf1_team(SweepArgs a, LgfGrid gr, long step, int mu) {
-  constexpr int MOK = LOW ? MO_LOW : MO;
-  constexpr int TEAM = LPW * GROUP;
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const long tid = (long)blockIdx.x * nw + warp;
-  if (tid >= gr.nthr) return;
-  const int SS = a.SS, N = a.N;
-  const unsigned tmask = (1u << TEAM) - 1u;
-  double2 *base = sm + (size_t)warp * (LPW * SWEEP_SLOTS) * SS;
-  double2 *T = base + (size_t)g * SWEEP_SLOTS * SS, *Y = T + SS, *W = Y + SS;
-  int x[4];
-  LgfWalk(gr, tid, step).site(gr, a.g, 0, x);
-  const int site = x[0] * a.g.s0 + x[1] * a.g.s1 + x[2] * a.g.s2 + x[3];
-  const int nu = g + (g >= mu ? 1 : 0);  // the g-th direction other than mu
-  Nb self;
-  self.site = site;
-  self.fwd = self.bwd = 0;
-  double2 wflag;
-  {  // upper U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag
-    const Nb m = neighbour(a.g, x, mu, 1);
-    const Nb b = neighbour(a.g, x, nu, 1);
-    sweep_stage<true>(T, a, nu, m, N, L);
-    sweep_stage<true>(Y, a, mu, b, N, L, true);
-    slot_mul<MOK>(T, Y, N, L);
-    sweep_stage<true>(Y, a, nu, self, N, L, true);
-    wflag = slot_acc<MOK>(W, T, Y, true, N, L);
-  }
-  {  // lower U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_nu(x-nu)
-    const Nb d = neighbour(a.g, x, nu, -1);
-    const Nb dm = neighbour(a.g, x, nu, -1, mu, 1);
-    sweep_stage<true>(T, a, nu, dm, N, L, true);
-    sweep_stage<true>(Y, a, mu, d, N, L, true);
-    slot_mul<MOK>(T, Y, N, L);
-    sweep_stage<true>(Y, a, nu, d, N, L);
-    wflag = cadd(wflag, slot_acc<MOK>(W, T, Y, false, N, L));
-  }
-  if (L.j == 0) W[0] = wflag;
-  __syncwarp(tmask);
-  double2 *W0 = base + 2 * SS, *W1 = W0 + SWEEP_SLOTS * SS, *W2 = W1 + SWEEP_SLOTS * SS;
-  for (int e = g * GROUP + L.j; e < 1 + 9 * N; e += TEAM) W0[e] = cadd(cadd(W0[e], W1[e]), W2[e]);
-  __syncwarp(tmask);
-  if (g == 0) sweep_tail<false, false, LOW, true>(a, L, T, Y, W, mu, site, W[0]);
-}
-
-// One on-the-fly link update, out of line: the walk's state stays outside
-// the update's registers.
-template <bool LOW>
-__device__ __noinline__ void sweep_one_otf(const SweepArgs &a, const Lane &L, double2 *T,
-                                           double2 *Y, double2 *W, int mu, int site) {
-  sweep_one<false, false, LOW, true>(a, L, T, Y, W, mu, site);
+template <bool FF, int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_link(SweepArgs a, int gpc) {
+  const Grp<G> w(LINK_SLOTS, a.SS, gpc, 4L * a.g.V);
+  if (!w.ok) return;
+  link_one<FF, G>(a, w.slot, w.slot + a.SS, w.slot + 2 * a.SS, (int)(w.id & 3), (int)(w.id >> 2));
 }
 
 // gauge_wilson with UPDATE_ONTHEFLY, the reference's default (choices.h:61,
-// nspt.cc:355-460): one barrier step of its OpenMP thread grid.  One group
-// per reference thread walks that thread's sites (LgfWalk) and updates
-// their links in place, mu = 0..3, each seeing the links updated before it;
-// the threads of one barrier step touch disjoint links.  Reads across a
-// twisted face come from a.Ut (the step's start field).
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : SWEEP_THREADS, LOW ? 2 : 1)
-    k_sweep_otf(SweepArgs a, LgfGrid gr, long step) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int gi;
-  if (!sweep_group(L, gi, a.gpc)) return;
-  const int SS = a.SS;
-  double2 *T = sm + (size_t)gi * (SWEEP_SLOTS * SS), *Y = T + SS;
-  double2 *W = Y + SS;
-  const long tid = (long)blockIdx.x * a.gpc + gi;
-  if (tid >= gr.nthr) return;
-  const LgfWalk walk(gr, tid, step);
+// nspt.cc:355-460): one barrier step of its OpenMP thread grid.  One group per
+// reference thread walks that thread's sites (LgfWalk) and updates their links
+// in place, mu = 0..3, each seeing the links updated before it; the threads of
+// one barrier step touch disjoint links.
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_otf(SweepArgs a, LgfGrid gr, long step, int gpc) {
+  const Grp<G> w(LINK_SLOTS, a.SS, gpc, gr.nthr);
+  if (!w.ok) return;
+  const LgfWalk walk(gr, w.id, step);
 #pragma unroll 1
-  for (long r = 0; r < gr.seg; r++) {
+  for (long r = 0; r < 4 * gr.seg; r++) {
     int x[4];
-    walk.site(gr, a.g, r, x);
+    walk.site(gr, a.g, r >> 2, x);
     const int site = x[0] * a.g.s0 + x[1] * a.g.s1 + x[2] * a.g.s2 + x[3];
-#pragma unroll 1
-    for (int mu = 0; mu < 4; mu++) {
-      sweep_one_otf<LOW>(a, L, T, Y, W, mu, site);
-      // the next link's stagings read what this one wrote
-      __syncwarp(L.mask);
-    }
+    link_one<false, G>(a, w.slot, w.slot + a.SS, w.slot + 2 * a.SS, (int)(r & 3), site);
+    // the next link's copies read what this one wrote
+    __threadfence();
+    gsync<G>();
   }
 }
 
 // ---------------- improved gauge actions ----------------
 
-// Jacobi sweep with an improved gauge action (TLSYM, IWA, DBW2; periodic
-// boundaries): gauge_wilson, nspt.cc:272-308.  Besides the Wilson staples W,
-// the six 2x1 rectangles of staple2x1 (QCDenvNODEpt_test.h:579-611) per
-// plane go to W2; the force is c0 U W + c1 U W2, and Tr(U W2) is the w2
-// observable.  Every staple is a chain of links (daggered where the
-// reference takes a dagger of a path: dag(A B C) = C^dag B^dag A^dag),
-// multiplied left to right in the work slot T while the next link is staged
-// into Y: four products per rectangle, as the reference's, associated the
-// other way (the truncated product is associative).  Four slots per group:
-// T, Y (work), W, W2 (sums).
+// Sweep with an improved gauge action (TLSYM, IWA, DBW2; periodic boundaries):
+// gauge_wilson, nspt.cc:272-308.  Besides the Wilson staples W, the six 2x1
+// rectangles of staple2x1 (QCDenvNODEpt_test.h:579-611) per plane go to W2; the
+// force is c0 U W + c1 U W2, and Tr(U W2) is the w2 observable.  Every staple
+// is a chain of links (daggered where the reference takes a dagger of a path:
+// dag(A B C) = C^dag B^dag A^dag), multiplied left to right in T.
+//
+// The chains of a plane as a table: link (direction m: mu, n: nu; offsets
+// along mu and nu; dagger) and what follows its product: nothing, the sum W,
+// or the sum W2.  Two rectangles begin with a Wilson staple's first two links,
+// whose product serves both:
+//   upper U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag, and
+//   U_nu(x+mu) U_mu(x+nu)^dag U_mu(x-mu+nu)^dag U_nu(x-mu)^dag U_mu(x-mu);
+//   lower U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_nu(x-nu), and
+//   U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_mu(x-mu-nu)^dag U_nu(x-mu-nu) U_mu(x-mu).
 constexpr int IMP_SLOTS = 4;
-
-// One link of a staple chain: direction, site and whether it is daggered.
-struct ImpLink {
-  int d, site;
-  bool dag;
+struct ImpStep {
+  signed char start, is_nu, i, j, dag, sum;  // sum: 0 T *= link, 1 W += T link, 2 W2 += T link
 };
+constexpr int IMP_STEPS = 32;
+__constant__ ImpStep c_imp[IMP_STEPS] = {
+    {1, 1, 1, 0, 0, 0},   {0, 0, 0, 1, 1, 0},   {0, 1, 0, 0, 1, 1},  // upper Wilson
+    {0, 0, -1, 1, 1, 0},  {0, 1, -1, 0, 1, 0},  {0, 0, -1, 0, 0, 2},
+    {1, 1, 1, -1, 1, 0},  {0, 0, 0, -1, 1, 0},  {0, 1, 0, -1, 0, 1},  // lower Wilson
+    {0, 0, -1, -1, 1, 0}, {0, 1, -1, -1, 0, 0}, {0, 0, -1, 0, 0, 2},
+    {1, 1, 1, 0, 0, 0},   {0, 1, 1, 1, 0, 0},   {0, 0, 0, 2, 1, 0},
+    {0, 1, 0, 1, 1, 0},   {0, 1, 0, 0, 1, 2},
+    {1, 0, 1, 0, 0, 0},   {0, 1, 2, 0, 0, 0},   {0, 0, 1, 1, 1, 0},
+    {0, 0, 0, 1, 1, 0},   {0, 1, 0, 0, 1, 2},
+    {1, 1, 1, -1, 1, 0},  {0, 1, 1, -2, 1, 0},  {0, 0, 0, -2, 1, 0},
+    {0, 1, 0, -2, 0, 0},  {0, 1, 0, -1, 0, 2},
+    {1, 0, 1, 0, 0, 0},   {0, 1, 2, -1, 1, 0},  {0, 0, 1, -1, 1, 0},
+    {0, 0, 0, -1, 1, 0},  {0, 1, 0, -1, 0, 2}};
 
-template <bool RW = false>
-__device__ __forceinline__ void imp_stage(const SweepArgs &a, double2 *slot, const ImpLink &l,
-                                          const Lane &L) {
-  Nb n;
-  n.site = l.site;
-  n.fwd = n.bwd = 0;
-  stage<RW>(slot, a.U, a.Uf, l.d, n, a.g, a.N, L, l.dag);
-}
-
-// Wacc (+)= l[0] l[1] ... l[n-1]; returns the flag of the chain
-template <int NL, int MOx = MO, bool RW = false>
-__device__ __forceinline__ double2 imp_chain(const SweepArgs &a, double2 *T, double2 *Y,
-                                             double2 *Wacc, const ImpLink (&l)[NL], bool first,
-                                             const Lane &L) {
-  imp_stage<RW>(a, T, l[0], L);
-#pragma unroll
-  for (int m = 1; m < NL - 1; m++) {
-    imp_stage<RW>(a, Y, l[m], L);
-    slot_mul<MOx>(T, Y, a.N, L);
-  }
-  imp_stage<RW>(a, Y, l[NL - 1], L);
-  return slot_acc<MOx>(Wacc, T, Y, first, a.N, L);
-}
-
-// The improved-action update of link (mu, site) by one group (slots T, Y,
-// W, W2); OTF: in place (a.F = a.U), coherent loads.
-template <bool LOW, bool OTF>
-__device__ __forceinline__ void imp_one(const SweepArgs &a, const Lane &L, double2 *T,
-                                        double2 *Y, double2 *W, double2 *W2, int mu, int site) {
-  constexpr int MOK = LOW ? MO_LOW : MO;
-  const int N = a.N;
-  const size_t V = (size_t)a.g.V;
-  const long link = (long)mu * a.g.V + site;
+template <int G>
+__device__ __forceinline__ void imp_one(const SweepArgs &a, int T, int Y, int W, int W2, int mu,
+                                        int site) {
+  double2 *sm = wsm();
+  const int N = a.N, lane = glane<G>(), n = (int)link_rec(N);
   int x[4];
   coords(a.g, site, x);
-
-  // site x + i mu + j nu (periodic)
-  int nu = 0;
-  auto at = [&](int i, int j) {
+  bool dag0 = false;  // T still holds the chain's first link as stored, daggered or not
+#pragma unroll 1
+  for (int h = 0; h < 3 * IMP_STEPS; h++) {
+    const int p = h / IMP_STEPS, nu = p + (p >= mu ? 1 : 0);
+    const ImpStep st = c_imp[h - p * IMP_STEPS];
     int y[4] = {x[0], x[1], x[2], x[3]};
-    y[mu] = ((y[mu] + i) % a.g.L[mu] + a.g.L[mu]) % a.g.L[mu];
-    y[nu] = ((y[nu] + j) % a.g.L[nu] + a.g.L[nu]) % a.g.L[nu];
-    return y[0] * a.g.s0 + y[1] * a.g.s1 + y[2] * a.g.s2 + y[3];
-  };
-  double2 wflag = cz(), w2flag = cz();
-  bool first = true, first2 = true;
-  auto acc = [&](double2 f) {
-    wflag = first ? f : cadd(wflag, f);
-    first = false;
-  };
-  auto acc2 = [&](double2 f) {
-    w2flag = first2 ? f : cadd(w2flag, f);
-    first2 = false;
-  };
-  for (nu = 0; nu < 4; nu++) {
-    if (nu == mu) continue;
-    const int m = mu, n = nu;
-    auto st = [&](double2 *slot, int d, int st_site, bool dag) {
-      imp_stage<OTF>(a, slot, ImpLink{d, st_site, dag}, L);
-    };
-    // ---- Wilson staples (QCDenvNODEpt_test.h:554-557) and the two
-    // rectangles that begin with a Wilson staple's first two links, which
-    // are formed once for both:
-    //   upper U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag, and
-    //   U_nu(a) dag(U_nu(f) U_mu(g) U_mu(c)) U_mu(f)
-    //     = U_nu(a) U_mu(c)^dag U_mu(g)^dag U_nu(f)^dag U_mu(f),
-    //     a=x+mu c=x+nu f=x-mu g=x-mu+nu;
-    //   lower U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_nu(x-nu), and
-    //   dag(U_mu(g) U_mu(c) U_nu(b)) U_nu(g) U_mu(h)
-    //     = U_nu(b)^dag U_mu(c)^dag U_mu(g)^dag U_nu(g) U_mu(h),
-    //     b=x+mu-nu c=x-nu g=x-mu-nu h=x-mu
-    {
-      st(T, n, at(1, 0), false);
-      st(Y, m, at(0, 1), true);
-      slot_mul<MOK>(T, Y, N, L);
-      st(Y, n, site, true);
-      acc(slot_acc<MOK>(W, T, Y, first, N, L));
-      st(Y, m, at(-1, 1), true);
-      slot_mul<MOK>(T, Y, N, L);
-      st(Y, n, at(-1, 0), true);
-      slot_mul<MOK>(T, Y, N, L);
-      st(Y, m, at(-1, 0), false);
-      acc2(slot_acc<MOK>(W2, T, Y, first2, N, L));
-    }
-    {
-      st(T, n, at(1, -1), true);
-      st(Y, m, at(0, -1), true);
-      slot_mul<MOK>(T, Y, N, L);
-      st(Y, n, at(0, -1), false);
-      acc(slot_acc<MOK>(W, T, Y, first, N, L));
-      st(Y, m, at(-1, -1), true);
-      slot_mul<MOK>(T, Y, N, L);
-      st(Y, n, at(-1, -1), false);
-      slot_mul<MOK>(T, Y, N, L);
-      st(Y, m, at(-1, 0), false);
-      acc2(slot_acc<MOK>(W2, T, Y, first2, N, L));
-    }
-    // ---- the other four rectangles of staple2x1, each its chain of five links
-    {
-      // U_nu(a) U_nu(b) dag(U_nu(x) U_nu(c) U_mu(d)),  a=x+mu b=x+mu+nu c=x+nu d=x+2nu
-      const ImpLink r1[5] = {{n, at(1, 0), false}, {n, at(1, 1), false}, {m, at(0, 2), true},
-                             {n, at(0, 1), true}, {n, site, true}};
-      acc2(imp_chain<5, MOK, OTF>(a, T, Y, W2, r1, first2, L));
-      // U_mu(a) U_nu(e) dag(U_nu(x) U_mu(c) U_mu(b)),  e=x+2mu
-      const ImpLink r2[5] = {{m, at(1, 0), false}, {n, at(2, 0), false}, {m, at(1, 1), true},
-                             {m, at(0, 1), true}, {n, site, true}};
-      acc2(imp_chain<5, MOK, OTF>(a, T, Y, W2, r2, first2, L));
-      // dag(U_mu(d) U_nu(e) U_nu(b)) U_nu(d) U_nu(c),
-      // b=x+mu-nu c=x-nu d=x-2nu e=x+mu-2nu
-      const ImpLink r4[5] = {{n, at(1, -1), true}, {n, at(1, -2), true}, {m, at(0, -2), true},
-                             {n, at(0, -2), false}, {n, at(0, -1), false}};
-      acc2(imp_chain<5, MOK, OTF>(a, T, Y, W2, r4, first2, L));
-      // U_mu(a) dag(U_mu(c) U_mu(b) U_nu(f)) U_nu(c),  f=x+2mu-nu
-      const ImpLink r5[5] = {{m, at(1, 0), false}, {n, at(2, -1), true}, {m, at(1, -1), true},
-                             {m, at(0, -1), true}, {n, at(0, -1), false}};
-      acc2(imp_chain<5, MOK, OTF>(a, T, Y, W2, r5, first2, L));
-    }
-  }
-  if (L.j == 0) {
-    W[0] = wflag;
-    W2[0] = w2flag;
-  }
-  __syncwarp(L.mask);
-  // ---- U W into T and U W2 into W2 in place (nspt.cc:286-303), traces,
-  // force c0 U W + c1 U W2
-  Nb self;
-  self.site = site;
-  self.fwd = self.bwd = 0;
-  stage<OTF>(Y, a.U, a.Uf, mu, self, a.g, N, L);
-  const double2 pflag = flag_mul(Y[0], wflag), p2flag = flag_mul(Y[0], w2flag);
-  slot_mul_to<MOK>(T, Y, W, N, L);
-  slot_mul_to<MOK>(W2, Y, W2, N, L);
-  if (L.j == 0) {
-    T[0] = pflag;
-    W2[0] = p2flag;
-  }
-  __syncwarp(L.mask);
-  {
-    const size_t nl4 = 4 * V;
-    if (L.j == 0) {
-      a.obs_tr[link] = make_double2(3. * pflag.x, 3. * pflag.y);
-      a.obs_tr2[link] = make_double2(3. * p2flag.x, 3. * p2flag.y);
-    }
-    for (int k = 1 + L.j; k <= N; k += GROUP) {
-      a.obs_tr[(size_t)k * nl4 + link] =
-          cadd(cadd(T[sidx(k, 0, 0)], T[sidx(k, 1, 1)]), T[sidx(k, 2, 2)]);
-      a.obs_tr2[(size_t)k * nl4 + link] =
-          cadd(cadd(W2[sidx(k, 0, 0)], W2[sidx(k, 1, 1)]), W2[sidx(k, 2, 2)]);
-      double nrm = 0.0;
 #pragma unroll
-      for (int i = 0; i < 3; i++) {
-        double d = 0.0;
-#pragma unroll
-        for (int l = 0; l < 3; l++) {
-          const double2 u = Y[sidx(k, i, l)];
-          d += u.x * u.x + u.y * u.y;
-        }
-        nrm += d;
-      }
-      a.obs_norm[(size_t)(k - 1) * nl4 + link] = nrm;
-      a.obs_tru[(size_t)(k - 1) * nl4 + link] =
-          cadd(cadd(Y[sidx(k, 0, 0)], Y[sidx(k, 1, 1)]), Y[sidx(k, 2, 2)]);
+    for (int d = 0; d < 4; d++) {
+      y[d] += (d == mu ? st.i : 0) + (d == nu ? st.j : 0);
+      y[d] = ((y[d] % a.g.L[d]) + a.g.L[d]) % a.g.L[d];
+    }
+    const int at = y[0] * a.g.s0 + y[1] * a.g.s1 + y[2] * a.g.s2 + y[3];
+    const int slot = st.start ? T : Y;
+    wstage<G>(slot, a.U + link_at(st.is_nu ? nu : mu, at, N), n);
+    if (st.start) {  // waited for with the second link
+      dag0 = st.dag != 0;
+      continue;
+    }
+    wstage_wait<G>();
+    const unsigned mode = MUL_DAG | (dag0 ? MUL_DA : 0) | (st.dag ? MUL_DB : 0);
+    if (st.sum == 0) {
+      ser_mul<G>(T, T, Y, N, mode);
+      dag0 = false;
+    } else {
+      // a plane's first term of each sum is the third and the sixth step
+      const bool first = p == 0 && (h == 2 || h == 5);
+      ser_mul<G>(st.sum == 1 ? W : W2, T, Y, N, mode | (first ? 0 : MUL_ACC));
     }
   }
-  __syncwarp(L.mask);
-  // W1 = c0 W1 + c1 W2 (ptSU3 operator*(double) and +, flags included)
-  for (int e = L.j; e < 1 + 9 * N; e += GROUP)
-    T[e] = cadd(cscale(T[e], a.c0), cscale(W2[e], a.c1));
-  __syncwarp(L.mask);
-  update_link<MOK, OTF>(a, T, Y, W, link, mu, site, self, L);
+  // U W and U W2 (nspt.cc:286-303), traces, force c0 U W + c1 U W2
+  wstage<G>(Y, a.U + link_at(mu, site, N), n);
+  wstage_wait<G>();
+  const size_t link = (size_t)site * 4 + mu;
+  link_obs<G>(a, Y, link);
+  ser_mul<G>(W, Y, W, N, MUL_DAG);
+  ser_mul<G>(W2, Y, W2, N, MUL_DAG);
+  link_trace<G>(a.obs_tr + link * 2 * (N + 1), W, N);
+  link_trace<G>(a.obs_tr2 + link * 2 * (N + 1), W2, N);
+  gsync<G>();
+  for (int e = lane; e < n; e += glanes<G>()) sm[W + e] = cadd(cscale(sm[W + e], a.c0), cscale(sm[W2 + e], a.c1));
+  gsync<G>();
+  update_link<G, true>(a, T, Y, W, mu, site);
 }
 
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_sweep_imp(SweepArgs a) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5;
-  const int SS = a.SS;
-  double2 *T = sm + (size_t)(warp * LPW + g) * (IMP_SLOTS * SS), *Y = T + SS;
-  double2 *W = Y + SS, *W2 = W + SS;
-  bool valid;
-  const long link = group_unit(g, 4L * a.g.V, valid);
-  if (!valid) return;
-  const int mu = (int)(link / a.g.V);
-  const int site = (int)(link - (long)mu * a.g.V);
-  imp_one<LOW, false>(a, L, T, Y, W, W2, mu, site);
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_imp(SweepArgs a, int gpc) {
+  const Grp<G> w(IMP_SLOTS, a.SS, gpc, 4L * a.g.V);
+  if (!w.ok) return;
+  imp_one<G>(a, w.slot, w.slot + a.SS, w.slot + 2 * a.SS, w.slot + 3 * a.SS, (int)(w.id & 3),
+             (int)(w.id >> 2));
 }
 
-// The improved-action sweep on the fly where each reference thread owns one
-// site per barrier step: link mu of that site, one launch per (step, mu),
-// the update inline without a walk around it.
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_sweep_imp_otf1(SweepArgs a, LgfGrid gr, long step, int mu) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const long tid = ((long)blockIdx.x * nw + warp) * LPW + g;
-  if (tid >= gr.nthr) return;
-  const int SS = a.SS;
-  double2 *T = sm + (size_t)(warp * LPW + g) * (IMP_SLOTS * SS), *Y = T + SS;
-  double2 *W = Y + SS, *W2 = W + SS;
-  int x[4];
-  LgfWalk(gr, tid, step).site(gr, a.g, 0, x);
-  const int site = x[0] * a.g.s0 + x[1] * a.g.s1 + x[2] * a.g.s2 + x[3];
-  imp_one<LOW, true>(a, L, T, Y, W, W2, mu, site);
-}
-
-// The improved-action sweep on the fly (periodic boundaries): as
-// k_sweep_otf, one group per reference thread walking its sites for one
-// barrier step, links mu_lo..mu_hi-1 of each site in place (a launch per
-// (step, mu) where each thread owns one site per barrier step).
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_sweep_imp_otf(SweepArgs a, LgfGrid gr, long step, int mu_lo, int mu_hi) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const long tid = ((long)blockIdx.x * nw + warp) * LPW + g;
-  if (tid >= gr.nthr) return;
-  const int SS = a.SS;
-  double2 *T = sm + (size_t)(warp * LPW + g) * (IMP_SLOTS * SS), *Y = T + SS;
-  double2 *W = Y + SS, *W2 = W + SS;
-  const LgfWalk walk(gr, tid, step);
+// The improved-action sweep on the fly: as k_sweep_otf
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_imp_otf(SweepArgs a, LgfGrid gr, long step, int gpc) {
+  const Grp<G> w(IMP_SLOTS, a.SS, gpc, gr.nthr);
+  if (!w.ok) return;
+  const LgfWalk walk(gr, w.id, step);
 #pragma unroll 1
-  for (long r = 0; r < gr.seg; r++) {
+  for (long r = 0; r < 4 * gr.seg; r++) {
     int x[4];
-    walk.site(gr, a.g, r, x);
+    walk.site(gr, a.g, r >> 2, x);
     const int site = x[0] * a.g.s0 + x[1] * a.g.s1 + x[2] * a.g.s2 + x[3];
+    imp_one<G>(a, w.slot, w.slot + a.SS, w.slot + 2 * a.SS, w.slot + 3 * a.SS, (int)(r & 3), site);
+    __threadfence();
+    gsync<G>();
+  }
+}
+
+// ---------------- plaquette measurement ----------------
+
+// Re Tr of the product of two slots' series, op(A) B^dag, orders 0..N, a lane
+// per order: Tr(X Y^dag)_k = sum over entries of X_ij conj(Y_ij)
+__device__ __forceinline__ double2 trace_dag(int X, int Y, int k) {
+  const double2 *sm = wsm();
+  const double2 x0 = sm[X], y0 = sm[Y];
+  if (k == 0) return cscale(cmul(x0, cconj(y0)), 3.0);
+  const double2 *xk = sm + X + 9 * k - 8, *yk = sm + Y + 9 * k - 8;
+  double2 s = cadd(cmul(x0, cconj(cadd(cadd(yk[0], yk[4]), yk[8]))),
+                   cmul(cadd(cadd(xk[0], xk[4]), xk[8]), cconj(y0)));
+  for (int i = 1; i < k; i++) {
+    const double2 *p = sm + X + 9 * i - 8, *q = sm + Y + 9 * (k - i) - 8;
+#pragma unroll
+    for (int e = 0; e < 9; e++) cfma(s, p[e], cconj(q[e]));
+  }
+  return s;
+}
+
+constexpr int MEASURE_SLOTS = 4;
+
+
+// plaquette_measure (nspt.cc:1362-1383): the sum over links of Tr(U * staples)
+// meets every plaquette four times, as Tr P or its conjugate, so a plaquette
+// takes two products and a trace.  Field: records of `ser` double2 per link.
+// A twisted link has flag 1 in the view of the link whose staple crosses the
+// face (nspt.cc:115-121); where stored flags are not 1 the four views differ and
+// are summed one by one.  Warps walk the plaquettes grid-stride, a lane per
+// order; a CTA adds its warps' sums in order into partial[blockIdx].
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_plaq_trace(const double2 *U, size_t ser, int N, int SS, Geo g, double2 *partial, int row, int gpc) {
+  const long units = 6L * g.V;
+  const Grp<G> w(MEASURE_SLOTS, SS, gpc, units);
+  double2 *sm = wsm();
+  const int S0 = w.slot, S1 = S0 + SS, S2 = S1 + SS, S3 = S2 + SS, n = (int)link_rec(N);
+  constexpr int PL = G == 32 ? 2 : 6;  // orders per lane, of 49 at most
+  double2 acc[PL];
+#pragma unroll
+  for (int h = 0; h < PL; h++) acc[h] = cz();
 #pragma unroll 1
-    for (int mu = mu_lo; mu < mu_hi; mu++) {
-      imp_one<LOW, true>(a, L, T, Y, W, W2, mu, site);
-      __syncwarp(L.mask);
+  for (long u = w.ok ? w.id : units; u < units; u += (long)gridDim.x * gpc) {
+    const int site = (int)(u / 6), pl = (int)(u - 6L * site);
+    int mu, nu, x[4];
+    plane_dirs(pl, mu, nu);
+    coords(g, site, x);
+    const Nb um = neighbour(g, x, mu, 1), un = neighbour(g, x, nu, 1);
+    const bool cm = um.fwd & g.twist, cn = un.fwd & g.twist;
+    bool odd = false;
+#pragma unroll 1
+    for (int view = 0; view < (odd ? 3 : 1); view++) {
+      gsync<G>();
+      wstage<G>(S0, U + ((size_t)site * 4 + mu) * ser, n);
+      wstage<G>(S1, U + ((size_t)um.site * 4 + nu) * ser, n);
+      wstage<G>(S2, U + ((size_t)site * 4 + nu) * ser, n);
+      wstage<G>(S3, U + ((size_t)un.site * 4 + mu) * ser, n);
+      wstage_wait<G>();
+      const double2 f1 = sm[S1], f3 = sm[S3];
+      if (cm || cn) {
+        auto not1 = [&](double2 f) { return f.x != 1.0 || f.y != 0.0; };
+        odd = not1(sm[S0]) || not1(f1) || not1(sm[S2]) || not1(f3);
+        gsync<G>();
+      }
+      twist_link<G>(S1, um, g, N);
+      twist_link<G>(S3, un, g, N);
+      if (view && w.lane == 0) {
+        // view 1: of the link (mu, x+nu), view 2: of (nu, x+mu)
+        if (view == 1 && cn) sm[S0] = sm[S1] = sm[S2] = make_double2(1.0, 0.0), sm[S3] = f3;
+        if (view == 2 && cm) sm[S0] = sm[S2] = sm[S3] = make_double2(1.0, 0.0), sm[S1] = f1;
+      }
+      gsync<G>();
+      ser_mul<G>(S1, S0, S1, N);
+      ser_mul<G>(S3, S2, S3, N);
+#pragma unroll
+      for (int h = 0; h < PL; h++) {
+        const int k = w.lane + glanes<G>() * h;
+        if (k > N) continue;
+        const double2 t = trace_dag(S1, S3, k);
+        if (view == 0) acc[h].x += (odd ? 2. : 4.) * t.x;
+        if (view == 1) acc[h] = cadd(acc[h], cconj(t));
+        if (view == 2) acc[h] = cadd(acc[h], t);
+      }
     }
+  }
+  __syncthreads();
+  if (w.ok) {
+    const int gi = (int)(w.id - (long)blockIdx.x * gpc);
+#pragma unroll
+    for (int h = 0; h < PL; h++)
+      if (w.lane + glanes<G>() * h <= N) sm[gi * (N + 1) + w.lane + glanes<G>() * h] = acc[h];
+  }
+  __syncthreads();
+  const long left = units - (long)blockIdx.x * gpc;
+  for (int k = threadIdx.x; k <= N; k += blockDim.x) {
+    double2 t = cz();
+    for (int q = 0; q < gpc && q < left; q++) t = cadd(t, sm[q * (N + 1) + k]);
+    partial[(size_t)blockIdx.x * row + k] = t;
+  }
+}
+
+// Sums over the lattice of the logs' records, one per mu and entry, in the order
+// that ORDERED runs keep: 256 partial sums over the sites s = t (mod 256), added
+// as a tree.  A block takes LOGSUM_COLS neighbouring entries.
+constexpr int LOGSUM_COLS = 8;
+__global__ void __launch_bounds__(256)
+    k_logsum(const double2 *__restrict__ Lg, long V, int width, double2 *out) {
+  __shared__ double2 sh[256];
+  const int t = threadIdx.x, c0 = blockIdx.x * LOGSUM_COLS;
+  double2 acc[LOGSUM_COLS];
+#pragma unroll
+  for (int c = 0; c < LOGSUM_COLS; c++) acc[c] = cz();
+  for (long s = t; s < V; s += 256) {
+    const double2 *p = Lg + (size_t)s * width + c0;
+#pragma unroll
+    for (int c = 0; c < LOGSUM_COLS; c++)
+      if (c0 + c < width) acc[c] = cadd(acc[c], p[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < LOGSUM_COLS; c++) {
+    sh[t] = acc[c];
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+      if (t < w) sh[t] = cadd(sh[t], sh[t + w]);
+      __syncthreads();
+    }
+    if (t == 0 && c0 + c < width) out[c0 + c] = sh[0];
+    __syncthreads();
   }
 }
 
@@ -1012,515 +809,237 @@ __global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
 __global__ void k_inc(unsigned long long *c) { *c += 1ull; }
 
 // U = exp(reH(log U - MM[mu]/V)) per link: zero_modes_subtraction,
-// nspt.cc:605-654 (log U is the per-link log stored by the sweep).  The
-// exponent Y = reH(log U - MM/V) goes back into Lg: log(exp(Y)) = Y holds
-// exactly for truncated series (one variable, so the log and exp series
-// invert each other order by order), so Lg then holds log U of the new
-// field, which FA gauge fixing would otherwise recompute (nspt.cc:874-875).
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_zero_modes(double2 *U, double2 *Uf, double2 *Lg, const double2 *MMs, int N, int SS,
-                 Geo geo) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5;
-  const size_t V = (size_t)geo.V;
-  double2 *P = sm + (size_t)(warp * LPW + g) * 3 * SS, *R = P + SS, *Y2 = R + SS;
-  bool valid;
-  const long link = group_unit(g, 4L * geo.V, valid);
-  if (!valid) return;
-  const int mu = (int)(link / geo.V);
-  const int site = (int)(link - (long)mu * geo.V);
-  const double2 *src = Lg + (size_t)mu * 9 * N * V + site;
-  const double2 *mm = MMs + (size_t)mu * 9 * N;
-  {
-    // (here loads through registers measured faster than cp.async plus a
-    // second pass for the subtraction: 6.7 against 7.0 ms at 16^4 x 20)
-    const int r = L.j / 3, c = L.j - 3 * (L.j / 3);
-    for (int k = 1; k <= N; k++) {
-      const int e = 9 * (k - 1) + L.j;
-      P[sidx(k, r, c)] = csub(__ldg(src + (size_t)e * V), mm[e]);
-    }
+// nspt.cc:605-654 (log U is the per-link log stored by the sweep; MM: its
+// sums over the lattice, one record per mu).  The exponent Y = reH(log U -
+// MM/V) goes back into Lg: log(exp(Y)) = Y holds exactly for truncated series
+// (one variable, so the log and exp series invert each other order by order),
+// so Lg then holds log U of the new field, which FA gauge fixing would
+// otherwise recompute (nspt.cc:874-875).
+constexpr int SERIES_SLOTS = 3;
+
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_zero_modes(double2 *U, double2 *Lg, const double2 *MM, double rvol, int N, int SS, Geo geo,
+                 int gpc) {
+  const Grp<G> w(SERIES_SLOTS, SS, gpc, 4L * geo.V);
+  if (!w.ok) return;
+  double2 *sm = wsm();
+  const int P = w.slot, Y = P + SS, R = Y + SS, n = (int)link_rec(N);
+  double2 *lg = Lg + (size_t)w.id * n;
+  const double2 *mm = MM + (size_t)(w.id & 3) * n;
+  for (int e = w.lane; e < n; e += glanes<G>()) {
+    const double2 m = __ldg(mm + e);  // MM / V rounded before it is subtracted
+    sm[P + e] = make_double2(lg[e].x - __dmul_rn(m.x, rvol), lg[e].y - __dmul_rn(m.y, rvol));
   }
-  if (L.j == 0) P[0] = cz();
-  __syncwarp(L.mask);
-  ser_reH(P, N, L);
-  __syncwarp(L.mask);
-  ser_exp<(LOW ? MO_LOW : MO)>(P, Y2, R, N, L);
-  double2 *dst = U + (size_t)mu * 9 * N * V + site;
-  double2 *lg = Lg + (size_t)mu * 9 * N * V + site;
-  const int r = L.j / 3, c = L.j - 3 * (L.j / 3);
-  for (int k = 1; k <= N; k++) {
-    dst[(size_t)(9 * (k - 1) + L.j) * V] = R[sidx(k, r, c)];
-    lg[(size_t)(9 * (k - 1) + L.j) * V] = P[sidx(k, r, c)];
-  }
-  if (L.j == 0) Uf[(size_t)mu * V + site] = make_double2(1.0, 0.0);
+  gsync<G>();
+  ser_reH<G>(P, N);
+  wstore<G>(lg, P, n);
+  wstore<G>(U + (size_t)w.id * n, ser_exp_to<G, false>(P, Y, R, N), n);
 }
 
 // U = exp(reH(log U)) per link: the unitarisation the reference applies to
 // a configuration loaded with fewer orders than it evolves
 // (ptGluon_fld::loadlowerorder, QCDenvNODEpt_test.h:414-417).  Flag 1.
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_unitarise(double2 *U, double2 *Uf, int N, int SS, Geo geo) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5;
-  const size_t V = (size_t)geo.V;
-  double2 *X = sm + (size_t)(warp * LPW + g) * 3 * SS, *Sc = X + SS, *Y2 = Sc + SS;
-  bool valid;
-  const long link = group_unit(g, 4L * geo.V, valid);
-  if (!valid) return;
-  const int mu = (int)(link / geo.V);
-  const int site = (int)(link - (long)mu * geo.V);
-  Nb n;
-  n.site = site;
-  n.fwd = n.bwd = 0;
-  stage(X, U, Uf, mu, n, geo, N, L);
-  const int c = L.c;
-  ser_log<(LOW ? MO_LOW : MO)>(X, Y2, Sc, N, L,
-                               [&](int k, int r, double2 v) { Sc[sidx(k, r, c)] = v; });
-  __syncwarp(L.mask);
-  ser_reH(Sc, N, L);
-  __syncwarp(L.mask);
-  ser_exp<(LOW ? MO_LOW : MO)>(Sc, Y2, X, N, L);
-  double2 *dst = U + (size_t)mu * 9 * N * V + site;
-  for (int k = L.s + 1; k <= N; k += 3) {
-#pragma unroll
-    for (int r = 0; r < 3; r++) dst[(size_t)(9 * (k - 1) + 3 * r + c) * V] = X[sidx(k, r, c)];
-  }
-  if (L.j == 0) Uf[(size_t)mu * V + site] = make_double2(1.0, 0.0);
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_unitarise(double2 *U, int N, int SS, Geo geo, int gpc) {
+  const Grp<G> w(SERIES_SLOTS, SS, gpc, 4L * geo.V);
+  if (!w.ok) return;
+  const int X = w.slot, Y = X + SS, R = Y + SS, n = (int)link_rec(N);
+  wstage<G>(X, U + (size_t)w.id * n, n);
+  wstage_wait<G>();
+  ser_log<G, false>(X, Y, R, N);
+  ser_reH<G>(R, N);
+  wstore<G>(U + (size_t)w.id * n, ser_exp_to<G, false>(R, Y, X, N), n);
 }
 
 // Lg = log(U) per link (the logs FAstochastic_gauge_fixing needs, nspt.cc:874-875).
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_log_links(const double2 *U, const double2 *Uf, double2 *Lg, int N, int SS, Geo geo) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5;
-  const size_t V = (size_t)geo.V;
-  double2 *X = sm + (size_t)(warp * LPW + g) * 3 * SS, *Sc = X + SS, *Y2 = Sc + SS;
-  bool valid;
-  const long link = group_unit(g, 4L * geo.V, valid);
-  if (!valid) return;
-  const int mu = (int)(link / geo.V);
-  const int site = (int)(link - (long)mu * geo.V);
-  Nb n;
-  n.site = site;
-  n.fwd = n.bwd = 0;
-  stage(X, U, Uf, mu, n, geo, N, L);
-  double2 *dst = Lg + (size_t)mu * 9 * N * V + site;
-  const int c = L.c;
-  ser_log<(LOW ? MO_LOW : MO)>(X, Y2, Sc, N, L, [&](int k, int r, double2 v) {
-    dst[(size_t)(9 * (k - 1) + 3 * r + c) * V] = v;
-  });
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_log_links(const double2 *U, double2 *Lg, int N, int SS, Geo geo, int gpc) {
+  const Grp<G> w(SERIES_SLOTS, SS, gpc, 4L * geo.V);
+  if (!w.ok) return;
+  const int X = w.slot, Y = X + SS, R = Y + SS, n = (int)link_rec(N);
+  wstage<G>(X, U + (size_t)w.id * n, n);
+  wstage_wait<G>();
+  ser_log<G, false>(X, Y, R, N);
+  wstore<G>(Lg + (size_t)w.id * n, R, n);
 }
 
-// G(x) = exp(reH(Wg(x) / V))  (nspt.cc:902-906), one group per site.
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_fa_gt(const double2 *Wg, double2 *Gx, int N, int SS, Geo geo) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5;
-  const size_t V = (size_t)geo.V;
-  double2 *P = sm + (size_t)(warp * LPW + g) * 3 * SS, *R = P + SS, *Y2 = R + SS;
-  bool valid;
-  const long site = group_unit(g, geo.V, valid);
-  if (!valid) return;
+// G(x) = exp(reH(Wg(x) / V))  (nspt.cc:902-906), a record per site.
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_fa_gt(const double2 *Wg, double2 *Gx, int N, int SS, Geo geo, int gpc) {
+  const Grp<G> w(SERIES_SLOTS, SS, gpc, geo.V);
+  if (!w.ok) return;
+  double2 *sm = wsm();
+  const int P = w.slot, Y = P + SS, R = Y + SS, n = (int)link_rec(N);
   const double dv = (double)geo.V;
-  const int r = L.j / 3, c = L.j - 3 * (L.j / 3);
-  for (int k = 1; k <= N; k++) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(P + sidx(k, r, c));
-    const double2 *gp = Wg + (size_t)(9 * (k - 1) + L.j) * V + site;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gp) : "memory");
+  for (int e = w.lane; e < 9 * N; e += glanes<G>()) {
+    const double2 v = __ldg(Wg + (size_t)e * geo.V + w.id);
+    sm[P + 1 + e] = make_double2(v.x / dv, v.y / dv);
   }
-  cp_commit();
-  cp_wait0();
-  for (int k = 1; k <= N; k++) {
-    const double2 w = P[sidx(k, r, c)];
-    P[sidx(k, r, c)] = make_double2(w.x / dv, w.y / dv);
-  }
-  if (L.j == 0) P[0] = cz();
-  __syncwarp(L.mask);
-  ser_reH(P, N, L);
-  __syncwarp(L.mask);
-  ser_exp<(LOW ? MO_LOW : MO)>(P, Y2, R, N, L);
-  for (int k = 1; k <= N; k++) Gx[(size_t)(9 * (k - 1) + L.j) * V + site] = R[sidx(k, r, c)];
+  gsync<G>();
+  ser_reH<G>(P, N);
+  wstore<G>(Gx + (size_t)w.id * n, ser_exp_to<G, false>(P, Y, R, N), n);
 }
 
 // U_mu(x) <- G(x) U_mu(x) G(x+mu)^dag  (nspt.cc:912-916), written to F.
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_fa_apply(const double2 *U, const double2 *Uf, const double2 *Gx, double2 *F, double2 *Ff,
-               int N, int SS, Geo geo) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5;
-  const size_t V = (size_t)geo.V;
-  double2 *T = sm + (size_t)(warp * LPW + g) * (2 * SS), *Y = T + SS;
-  bool valid;
-  const long link = group_unit(g, 4L * geo.V, valid);
-  const int mu = (int)(link / geo.V);
-  const int site = (int)(link - (long)mu * geo.V);
+constexpr int APPLY_SLOTS = 3;
+
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_fa_apply(const double2 *U, const double2 *Gx, double2 *F, int N, int SS, Geo geo,
+               int gpc) {
+  const Grp<G> w(APPLY_SLOTS, SS, gpc, 4L * geo.V);
+  if (!w.ok) return;
+  const int T = w.slot, Y = T + SS, H = Y + SS, n = (int)link_rec(N);
+  const int site = (int)(w.id >> 2), mu = (int)(w.id & 3);
   int x[4];
   coords(geo, site, x);
-  const int c = L.c;
-  const double2 one = make_double2(1.0, 0.0);
-  Nb n;
-  n.site = site;
-  n.fwd = n.bwd = 0;
-  // T = G(x), Y = U_mu(x), then T <- T Y in place
-  stage_site(T, Gx, site, V, N, L, one);
-  stage(Y, U, Uf, mu, n, geo, N, L);
-  const double2 tflag = cmul(one, Y[0]);
-  product<(LOW ? MO_LOW : MO), false>(LeftS{T}, one, Y, Y[0], N, L,
-                     [&](int k, int r, double2 v) { T[sidx(k, r, c)] = v; });
-  if (L.j == 0) T[0] = tflag;
-  __syncwarp(L.mask);
-  const Nb up = neighbour(geo, x, mu, 1);
-  stage_site(Y, Gx, up.site, V, N, L, one, true);
-  double2 *dst = F + (size_t)mu * 9 * N * V + site;
-  product<(LOW ? MO_LOW : MO), false>(LeftS{T}, tflag, Y, one, N, L, [&](int k, int r, double2 v) {
-    if (valid) dst[(size_t)(9 * (k - 1) + 3 * r + c) * V] = v;
-  });
-  if (L.j == 0 && valid) Ff[(size_t)mu * V + site] = cmul(tflag, one);
+  wstage<G>(T, Gx + (size_t)site * n, n);
+  wstage<G>(Y, U + (size_t)w.id * n, n);
+  wstage<G>(H, Gx + (size_t)neighbour(geo, x, mu, 1).site * n, n);
+  wstage_wait<G>();
+  ser_mul<G>(Y, T, Y, N, MUL_DAG);
+  ser_mul<G>(Y, Y, H, N, MUL_DB);
+  wstore<G>(F + (size_t)w.id * n, Y, n);
 }
 
 // ---------------- local stochastic gauge fixing ----------------
 
-// A <- A - A^dag, then Trless (W -= dag(W); W.Trless(), nspt.cc:679-682,
-// QCDpt.cc:124-136 and 185-194): flag 0.  Lanes split the orders.
-__device__ __forceinline__ void ser_aherm_trless(double2 *P, int N, const Lane &L) {
-  const double D3 = 1.0 / 3.0;
-  for (int k = 1 + L.j; k <= N; k += GROUP) {
-    double2 *m = P + 1 + 9 * (k - 1);
-    double2 a[9], b[9];
-#pragma unroll
-    for (int e = 0; e < 9; e++) a[e] = m[e];
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-#pragma unroll
-      for (int q = 0; q < 3; q++) b[3 * r + q] = csub(a[3 * r + q], cconj(a[3 * q + r]));
-    const double2 tr = cadd(cadd(b[0], b[4]), b[8]);
-    const double2 z = make_double2(D3 * tr.x, D3 * tr.y);
-    b[0] = csub(b[0], z);
-    b[4] = csub(b[4], z);
-    b[8] = csub(b[8], z);
-#pragma unroll
-    for (int e = 0; e < 9; e++) m[e] = b[e];
-  }
-  if (L.j == 0) P[0] = cz();
-  __syncwarp(L.mask);
-}
-
 // One barrier step of stochastic_gauge_fixing (nspt.cc:660-862), in place:
 // one group per reference thread, walking its segment site by site.  Sites
-// of different groups are >= 2 apart and share no link, so the result is
+// of different threads are >= 2 apart and share no link, so the result is
 // the reference's with the same thread grid.  Per site: W = sum_mu U_mu(x) -
 // U_mu(x-mu) (twisted read across a twisted face), W -= W^dag, Trless,
 // U_mu(x) <- exp(alpha W) U_mu(x), U_mu(x-mu) <- U_mu(x-mu) exp(-alpha W)
 // (twist_mu(exp(-alpha W)) = Omega W2 Omega^dag when x-mu wraps a twisted
-// face, nspt.cc:690-719).  Four slots per group.
-template <bool LOW = false>
-__global__ void __launch_bounds__(LOW ? SWEEP_THREADS_LOW : 256, LOW ? 2 : 1)
-    k_local_gf(double2 *U, double2 *Uf, const double2 *Ut, const double2 *Utf, int N, int SS,
-               Geo geo, double alpha, LgfGrid gr, long step) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const long tid = ((long)blockIdx.x * nw + warp) * LPW + g;
-  if (tid >= gr.nthr) return;
-  double2 *A = sm + (size_t)(warp * LPW + g) * 4 * SS, *Y2 = A + SS, *E1 = Y2 + SS, *E2 = E1 + SS;
-  const size_t V = (size_t)geo.V;
-  const size_t plane = (size_t)9 * N * V;
-  const int c = L.c;
-  const double2 one = make_double2(1.0, 0.0);
-  const LgfWalk walk(gr, tid, step);
+// face, nspt.cc:690-719).  alpha W is antihermitian, so exp(-alpha W) is the
+// dagger of exp(alpha W): one exponential and daggered products.
+template <int G>
+__host__ __device__ constexpr int lgf_slots() {
+  return G == ORDERED ? 4 : 3;
+}
+
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_local_gf(double2 *U, const double2 *Ut, int N, int SS, Geo geo, double alpha, LgfGrid gr,
+               long step, int gpc) {
+  const Grp<G> w(lgf_slots<G>(), SS, gpc, gr.nthr);
+  if (!w.ok) return;
+  double2 *sm = wsm();
+  const int X = w.slot, Y = X + SS, E = Y + SS, n = (int)link_rec(N);
+  const double D3 = 1.0 / 3.0;
+  const LgfWalk walk(gr, w.id, step);
+#pragma unroll 1
   for (long r = 0; r < gr.seg; r++) {
     int x[4];
     walk.site(gr, geo, r, x);
-    Nb self;
-    self.site = x[0] * geo.s0 + x[1] * geo.s1 + x[2] * geo.s2 + x[3];
-    self.fwd = self.bwd = 0;
+    const int site = x[0] * geo.s0 + x[1] * geo.s1 + x[2] * geo.s2 + x[3];
     // W = sum_mu U_mu(x) - U_mu(x-mu)  (nspt.cc:672-675)
+#pragma unroll 1
     for (int mu = 0; mu < 4; mu++) {
-      stage<true>(Y2, U, Uf, mu, self, geo, N, L);
       const Nb bn = neighbour(geo, x, mu, -1);
       const bool cross = (bn.bwd & geo.twist) != 0;
-      stage<true>(E1, cross ? Ut : U, cross ? Utf : Uf, mu, bn, geo, N, L);
-      for (int e = L.j; e < 1 + 9 * N; e += GROUP)
-        A[e] = cadd(mu == 0 ? cz() : A[e], csub(Y2[e], E1[e]));
-      __syncwarp(L.mask);
+      wstage<G>(Y, U + link_at(mu, site, N), n);
+      wstage<G>(E, (cross ? Ut : U) + link_at(mu, bn.site, N), n);
+      wstage_wait<G>();
+      twist_link<G>(E, bn, geo, N);
+      for (int e = w.lane; e < n; e += glanes<G>())
+        sm[X + e] = cadd(mu == 0 ? cz() : sm[X + e], csub(sm[Y + e], sm[E + e]));
+      gsync<G>();
     }
-    ser_aherm_trless(A, N, L);
-    for (int e = L.j; e < 1 + 9 * N; e += GROUP) A[e] = cscale(A[e], alpha);
-    __syncwarp(L.mask);
-    // E1 = exp(alpha W), E2 = exp(-alpha W), sharing (alpha W)^2
-    ser_square<(LOW ? MO_LOW : MO)>(A, Y2, N, L);
-    // one call site for both (the odd terms negated for E2): the inlined
-    // series code once instead of twice
-    for (int h = 0; h < 2; h++) {
-      double2 *E = h == 0 ? E1 : E2;
-      const double odd = h == 0 ? 1.0 : -1.0;
-      ser_horner2<(LOW ? MO_LOW : MO)>(
-          A, Y2, E, N, L,
-          [odd](int n) { return (n & 1) ? odd * inv_factorial(n) : inv_factorial(n); },
-          [&](int k, int rr, double2 v) { E[sidx(k, rr, c)] = v; });
-    }
-    if (L.j == 0) E1[0] = E2[0] = one;
-    __syncwarp(L.mask);
-    for (int mu = 0; mu < 4; mu++) {
-      const Nb back = neighbour(geo, x, mu, -1);
-      for (int h = 0; h < 2; h++) {
-        // h = 0: U_mu(x) <- E1 U_mu(x); h = 1: U_mu(x-mu) <- U_mu(x-mu) E2,
-        // E2 twisted across a twisted face.  One product call site for both.
-        Nb at;
-        at.site = h == 0 ? self.site : back.site;
-        at.fwd = at.bwd = 0;
-        double2 *Sl = h == 0 ? Y2 : A;
-        stage<true>(Sl, U, Uf, mu, at, geo, N, L);
-        const double2 *R = E2;
-        if (h == 1 && ((back.bwd & geo.twist) >> mu & 1u)) {
-          for (int k = 1 + L.j; k <= N; k += GROUP) {
-            const double2 *src = E2 + 1 + 9 * (k - 1);
-            double2 m[9];
+    // X = alpha Trless(W - W^dag) (nspt.cc:679-682, QCDpt.cc:124-136, 185-194)
+    for (int k = 1 + w.lane; k <= N; k += glanes<G>()) {
+      double2 *p = sm + X + 9 * k - 8;
+      double2 a[9], b[9];
 #pragma unroll
-            for (int rr = 0; rr < 3; rr++)
+      for (int e = 0; e < 9; e++) a[e] = p[e];
 #pragma unroll
-              for (int q = 0; q < 3; q++) m[3 * rr + q] = src[3 * q + rr];
-            twist3(m, 0u, 1u << mu);
-            double2 *o = Y2 + 1 + 9 * (k - 1);
+      for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int rr = 0; rr < 3; rr++)
-#pragma unroll
-              for (int q = 0; q < 3; q++) o[3 * q + rr] = m[3 * rr + q];
-          }
-          if (L.j == 0) Y2[0] = one;  // twist_* returns flag VACUUM
-          __syncwarp(L.mask);
-          R = Y2;
-        }
-        const double2 *left = h == 0 ? E1 : A, *right = h == 0 ? Y2 : R;
-        const double2 lf = left[0], rf = right[0];
-        double2 *dst = U + mu * plane + at.site;
-        product<(LOW ? MO_LOW : MO), false>(LeftS{left}, lf, right, rf, N, L,
-                                            [&](int k, int rr, double2 v) {
-                                              dst[(size_t)(9 * (k - 1) + 3 * rr + c) * V] = v;
-                                            });
-        if (L.j == 0) Uf[(size_t)mu * V + at.site] = flag_mul(lf, rf);
-        __syncwarp(L.mask);
-      }
-    }
-  }
-}
-
-// Copy link (mu, site) as stored (no twist, no dagger) into a slot without
-// waiting: the caller commits and waits for the copies of all its stagings
-// at once.  Lane j copies colour component j of every order, as in stage().
-__device__ __forceinline__ void stage_issue(double2 *slot, const double2 *U, const double2 *Uf,
-                                            int mu, int site, size_t V, int N, const Lane &L) {
-  const double2 *src = U + (size_t)mu * 9 * N * V + site;
-  const int r = L.j / 3, c = L.j - 3 * (L.j / 3);
-  for (int k = 1; k <= N; k++) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(slot + 1 + 9 * (k - 1) + 3 * c + r);
-    const double2 *gp = src + (size_t)(9 * (k - 1) + L.j) * V;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gp) : "memory");
-  }
-  if (L.j == 0) slot[0] = __ldcg(Uf + (size_t)mu * V + site);
-}
-
-// The team form of k_local_gf, for barrier steps with too few reference
-// threads to fill the GPU (the 12^4 lattice's 6^4 threads, one site each):
-// one warp of three link groups per reference thread, visiting the same
-// sites in the same order.  Per site the team
-//   - stages the eight links U_mu(x), U_mu(x-mu) at once (group g the links
-//     of tasks g, g+3, g+6; task t < 4 is U_t(x), t >= 4 is U_{t-4}(x-mu)),
-//   - forms alpha Trless(W - W^dag), W = sum_mu U_mu(x) - U_mu(x-mu), with
-//     all 27 lanes (one order each, the back link twisted across a twisted
-//     face as stage() twists it),
-//   - squares it in group 0, then runs exp(alpha W) in group 0 and
-//     exp(-alpha W) in group 1 side by side,
-//   - and multiplies the eight links by them, the tasks dealt over the
-//     three groups as the stagings were, from the staged copies (no other
-//     thread writes those links between the barriers, and L_d >= 2 keeps
-//     U_mu(x-mu) apart from the site's forward links).
-// The operations and their order per value are those of k_local_gf.  Slots
-// per team: the eight links, alpha W, (alpha W)^2, E1, E2, and one scratch
-// slot per group for a twisted E2.
-constexpr int LGF_TEAM_SLOTS = 15;
-
-template <bool LOW = false>
-__global__ void __launch_bounds__(64, LOW ? 5 : 4)
-    k_local_gf_team(double2 *U, double2 *Uf, const double2 *Ut, const double2 *Utf, int N,
-                    int SS, Geo geo, double alpha, LgfGrid gr, long step) {
-  constexpr int MOK = LOW ? MO_LOW : MO;
-  constexpr int TEAM = LPW * GROUP;
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  if (!make_lane(L, g)) return;
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const long tid = (long)blockIdx.x * nw + warp;
-  if (tid >= gr.nthr) return;
-  const int tl = g * GROUP + L.j;
-  const unsigned tmask = (1u << TEAM) - 1u;
-  double2 *S = sm + (size_t)warp * LGF_TEAM_SLOTS * SS;
-  double2 *X = S + 8 * SS, *X2 = X + SS, *E1 = X2 + SS, *E2 = E1 + SS;
-  double2 *Tw = E2 + SS + (size_t)g * SS;
-  const size_t V = (size_t)geo.V;
-  const size_t plane = (size_t)9 * N * V;
-  const int c = L.c;
-  const double2 one = make_double2(1.0, 0.0);
-  const double D3 = 1.0 / 3.0;
-  const LgfWalk walk(gr, tid, step);
-  for (long r = 0; r < gr.seg; r++) {
-    int x[4];
-    walk.site(gr, geo, r, x);
-    const int self = x[0] * geo.s0 + x[1] * geo.s1 + x[2] * geo.s2 + x[3];
-    for (int t = g; t < 8; t += LPW) {
-      const int mu = t & 3;
-      const Nb bn = neighbour(geo, x, mu, -1);
-      stage_issue(S + (size_t)t * SS, U, Uf, mu, t < 4 ? self : bn.site, V, N, L);
-      // a back link read across a twisted face, as the step's start field
-      // holds it (the same as U except after an on-the-fly sweep); the
-      // scratch slots are free until the link products
-      if (t >= 4 && Ut != U && (bn.bwd & geo.twist))
-        stage_issue(E2 + (size_t)mu * SS, Ut, Utf, mu, bn.site, V, N, L);
-    }
-    cp_commit();
-    cp_wait0();
-    __syncwarp(tmask);
-    // alpha Trless(W - W^dag), order k by team lane k-1 (slots column major)
-    for (int k = 1 + tl; k <= N; k += TEAM) {
-      double2 w[9];
-#pragma unroll
-      for (int mu = 0; mu < 4; mu++) {
-        const double2 *f = S + (size_t)mu * SS + 1 + 9 * (k - 1);
-        const unsigned tb = neighbour(geo, x, mu, -1).bwd & geo.twist;
-        const double2 *bk = (tb && Ut != U ? E2 + (size_t)mu * SS : S + (size_t)(4 + mu) * SS) +
-                            1 + 9 * (k - 1);
-        double2 bv[9];
-        if (tb) {
-          double2 m[9];
-#pragma unroll
-          for (int rr = 0; rr < 3; rr++)
-#pragma unroll
-            for (int q = 0; q < 3; q++) m[3 * rr + q] = bk[3 * q + rr];
-          twist3(m, tb, 0u);
-#pragma unroll
-          for (int rr = 0; rr < 3; rr++)
-#pragma unroll
-            for (int q = 0; q < 3; q++) bv[3 * q + rr] = m[3 * rr + q];
-        } else {
-#pragma unroll
-          for (int e = 0; e < 9; e++) bv[e] = bk[e];
-        }
-#pragma unroll
-        for (int e = 0; e < 9; e++) w[e] = cadd(mu == 0 ? cz() : w[e], csub(f[e], bv[e]));
-      }
-      double2 b[9];
-#pragma unroll
-      for (int rr = 0; rr < 3; rr++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) b[3 * rr + q] = csub(w[3 * rr + q], cconj(w[3 * q + rr]));
+        for (int q = 0; q < 3; q++) b[3 * i + q] = csub(a[3 * i + q], cconj(a[3 * q + i]));
       const double2 tr = cadd(cadd(b[0], b[4]), b[8]);
       const double2 z = make_double2(D3 * tr.x, D3 * tr.y);
       b[0] = csub(b[0], z);
       b[4] = csub(b[4], z);
       b[8] = csub(b[8], z);
-      double2 *o = X + 1 + 9 * (k - 1);
 #pragma unroll
-      for (int e = 0; e < 9; e++) o[e] = cscale(b[e], alpha);
+      for (int e = 0; e < 9; e++) p[e] = cscale(b[e], alpha);
     }
-    if (tl == 0) X[0] = cscale(cz(), alpha);
-    __syncwarp(tmask);
-    // E1 = exp(alpha W), E2 = exp(-alpha W), sharing (alpha W)^2
-    if (g == 0) ser_square<MOK>(X, X2, N, L);
-    __syncwarp(tmask);
-    if (g < 2) {
-      // group 0: exp(alpha W); group 1: exp(-alpha W), the odd terms negated
-      double2 *E = g == 0 ? E1 : E2;
-      const double odd = g == 0 ? 1.0 : -1.0;
-      ser_horner2<MOK>(X, X2, E, N, L,
-                       [odd](int n) { return (n & 1) ? odd * inv_factorial(n) : inv_factorial(n); },
-                       [&](int k, int rr, double2 v) { E[sidx(k, rr, c)] = v; });
+    if (w.lane == 0) sm[X] = cz();
+    gsync<G>();
+    // P = exp(X), and M = exp(-X): P's dagger, or with ORDERED summed by itself
+    int P = X, M = X;
+    if constexpr (G == ORDERED) {
+      P = E;
+      M = E + SS;
+      ser_exp_horner<G, true>(X, Y, P, N);
+      ser_exp_horner<G, true>(X, Y, M, N, -1.0);
+    } else {
+      ser_exp<G, true>(X, Y, E, N);
     }
-    __syncwarp(tmask);
-    if (tl == 0) E1[0] = E2[0] = one;
-    __syncwarp(tmask);
-    for (int t = g; t < 8; t += LPW) {
-      // t < 4: U_mu(x) <- E1 U_mu(x); t >= 4: U_mu(x-mu) <- U_mu(x-mu) E2,
-      // E2 twisted across a twisted face
-      const int mu = t & 3;
-      const double2 *Sl = S + (size_t)t * SS;
-      const bool fwd = t < 4;
+#pragma unroll 1
+    for (int t = 0; t < 8; t++) {
+      // even: U_mu(x) <- P U_mu(x); odd: U_mu(x-mu) <- U_mu(x-mu) M, twisted
+      // across a twisted face
+      const int mu = t >> 1;
+      const bool fwd = !(t & 1);
+      const int S = G == ORDERED ? X : E;  // a slot free now
       const Nb back = neighbour(geo, x, mu, -1);
-      const double2 *R = E2;
+      double2 *rec = U + link_at(mu, fwd ? site : back.site, N);
+      wstage<G>(Y, rec, n);
+      int R = M;
       if (!fwd && ((back.bwd & geo.twist) >> mu & 1u)) {
-        for (int k = 1 + L.j; k <= N; k += GROUP) {
-          const double2 *src = E2 + 1 + 9 * (k - 1);
-          double2 m[9];
-#pragma unroll
-          for (int rr = 0; rr < 3; rr++)
-#pragma unroll
-            for (int q = 0; q < 3; q++) m[3 * rr + q] = src[3 * q + rr];
-          twist3(m, 0u, 1u << mu);
-          double2 *o = Tw + 1 + 9 * (k - 1);
-#pragma unroll
-          for (int rr = 0; rr < 3; rr++)
-#pragma unroll
-            for (int q = 0; q < 3; q++) o[3 * q + rr] = m[3 * rr + q];
-        }
-        if (L.j == 0) Tw[0] = one;  // twist_* returns flag VACUUM
-        __syncwarp(L.mask);
-        R = Tw;
+        for (int e = w.lane; e < n; e += glanes<G>()) sm[S + e] = sm[M + e];
+        gsync<G>();
+        wtwist<G>(S, 0u, 1u << mu, N);
+        R = S;
       }
-      const double2 *left = fwd ? E1 : Sl, *right = fwd ? Sl : R;
-      const double2 lf = left[0], rf = right[0];
-      const int site = fwd ? self : back.site;
-      double2 *dst = U + mu * plane + site;
-      product<MOK, false>(LeftS{left}, lf, right, rf, N, L, [&](int k, int rr, double2 v) {
-        dst[(size_t)(9 * (k - 1) + 3 * rr + c) * V] = v;
-      });
-      if (L.j == 0) Uf[(size_t)mu * V + site] = flag_mul(lf, rf);
-      __syncwarp(L.mask);
+      wstage_wait<G>();
+      ser_mul<G>(Y, fwd ? P : Y, fwd ? Y : R, N, fwd || G == ORDERED ? MUL_DAG : MUL_DB);
+      wstore<G>(rec, Y, n);
+      gsync<G>();
     }
-    // the next site's stagings read links written here
-    __syncwarp(tmask);
+    // the next site's copies read links written here
+    __threadfence();
+    gsync<G>();
   }
 }
 
-// Wg(x) = sum_mu [log U_mu(x) - log U_mu(x-mu)]  (nspt.cc:871-877)
-__global__ void k_fa_div(const double2 *__restrict__ Lg, double2 *__restrict__ Wg, int N, Geo geo) {
-  const size_t V = (size_t)geo.V;
-  const size_t tot = (size_t)9 * N * V;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const size_t e = i / V;
-    const int site = (int)(i - e * V);
-    int x[4];
-    coords(geo, site, x);
-    double2 w = cz();
+// ---------------- Fourier-accelerated gauge fixing ----------------
+
+// Wg(x) = sum_mu [log U_mu(x) - log U_mu(x-mu)]  (nspt.cc:871-877), from
+// records to planes: a CTA takes 32 sites and 32 entries at a time, reads each
+// record's run of entries and writes each plane's run of sites through a
+// shared tile.
+__global__ void __launch_bounds__(256) k_fa_div(const double2 *__restrict__ Lg,
+                                                double2 *__restrict__ Wg, int N, Geo geo) {
+  __shared__ double2 tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int n9 = 9 * N;
+  const size_t rec = link_rec(N), V = (size_t)geo.V;
+  const int e = blockIdx.y * 32 + tx, s0 = blockIdx.x * 32;
+  for (int q = ty; q < 32; q += 8) {
+    const int site = s0 + q;
+    double2 v = cz();
+    if (site < geo.V && e < n9) {
+      int x[4];
+      coords(geo, site, x);
 #pragma unroll
-    for (int mu = 0; mu < 4; mu++) {
-      const Nb b = neighbour(geo, x, mu, -1, 0, 0);
-      const double2 *pl = Lg + ((size_t)mu * 9 * N + e) * V;
-      w = cadd(w, csub(pl[site], pl[b.site]));
+      for (int mu = 0; mu < 4; mu++) {
+        const int b = neighbour(geo, x, mu, -1).site;
+        v = cadd(v, csub(__ldg(Lg + ((size_t)site * 4 + mu) * rec + 1 + e),
+                         __ldg(Lg + ((size_t)b * 4 + mu) * rec + 1 + e)));
+      }
     }
-    Wg[i] = w;
+    tile[q][tx] = v;
+  }
+  __syncthreads();
+  for (int q = ty; q < 32; q += 8) {
+    const int ee = blockIdx.y * 32 + q, site = s0 + tx;
+    if (site < geo.V && ee < n9) Wg[(size_t)ee * V + site] = tile[tx][q];
   }
 }
 
@@ -1604,34 +1123,26 @@ __global__ void k_fft_direct(double2 *data, long nlines, int n, int st, size_t V
   }
 }
 
-// Deterministic row sums: out[r] = sum_i in[r*stride + i], i < n.
-template <class T>
-__global__ void k_rowsum(const T *__restrict__ in, size_t stride, long n, T *out) {
-  __shared__ T sh[256];
-  const T *row = in + (size_t)blockIdx.x * stride;
-  T acc;
-  if constexpr (sizeof(T) == 16) {
-    acc = cz();
-    for (long i = threadIdx.x; i < n; i += blockDim.x) acc = cadd(acc, row[i]);
-  } else {
-    acc = 0.0;
-    for (long i = threadIdx.x; i < n; i += blockDim.x) acc += row[i];
-  }
-  sh[threadIdx.x] = acc;
+// Column sums of a matrix of `rows` rows of `width` doubles, rows in a fixed
+// order: block (i, j) sums the j-th chunk of rows of columns 32 i .. 32 i + 31
+// into out[j][width].  Launched twice, the second time over the chunks.
+__global__ void __launch_bounds__(256)
+    k_colsum(const double *__restrict__ in, long rows, int width, long chunk, double *out) {
+  __shared__ double sh[8][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + tx;
+  const long r0 = blockIdx.y * chunk, r1 = r0 + chunk < rows ? r0 + chunk : rows;
+  double s = 0.0;
+  if (c < width)
+    for (long r = r0 + ty; r < r1; r += 8) s += in[(size_t)r * width + c];
+  sh[ty][tx] = s;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      if constexpr (sizeof(T) == 16)
-        sh[threadIdx.x] = cadd(sh[threadIdx.x], sh[threadIdx.x + w]);
-      else
-        sh[threadIdx.x] += sh[threadIdx.x + w];
-    }
-    __syncthreads();
+  if (ty == 0 && c < width) {
+    for (int q = 1; q < 8; q++) s += sh[q][tx];
+    out[(size_t)blockIdx.y * width + c] = s;
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
-// MMs[mu][e] = MM[mu][e] * (1/V)  (MM[mu] *= rVol, nspt.cc:607-609)
 // ---------------- float-float scale exponent ----------------
 
 // mx[k-1] = max over the field's order-k entries of max(|re|, |im|), as the
@@ -1640,12 +1151,12 @@ __global__ void k_rowsum(const T *__restrict__ in, size_t stride, long n, T *out
 __global__ void k_order_absmax(const double2 *__restrict__ U, int N, size_t V,
                                unsigned long long *mx) {
   const int k = blockIdx.y + 1;
-  const size_t per = 9 * V;  // entries of one order in one direction plane
+  const size_t per = 36 * V;  // entries of one order
   double m = 0.0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < 4 * per;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < per;
        i += (size_t)gridDim.x * blockDim.x) {
-    const size_t mu = i / per, r = i - mu * per;
-    const double2 v = __ldg(U + (mu * 9 * N + 9 * (size_t)(k - 1)) * V + r);
+    const size_t l = i / 9;
+    const double2 v = __ldg(U + l * link_rec(N) + 1 + 9 * (size_t)(k - 1) + (i - 9 * l));
     m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
   }
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -1680,60 +1191,33 @@ __global__ void k_ff_fit(const unsigned long long *mx, int N, int *e_out) {
   *e_out = max(-lim, min(lim, e));
 }
 
-__global__ void k_scale_mm(double2 *MM, int n, double rvol) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) MM[i] = cscale(MM[i], rvol);
-}
-
-// Host AoS chunk (sites [s0, s0+cs), reference ptGluon layout with A orders)
-// <-> device planes.
+// Host field chunk (sites [s0, s0+cs), the reference's layout with A >= N
+// orders per link) <-> device records; with A = N the two are one copy.
 __global__ void k_unpack(const double2 *__restrict__ aos, int A, int s0, int cs, double2 *U,
-                         double2 *Uf, int N, size_t V) {
-  const int ser = 1 + 9 * A;
-  const long tot = (long)cs * 4 * (1 + 9 * N);
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < tot;
-       i += (long)gridDim.x * blockDim.x) {
-    const int ls = (int)(i % cs);
-    const long q = i / cs;
-    const int e = (int)(q % (1 + 9 * N));
-    const int mu = (int)(q / (1 + 9 * N));
-    const double2 v = aos[((size_t)ls * 4 + mu) * ser + e];
-    const size_t site = (size_t)s0 + ls;
-    if (e == 0)
-      Uf[(size_t)mu * V + site] = v;
-    else
-      U[((size_t)mu * 9 * N + (e - 1)) * V + site] = v;
+                         int N) {
+  const size_t rec = link_rec(N), ser = 1 + 9 * (size_t)A, tot = (size_t)cs * 4 * rec;
+  double2 *dst = U + (size_t)s0 * 4 * rec;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const size_t l = i / rec;
+    dst[i] = aos[l * ser + (i - l * rec)];
   }
 }
-__global__ void k_pack(double2 *__restrict__ aos, int A, int s0, int cs, const double2 *U,
-                       const double2 *Uf, int N, size_t V) {
-  const int ser = 1 + 9 * A;
-  const long tot = (long)cs * 4 * ser;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < tot;
-       i += (long)gridDim.x * blockDim.x) {
-    const int ls = (int)(i % cs);
-    const long q = i / cs;
-    const int e = (int)(q % ser);
-    const int mu = (int)(q / ser);
-    const size_t site = (size_t)s0 + ls;
-    double2 v;
-    if (e == 0)
-      v = Uf[(size_t)mu * V + site];
-    else if (e - 1 < 9 * N)
-      v = U[((size_t)mu * 9 * N + (e - 1)) * V + site];
-    else
-      v = cz();
-    aos[((size_t)ls * 4 + mu) * ser + e] = v;
+__global__ void k_pack(double2 *__restrict__ aos, int A, int s0, int cs, const double2 *U, int N) {
+  const size_t rec = link_rec(N), ser = 1 + 9 * (size_t)A, tot = (size_t)cs * 4 * ser;
+  const double2 *src = U + (size_t)s0 * 4 * rec;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const size_t l = i / ser, e = i - l * ser;
+    aos[i] = e < rec ? src[l * rec + e] : cz();
   }
 }
 
-__global__ void k_cold(double2 *U, double2 *Uf, size_t nU, size_t nF) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nU;
+__global__ void k_cold(double2 *U, size_t nlinks, int N) {
+  const size_t rec = link_rec(N), tot = nlinks * rec;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot;
        i += (size_t)gridDim.x * blockDim.x)
-    U[i] = cz();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nF;
-       i += (size_t)gridDim.x * blockDim.x)
-    Uf[i] = make_double2(1.0, 0.0);
+    U[i] = i % rec ? cz() : make_double2(1.0, 0.0);
 }
 
 // FP64 FMA throughput probe: 8 independent chains per thread.

@@ -3,7 +3,7 @@
 // summed over the lattice and traced, per order.  Periodic boundaries, as
 // the reference computes them only there (__MANY_LOOP__ under PERIODIC_BC).
 //
-// One 9-lane group per (plane, site).  The reference closes each loop with a
+// One group per (plane, site).  The reference closes each loop with a
 // product by a daggered path, W += P Q^dag; only Tr W is printed, so the last
 // product is replaced by Tr(P Q^dag) = sum over cells of P_ij conj(Q_ij),
 // order by order.  Three slots per group (two paths and a staging slot) and
@@ -13,46 +13,25 @@
 
 namespace nspt {
 
-constexpr int LOOP_SLOTS = 3;
+constexpr int LOOP_SLOTS = 3, LOOP_EXTRA = 1;  // 1 + 9 N >= 4 (N + 1) for the accumulators (N = 1: 10)
 
-// acc[k] += Tr(X Y^dag)_k, k = 0..N (flags are multiples of the identity)
-__device__ __forceinline__ void trace_dag_acc(const double2 *X, const double2 *Y, int N,
-                                              const Lane &L, double2 *acc) {
-  const double2 x0 = X[0], y0 = Y[0];
-  for (int k = L.j; k <= N; k += GROUP) {
-    double2 s;
-    if (k == 0) {
-      s = cscale(cmul(x0, cconj(y0)), 3.0);
-    } else {
-      const double2 trX = cadd(cadd(X[sidx(k, 0, 0)], X[sidx(k, 1, 1)]), X[sidx(k, 2, 2)]);
-      const double2 trY = cadd(cadd(Y[sidx(k, 0, 0)], Y[sidx(k, 1, 1)]), Y[sidx(k, 2, 2)]);
-      s = cadd(cmul(x0, cconj(trY)), cmul(trX, cconj(y0)));
-      for (int i = 1; i < k; i++) {
-        const double2 *xi = X + 1 + 9 * (i - 1), *yj = Y + 1 + 9 * (k - i - 1);
-#pragma unroll
-        for (int e = 0; e < 9; e++) {
-          const double2 a = xi[e], b = yj[e];
-          s.x = fma(a.x, b.x, s.x);
-          s.x = fma(a.y, b.y, s.x);
-          s.y = fma(a.y, b.x, s.y);
-          s.y = fma(-a.x, b.y, s.y);
-        }
-      }
-    }
-    acc[k] = cadd(acc[k], s);
-  }
-  __syncwarp(L.mask);
+// acc[k] += Tr(X Y^dag)_k, k = 0..N, a lane per order
+template <int G>
+__device__ __forceinline__ void trace_dag_acc(int X, int Y, int N, int acc) {
+  double2 *sm = wsm();
+  for (int k = glane<G>(); k <= N; k += glanes<G>()) sm[acc + k] = cadd(sm[acc + k], trace_dag(X, Y, k));
+  gsync<G>();
 }
 
-// A path of the loops: a chain of forward links, link m in direction
-// dir[m] at the site reached by the steps of the links before it.
+// A path of the loops: a chain of n forward links, link m in direction
+// (dirs >> m) & 1 (0: mu, 1: nu) at the site reached by the links before it.
 struct LoopPath {
-  int n;         // links
-  int dir[8];    // 0: mu, 1: nu
+  int n;
+  unsigned dirs;
 };
 
 struct LoopCtx {
-  const double2 *U, *Uf;
+  const double2 *U;
   int N, mu, nu;
   int X[4];
   Geo geo;
@@ -60,39 +39,27 @@ struct LoopCtx {
 
 // site X + i mu + j nu (periodic)
 __device__ __forceinline__ int loop_site(const LoopCtx &q, int i, int j) {
-  int y[4] = {q.X[0], q.X[1], q.X[2], q.X[3]};
-  y[q.mu] = (y[q.mu] + i) % q.geo.L[q.mu];
-  y[q.nu] = (y[q.nu] + j) % q.geo.L[q.nu];
+  int y[4];
+#pragma unroll
+  for (int d = 0; d < 4; d++)
+    y[d] = (q.X[d] + (d == q.mu ? i : 0) + (d == q.nu ? j : 0)) % q.geo.L[d];
   return y[0] * q.geo.s0 + y[1] * q.geo.s1 + y[2] * q.geo.s2 + y[3];
-}
-
-__device__ __forceinline__ void loop_stage(const LoopCtx &q, double2 *slot, int dir, int i, int j,
-                                           const Lane &L) {
-  Nb n;
-  n.site = loop_site(q, i, j);
-  n.fwd = n.bwd = 0;
-  stage(slot, q.U, q.Uf, dir ? q.nu : q.mu, n, q.geo, q.N, L);
-}
-
-// A <- A S, in place
-__device__ __noinline__ void loop_mul(double2 *A, const double2 *S, int N, const Lane &L) {
-  const double2 a0 = A[0], b0 = S[0];
-  const int c = L.c;
-  product<MO, false>(LeftS{A}, a0, S, b0, N, L,
-                     [&](int k, int r, double2 v) { A[sidx(k, r, c)] = v; });
-  if (L.j == 0) A[0] = flag_mul(a0, b0);
-  __syncwarp(L.mask);
 }
 
 // A <- path[from..n) applied to A (from = 0: A is formed from the first
 // link); (i, j) is the site where link `from` starts, updated to the end
-__device__ __forceinline__ void loop_chain(const LoopCtx &q, double2 *A, double2 *S,
-                                           const LoopPath &p, int from, int &i, int &j,
-                                           const Lane &L) {
+template <int G>
+__device__ __forceinline__ void loop_chain(const LoopCtx &q, int A, int S, const LoopPath &p,
+                                           int from, int &i, int &j) {
+#pragma unroll 1
   for (int m = from; m < p.n; m++) {
-    loop_stage(q, m == 0 ? A : S, p.dir[m], i, j, L);
-    if (m > 0) loop_mul(A, S, q.N, L);
-    if (p.dir[m]) j++; else i++;
+    wstage<G>(m == 0 ? A : S, q.U + link_at((p.dirs >> m & 1) ? q.nu : q.mu, loop_site(q, i, j), q.N),
+           (int)link_rec(q.N));
+    if (m > 0) {  // the first link is waited for with the second
+      wstage_wait<G>();
+      ser_mul<G>(A, A, S, q.N);
+    }
+    if (p.dirs >> m & 1) j++; else i++;
   }
 }
 
@@ -109,36 +76,32 @@ __device__ __forceinline__ void loop_chain(const LoopCtx &q, double2 *A, double2
 // link) and S (the staged link).  A path is extended when the next loop's
 // path starts with it (bl cd -> bl cd cu, ld lu tl -> ld lu tl tr) and
 // formed afresh otherwise: 40 products and 6 traces per (plane, site).
-__global__ void __launch_bounds__(256, 1)
-    k_loops(const double2 *U, const double2 *Uf, int N, int SS, Geo geo, double2 *partial) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  const bool grouped = make_lane(L, g);
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_loops(const double2 *U, int N, int SS, Geo geo, double2 *partial, int gpc) {
+  double2 *sm = wsm();
   const int row = 4 * (N + 1);
-  const size_t gsz = (size_t)LOOP_SLOTS * SS + row;
-  double2 *base = sm + (size_t)(warp * LPW + g) * gsz;
-  double2 *acc = base + (size_t)LOOP_SLOTS * SS;
-  if (grouped) {
-    double2 *P = base, *Q = base + SS, *S = base + 2 * SS;
-    for (int e = L.j; e < row; e += GROUP) acc[e] = cz();
-    __syncwarp(L.mask);
-    double2 *a21 = acc, *a22 = acc + (N + 1), *a42 = acc + 2 * (N + 1), *a44 = acc + 3 * (N + 1);
+  const long units = 6L * geo.V;
+  // the accumulators follow the three slots, in a stretch of LOOP_EXTRA slots
+  const Grp<G> w(LOOP_SLOTS + LOOP_EXTRA, SS, gpc, units);
+  const int P = w.slot, Q = P + SS, S = Q + SS, acc = S + SS;
+  if (w.ok) {
+    for (int e = w.lane; e < row; e += glanes<G>()) sm[acc + e] = cz();
+    gsync<G>();
+    const int a21 = acc, a22 = acc + (N + 1), a42 = acc + 2 * (N + 1), a44 = acc + 3 * (N + 1);
     LoopCtx q;
     q.U = U;
-    q.Uf = Uf;
     q.N = N;
     q.geo = geo;
-    const LoopPath p22{4, {0, 0, 1, 1}}, q22{4, {1, 1, 0, 0}};
-    const LoopPath p42u{6, {0, 0, 1, 1, 1, 1}}, q42u{6, {1, 1, 1, 1, 0, 0}};
-    const LoopPath p44{8, {0, 0, 0, 0, 1, 1, 1, 1}}, q44{8, {1, 1, 1, 1, 0, 0, 0, 0}};
-    const LoopPath p42r{6, {0, 0, 0, 0, 1, 1}}, q42r{6, {1, 1, 0, 0, 0, 0}};
-    const LoopPath p21a{3, {0, 0, 1}}, q21a{3, {1, 0, 0}};
-    const LoopPath p21b{3, {0, 1, 1}}, q21b{3, {1, 1, 0}};
-    const long units = 6L * geo.V;
-    const long stride = (long)gridDim.x * nw * LPW;
-    for (long u = ((long)blockIdx.x * nw + warp) * LPW + g; u < units; u += stride) {
+    const LoopPath p22{4, 0xcu}, q22{4, 0x3u};
+    const LoopPath p42u{6, 0x3cu}, q42u{6, 0xfu};
+    const LoopPath p44{8, 0xf0u}, q44{8, 0xfu};
+    const LoopPath p42r{6, 0x30u}, q42r{6, 0x3u};
+    const LoopPath p21a{3, 0x4u}, q21a{3, 0x1u};
+    const LoopPath p21b{3, 0x6u}, q21b{3, 0x3u};
+    const long stride = (long)gridDim.x * gpc;
+#pragma unroll 1
+    for (long u = w.id; u < units; u += stride) {
       const int pl = (int)(u / geo.V);
       const int x = (int)(u - (long)pl * geo.V);
       q.mu = pl < 3 ? 0 : (pl < 5 ? 1 : 2);
@@ -146,41 +109,41 @@ __global__ void __launch_bounds__(256, 1)
       coords(geo, x, q.X);
       int pi = 0, pj = 0, qi = 0, qj = 0;
       // 2x2
-      loop_chain(q, P, S, p22, 0, pi, pj, L);
-      loop_chain(q, Q, S, q22, 0, qi, qj, L);
-      trace_dag_acc(P, Q, N, L, a22);
+      loop_chain<G>(q, P, S, p22, 0, pi, pj);
+      loop_chain<G>(q, Q, S, q22, 0, qi, qj);
+      trace_dag_acc<G>(P, Q, N, a22);
       // 2x4 up: P = bl cd extended by cu
-      loop_chain(q, P, S, p42u, 4, pi, pj, L);
+      loop_chain<G>(q, P, S, p42u, 4, pi, pj);
       qi = qj = 0;
-      loop_chain(q, Q, S, q42u, 0, qi, qj, L);
-      trace_dag_acc(P, Q, N, L, a42);
+      loop_chain<G>(q, Q, S, q42u, 0, qi, qj);
+      trace_dag_acc<G>(P, Q, N, a42);
       // 4x4: Q = ld lu tl extended by tr
-      loop_chain(q, Q, S, q44, 6, qi, qj, L);
+      loop_chain<G>(q, Q, S, q44, 6, qi, qj);
       pi = pj = 0;
-      loop_chain(q, P, S, p44, 0, pi, pj, L);
-      trace_dag_acc(P, Q, N, L, a44);
+      loop_chain<G>(q, P, S, p44, 0, pi, pj);
+      trace_dag_acc<G>(P, Q, N, a44);
       // 2x4 right
       pi = pj = qi = qj = 0;
-      loop_chain(q, P, S, p42r, 0, pi, pj, L);
-      loop_chain(q, Q, S, q42r, 0, qi, qj, L);
-      trace_dag_acc(P, Q, N, L, a42);
+      loop_chain<G>(q, P, S, p42r, 0, pi, pj);
+      loop_chain<G>(q, Q, S, q42r, 0, qi, qj);
+      trace_dag_acc<G>(P, Q, N, a42);
       // 1x2, both orientations
       pi = pj = qi = qj = 0;
-      loop_chain(q, P, S, p21a, 0, pi, pj, L);
-      loop_chain(q, Q, S, q21a, 0, qi, qj, L);
-      trace_dag_acc(P, Q, N, L, a21);
+      loop_chain<G>(q, P, S, p21a, 0, pi, pj);
+      loop_chain<G>(q, Q, S, q21a, 0, qi, qj);
+      trace_dag_acc<G>(P, Q, N, a21);
       pi = pj = qi = qj = 0;
-      loop_chain(q, P, S, p21b, 0, pi, pj, L);
-      loop_chain(q, Q, S, q21b, 0, qi, qj, L);
-      trace_dag_acc(P, Q, N, L, a21);
+      loop_chain<G>(q, P, S, p21b, 0, pi, pj);
+      loop_chain<G>(q, Q, S, q21b, 0, qi, qj);
+      trace_dag_acc<G>(P, Q, N, a21);
     }
   }
   __syncthreads();
-  const int ngroups = nw * LPW;
   for (int e = threadIdx.x; e < row; e += blockDim.x) {
     double2 sum = cz();
-    for (int gi = 0; gi < ngroups; gi++)
-      sum = cadd(sum, sm[(size_t)gi * gsz + (size_t)LOOP_SLOTS * SS + e]);
+    const int gs = group_stride(LOOP_SLOTS + LOOP_EXTRA, SS);
+    for (int g = 0; g < gpc && (long)blockIdx.x * gpc + g < units; g++)
+      sum = cadd(sum, sm[LEAD + g * gs + LOOP_SLOTS * SS + e]);
     partial[(size_t)blockIdx.x * row + e] = sum;
   }
 }

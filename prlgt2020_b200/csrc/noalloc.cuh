@@ -25,162 +25,6 @@ constexpr int NOALLOC_MAX_DEVICES = 64;
 // (NOALLOC_BLOCKS + 1) rows of NOALLOC_ROW complex doubles: 803,600 bytes
 static __device__ __align__(256) double2 g_noalloc_scratch[(NOALLOC_BLOCKS + 1) * NOALLOC_ROW];
 
-struct AosField {
-  const double2 *p;  // V * 4 series of 1 + 9A complex doubles (site, mu)
-  int A;             // allocORD of the caller's layout (>= N)
-  int N;
-  int SS;
-  Geo g;
-};
-
-// Copy link (mu, n.site) of an AoS field into a column-major slot (DAG:
-// its dagger), applying the twists of the faces the read crossed; a twisted
-// link gets flag 1 (nspt.cc:115-121).
-__device__ __forceinline__ void stage_aos(double2 *slot, const AosField &f, int mu, Nb n,
-                                          const Lane &L, bool dag = false) {
-  const double2 *src = f.p + ((size_t)n.site * 4 + mu) * (1 + 9 * (size_t)f.A);
-  const unsigned tb = n.bwd & f.g.twist, tf = n.fwd & f.g.twist;
-  if (!(tb | tf)) {
-    const int r = L.j / 3, c = L.j - 3 * (L.j / 3);
-    const int off = dag ? 3 * r + c : 3 * c + r;
-    for (int k = 1; k <= f.N; k++) {
-      const double2 v = __ldg(src + 1 + 9 * (k - 1) + L.j);
-      slot[1 + 9 * (k - 1) + off] = dag ? cconj(v) : v;
-    }
-    if (L.j == 0) {
-      const double2 fl = __ldg(src);
-      slot[0] = dag ? cconj(fl) : fl;
-    }
-  } else {
-    for (int k = 1 + L.j; k <= f.N; k += GROUP) {
-      double2 m[9];
-#pragma unroll
-      for (int e = 0; e < 9; e++) m[e] = __ldg(src + 1 + 9 * (k - 1) + e);
-      twist3(m, tb, tf);
-      double2 *p = slot + 1 + 9 * (k - 1);
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) p[dag ? 3 * r + c : 3 * c + r] = dag ? cconj(m[3 * r + c]) : m[3 * r + c];
-    }
-    if (L.j == 0) slot[0] = make_double2(1.0, 0.0);
-  }
-  __syncwarp(L.mask);
-}
-
-// Per-CTA partial sums of Tr(U_mu(x) * staples) per order.  Groups walk the
-// links grid-stride; each lane keeps the orders k = 1 + j (mod 9) it owns in
-// registers; the CTA sums its groups in a fixed order into partial[blockIdx].
-constexpr int NOALLOC_PER_LANE = (NSPT_MAX_ORDER + GROUP - 1) / GROUP;
-
-__global__ void __launch_bounds__(256, 1) k_plaq_noalloc(AosField f, double2 *partial) {
-  extern __shared__ double2 sm[];
-  Lane L;
-  int g;
-  const bool grouped = make_lane(L, g);
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int N = f.N, SS = f.SS;
-  double2 acc[NOALLOC_PER_LANE];
-#pragma unroll
-  for (int q = 0; q < NOALLOC_PER_LANE; q++) acc[q] = cz();
-  double2 acc0 = cz();
-  if (grouped) {
-    const int c = L.c;
-    double2 *W = sm + (size_t)(warp * LPW + g) * (3 * SS), *T = W + SS, *Y = T + SS;
-    const long nl = 4L * f.g.V;
-    const long stride = (long)gridDim.x * nw * LPW;
-    for (long link = ((long)blockIdx.x * nw + warp) * LPW + g; link < nl; link += stride) {
-      const int mu = (int)(link / f.g.V);
-      const int site = (int)(link - (long)mu * f.g.V);
-      int x[4];
-      coords(f.g, site, x);
-      Nb self;
-      self.site = site;
-      self.fwd = self.bwd = 0;
-      double2 wflag = cz();
-      bool first = true;
-      for (int nu = 0; nu < 4; nu++) {
-        if (nu == mu) continue;
-        // upper staple, as the dagger of U_nu(x) U_mu(x+nu) U_nu(x+mu)^dag
-        // (QCDenvNODEpt_test.h:555), accumulated transposed and conjugated
-        {
-          stage_aos(T, f, nu, self, L);
-          stage_aos(Y, f, mu, neighbour(f.g, x, nu, 1), L);
-          const double2 t0 = T[0], y0 = Y[0];
-          product<MO, false>(LeftS{T}, t0, Y, y0, N, L,
-                             [&](int k, int r, double2 v) { T[sidx(k, r, c)] = v; });
-          if (L.j == 0) T[0] = flag_mul(t0, y0);
-          __syncwarp(L.mask);
-          stage_aos(Y, f, nu, neighbour(f.g, x, mu, 1), L, true);
-          const double2 a0 = T[0], b0 = Y[0];
-          const bool f0 = first;
-          product<MO, false>(LeftS{T}, a0, Y, b0, N, L, [&](int k, int r, double2 v) {
-            double2 &w = W[sidx(k, c, r)];
-            w = f0 ? cconj(v) : cadd(w, cconj(v));
-          });
-          const double2 fl = cconj(flag_mul(a0, b0));
-          wflag = first ? fl : cadd(wflag, fl);
-          first = false;
-          __syncwarp(L.mask);
-        }
-        // lower staple [U_mu(x-nu) U_nu(x-nu+mu)]^dag U_nu(x-nu) (QCDenvNODEpt_test.h:556)
-        {
-          const Nb d = neighbour(f.g, x, nu, -1);
-          stage_aos(Y, f, nu, neighbour(f.g, x, nu, -1, mu, 1), L);
-          stage_aos(T, f, mu, d, L);
-          const double2 a0 = T[0], y0 = Y[0];
-          product<MO, false>(LeftS{T}, a0, Y, y0, N, L,
-                             [&](int k, int r, double2 v) { T[sidx(k, r, c)] = v; });
-          if (L.j == 0) T[0] = flag_mul(a0, y0);
-          __syncwarp(L.mask);
-          stage_aos(Y, f, nu, d, L);
-          const double2 ta = cconj(T[0]);
-          product<MO, true>(LeftS{T}, ta, Y, Y[0], N, L, [&](int k, int r, double2 v) {
-            double2 &w = W[sidx(k, r, c)];
-            w = cadd(w, v);
-          });
-          wflag = cadd(wflag, flag_mul(ta, Y[0]));
-          __syncwarp(L.mask);
-        }
-      }
-      if (L.j == 0) W[0] = wflag;
-      // Tr(U_mu(x) * staples) per order (ptSU3::Tr, QCDpt.cc:115-122)
-      stage_aos(Y, f, mu, self, L);
-      const double2 pflag = flag_mul(Y[0], wflag);
-      product<MO, false>(LeftS{Y}, Y[0], W, wflag, N, L,
-                         [&](int k, int r, double2 v) { T[sidx(k, r, c)] = v; });
-      __syncwarp(L.mask);
-      if (L.j == 0) acc0 = cadd(acc0, make_double2(3. * pflag.x, 3. * pflag.y));
-#pragma unroll
-      for (int q = 0; q < NOALLOC_PER_LANE; q++) {
-        const int k = 1 + L.j + GROUP * q;
-        if (k <= N)
-          acc[q] = cadd(acc[q], cadd(cadd(T[sidx(k, 0, 0)], T[sidx(k, 1, 1)]), T[sidx(k, 2, 2)]));
-      }
-      __syncwarp(L.mask);
-    }
-  }
-  // CTA reduction in a fixed order over the groups (the slots are free now)
-  __syncthreads();
-  const int ngroups = nw * LPW;
-  double2 *red = sm;  // [ngroups][N + 1]
-  if (grouped) {
-    double2 *row = red + (size_t)(warp * LPW + g) * (N + 1);
-    if (L.j == 0) row[0] = acc0;
-#pragma unroll
-    for (int q = 0; q < NOALLOC_PER_LANE; q++) {
-      const int k = 1 + L.j + GROUP * q;
-      if (k <= N) row[k] = acc[q];
-    }
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k <= N; k += blockDim.x) {
-    double2 s = cz();
-    for (int gi = 0; gi < ngroups; gi++) s = cadd(s, red[(size_t)gi * (N + 1) + k]);
-    partial[(size_t)blockIdx.x * NOALLOC_ROW + k] = s;
-  }
-}
-
 // Sum the CTAs' partial rows in block order into the result row.
 __global__ void k_plaq_noalloc_sum(const double2 *partial, int nblocks, int N, double2 *out) {
   for (int k = threadIdx.x; k <= N; k += blockDim.x) {
@@ -221,7 +65,7 @@ int noalloc_setup(int dev, NoallocDevice **out) {
     if (cudaDeviceGetAttribute(&d.smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
         cudaSuccess)
       return NSPT_ERR_CUDA;
-    if (cudaFuncSetAttribute(k_plaq_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(k_plaq_trace<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              d.smem_optin) != cudaSuccess)
       return NSPT_ERR_CUDA;
     // twist matrices (twistmatrices.h:158-240), the values nspt_create uploads
@@ -272,40 +116,29 @@ extern "C" int nspt_plaquette_measure_noalloc(const void *links_dev, int allocOR
   int rc = noalloc_setup(dev, &d);
   if (rc) return rc;
 
-  AosField f;
-  f.p = static_cast<const double2 *>(links_dev);
-  f.A = allocORD;
-  f.N = N;
-  f.SS = 1 + 9 * N;
-  while (f.SS % 8 != 3) f.SS++;  // bank quads: see series.cuh
-  Geo &g = f.g;
+  const size_t ser = 1 + 9 * (size_t)allocORD;
+  const int SS = (int)link_rec(N);
+  Geo g;
   for (int k = 0; k < 4; k++) g.L[k] = L[k];
   g.s2 = L[3];
   g.s1 = L[2] * g.s2;
   g.s0 = L[1] * g.s1;
   g.V = (int)V;
-  g.t0 = g.t1 = 1;
-  g.t2 = L[2];
   g.twist = 0;
   if (flags & NSPT_TWIST_Y) g.twist |= 2u;
   if (flags & NSPT_TWIST_Z) g.twist |= 4u;
   if (flags & NSPT_TWIST_T) g.twist |= 8u;
 
-  // 3 slots per group; as many warps (<= 8) as shared memory allows
-  const size_t per_warp = (size_t)LPW * 3 * f.SS * sizeof(double2);
-  const int warps = (int)std::min<size_t>(8, (size_t)d->smem_optin / per_warp);
-  if (warps < 1) return NSPT_ERR_ORDER;
-  const size_t smem = std::max((size_t)warps * per_warp,
-                               (size_t)warps * LPW * (N + 1) * sizeof(double2));
-  if (smem > (size_t)d->smem_optin) return NSPT_ERR_ORDER;
-  const long groups = 4 * V;
-  const long per_cta = (long)warps * LPW;
-  const long want = (groups + per_cta - 1) / per_cta;
+  const Shape sh = group_shape(32, 4, MEASURE_SLOTS, SS, (size_t)d->smem_optin);
+  if (sh.gpc < 1) return NSPT_ERR_ORDER;
+  const long want = (6 * V + sh.gpc - 1) / sh.gpc;
   const int blocks = (int)std::min<long>(want, NOALLOC_BLOCKS);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   double2 *partial = d->scratch;
   double2 *result = d->scratch + (size_t)NOALLOC_BLOCKS * NOALLOC_ROW;
-  k_plaq_noalloc<<<blocks, 32 * warps, smem, st>>>(f, partial);
+  const double2 *U = static_cast<const double2 *>(links_dev);
+  k_plaq_trace<32><<<blocks, 32 * sh.warps, sh.smem, st>>>(U, ser, N, SS, g, partial, NOALLOC_ROW,
+                                                       sh.gpc);
   if (cudaGetLastError() != cudaSuccess) return NSPT_ERR_CUDA;
   k_plaq_noalloc_sum<<<1, 64, 0, st>>>(partial, blocks, N, result);
   if (cudaGetLastError() != cudaSuccess) return NSPT_ERR_CUDA;

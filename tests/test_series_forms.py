@@ -1,0 +1,95 @@
+"""The series kernels where their forms and blocks change, against the oracle
+(GPU, through the C ABI).
+
+A launch takes one of three forms of the Cauchy product: 9 lanes per link
+(launches of at least 24 links per SM, up to 14 orders), a warp per link, and
+the ordered sums (zero modes or Fourier-accelerated gauge fixing above 14
+orders).  A product works on blocks of 8 orders, the lowest of which may stick
+out below order 1; the exponential serves two orders per lane.  The Wilson
+sweep goes plaquette by plaquette, in slabs of direction 0 on large lattices,
+and link by link where a flag other than 1 meets a twisted face.
+
+Tolerance: that of tests/test_gpu_parity.py, 1e-12 per order after one sweep
+(a few hundred roundings of 1e-16 in sums of terms of the coefficients' size).
+"""
+import numpy as np
+import pytest
+
+from helpers import flag_diff, obs_close, per_order_rel
+
+pytestmark = pytest.mark.gpu
+
+TWIST = {"y": 2, "z": 4, "t": 8}
+
+
+def one_sweep(P, O, L, N, twist="", start=3, links=None, **kw):
+    o = O.Oracle(L, N, twist_mask=sum(TWIST[d] for d in twist))
+    o.random_start(start, 0.5)
+    if links is not None:
+        links(o.links)
+    e = P.NsptEngine(L, N, twist=twist, **kw)
+    e.upload(o.links)
+    nz = O.Rand55(11).gauss(o.V * 32)
+    e.set_noise(nz)
+    eo = e.gauge_wilson(0.01)
+    oo = o.sweep(0.01, nz, zero_modes=bool(kw.get("zero_modes")))
+    for a, b in ((eo.plaq, oo.plaq), (eo.norm, oo.norm), (eo.tru, oo.tru)):
+        ok, worst = obs_close(a, b, 1e-12)
+        assert ok, worst
+    return e, o
+
+
+@pytest.mark.parametrize("L", [(2, 2, 2, 2), (6, 6, 5, 6)], ids=["warp_per_link", "nine_lanes"])
+@pytest.mark.parametrize("N", [1, 2, 7, 8, 9, 14])
+def test_block_edges(engine_mod, oracle_mod, L, N):
+    """One sweep at the edges of the product's blocks, in the form for few
+    links (64) and for many (4320)."""
+    e, o = one_sweep(engine_mod, oracle_mod, L, N)
+    assert per_order_rel(e.download(), o.links, N).max() <= 1e-12
+    assert flag_diff(e.download(), o.links, N) == 0.0
+
+
+@pytest.mark.parametrize("N", [15, 17, 18, 31, 33])
+def test_high_order_edges(engine_mod, oracle_mod, N):
+    """One sweep at orders above the 9-lane form: past two blocks, and where
+    the exponential's second order per lane begins."""
+    e, o = one_sweep(engine_mod, oracle_mod, (2, 2, 2, 4), N)
+    assert per_order_rel(e.download(), o.links, N).max() <= 1e-12
+
+
+@pytest.mark.parametrize("L,N,twist", [((9, 10, 10, 12), 2, ""), ((9, 10, 10, 12), 2, "yzt"),
+                                       ((3, 4, 3, 5), 5, "yz")],
+                         ids=["slabs_4_4_1", "slabs_twisted", "whole_odd_twisted"])
+def test_plaquette_slabs(engine_mod, oracle_mod, L, N, twist):
+    """The sweep in slabs (the first needs the last plane's plaquettes, the
+    last slab is shorter) and on a whole odd lattice."""
+    e, o = one_sweep(engine_mod, oracle_mod, L, N, twist=twist)
+    assert per_order_rel(e.download(), o.links, N).max() <= 1e-12
+    ok, worst = obs_close(e.plaquette_measure(), o.plaquette(), 1e-12)
+    assert ok, worst
+
+
+@pytest.mark.parametrize("twist", ["", "yz"])
+def test_flags_other_than_one(engine_mod, oracle_mod, twist):
+    """Flags that are not 1: general flag terms of every product and, across a
+    twisted face, the link-by-link sweep and the four views of a plaquette."""
+    def flags(links):
+        rng = np.random.default_rng(5)
+        links[:, :, :2] = rng.normal(size=links[:, :, :2].shape)
+
+    e, o = one_sweep(engine_mod, oracle_mod, (4, 2, 3, 4), 5, twist=twist, links=flags)
+    assert per_order_rel(e.download(), o.links, 5).max() <= 1e-12
+    ok, worst = obs_close(e.plaquette_measure(), o.plaquette(), 1e-12)
+    assert ok, worst
+
+
+@pytest.mark.parametrize("N", [14, 15, 20])
+def test_logarithms_across_the_ordered_form(engine_mod, oracle_mod, N):
+    """A sweep with zero modes on the two sides of the order where the sums
+    are kept in order.  The logarithm amplifies rounding by about 4 per order:
+    max(1e-12, 1e-16 * 4^k) per order."""
+    e, o = one_sweep(engine_mod, oracle_mod, (4, 4, 2, 4), N, zero_modes=True)
+    e.zero_modes_subtraction()
+    o.zero_modes()
+    rel = per_order_rel(e.download(), o.links, N)
+    assert np.all(rel <= np.maximum(1e-12, 1e-16 * 4.0 ** np.arange(1, N + 1))), rel
