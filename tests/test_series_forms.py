@@ -93,3 +93,17 @@ def test_logarithms_across_the_ordered_form(engine_mod, oracle_mod, N):
     o.zero_modes()
     rel = per_order_rel(e.download(), o.links, N)
     assert np.all(rel <= np.maximum(1e-12, 1e-16 * 4.0 ** np.arange(1, N + 1))), rel
+
+
+def test_large_fields_cross_the_bus_whole(engine_mod):
+    """Upload and download of a field that goes through the pinned buffers
+    (28.7 MB: 14 chunks and a part of one), and of part of its orders."""
+    P = engine_mod
+    L, N = (8, 8, 8, 12), 8
+    rng = np.random.default_rng(9)
+    a = rng.normal(size=(int(np.prod(L)), 4, P.series_len(N)))
+    with P.NsptEngine(L, N) as e, P.NsptEngine(L, N - 1) as f:
+        e.upload(a)
+        assert np.array_equal(e.download(), a)
+        f.upload(a, allocORD=N)
+        assert np.array_equal(f.download(), a[:, :, :P.series_len(N - 1)])
