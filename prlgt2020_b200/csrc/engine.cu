@@ -1158,10 +1158,14 @@ static int loop_sums(nspt_ctx *ctx, std::vector<double2> &h) {
   int rc = timed_begin(ctx);
   if (rc) return rc;
   measure_form(ctx, units, [&](auto G) {
+    // the two-link lines go where the next sweep's field will
+    rc = wlaunch(ctx, G, k_lines<G.value>, 2, 4L * ctx->V, "lines", (const double2 *)ctx->U, ctx->F,
+                 N, ctx->SS, ctx->geo);
+    if (rc) return;
     cudaFuncSetAttribute(k_loops<G.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)ctx->smem_optin);
-    k_loops<G.value><<<grid, 32 * sh.warps, sh.smem, ctx->st>>>(ctx->U, N, ctx->SS, ctx->geo, part,
-                                                                sh.gpc);
+    k_loops<G.value><<<grid, 32 * sh.warps, sh.smem, ctx->st>>>(ctx->U, ctx->F, N, ctx->SS,
+                                                                ctx->geo, part, sh.gpc);
   });
   if (rc) return rc;
   CK(cudaGetLastError());
