@@ -154,8 +154,8 @@ int nspt_set_gf_grid(nspt_ctx *ctx, const int grid[4]);
  * local gauge fixing and the on-the-fly sweep; both visit the sites in the
  * grid's order and give the same links to rounding.  NSPT_LGF_GROUP: 9 lanes
  * per reference thread (orders below 18; above, as TEAM).  NSPT_LGF_TEAM: a
- * warp per thread, a third of the instructions in a row: shorter latency for
- * grids with few threads.  NSPT_LGF_AUTO (the default): by the number of
+ * CTA per thread in the gauge fixing, a warp in the on-the-fly sweep: shorter
+ * latency for grids with few threads.  NSPT_LGF_AUTO (the default): by the number of
  * threads and the order.  Anything else: NSPT_ERR_ARG. */
 #define NSPT_LGF_AUTO 0
 #define NSPT_LGF_GROUP 1

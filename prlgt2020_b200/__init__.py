@@ -287,9 +287,9 @@ class NsptEngine:
 
     def set_local_gf_form(self, form: str):
         """Form of the kernels that follow the thread grid: "group" (9 lanes
-        per reference thread), "team" (a warp per thread) or "auto" (by the
-        number of threads and the order).  Both give the same links to
-        rounding."""
+        per reference thread), "team" (a CTA per thread in the gauge
+        fixing, a warp in the on-the-fly sweep) or "auto" (by the number of
+        threads and the order).  Both give the same links to rounding."""
         code = {"auto": 0, "group": 1, "team": 2}.get(form)
         if code is None:
             raise ValueError(f"local gauge fixing form {form!r}: auto, group or team")

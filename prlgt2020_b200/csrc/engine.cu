@@ -573,8 +573,43 @@ static int do_fa(nspt_ctx *ctx, double alpha) {
   return NSPT_OK;
 }
 
+// Whether a barrier step of the local gauge fixing has a team (k_local_gf_team)
+// and not a group per reference thread.  A team is the shorter chain, a CTA of 8
+// warps for it the dearer occupancy: 12^4 N=8 with blocks of 2 (16 steps of 1296
+// threads) takes 1.16 ms with teams and 0.63 with groups, 10^3*8 (500 threads)
+// 0.505 and 0.53, 8^4 (256) 0.30 and 0.52, 6*8*8*9 N=11 (48 threads, 9 sites
+// each) 1.28 and 3.18.  So teams serve up to two waves of the CTAs that fit, and
+// the ORDERED form, with one team on an SM, one: 6*8*8*9 N=15 4.7 and 7.5 ms,
+// but 8^4 N=16 2.5 and 2.1.
+template <int G>
+static bool team_fits(const nspt_ctx *ctx, long nthr, size_t &smem) {
+  smem = (LEAD + (size_t)team_slots<G>() * group_stride(1, ctx->SS)) * sizeof(double2);
+  if (ctx->gf_form == NSPT_LGF_GROUP || smem > ctx->smem_optin) return false;
+  if (ctx->gf_form == NSPT_LGF_TEAM) return true;
+  const long fit = std::min<long>(G == ORDERED ? 1 : 2, (long)(228 * 1024 / (smem + 1024)));
+  return nthr <= (G == ORDERED ? 1 : 2) * fit * ctx->nsm;
+}
+
+template <int G>
+static bool local_gf_team(nspt_ctx *ctx, const double2 *Ut, double alpha, const LgfGrid &gr,
+                          long steps, int &rc) {
+  size_t smem;
+  if (!team_fits<G>(ctx, gr.nthr, smem)) return false;
+  cudaFuncSetAttribute(k_local_gf_team<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)ctx->smem_optin);
+  for (long p = 0; p < steps; p++)
+    k_local_gf_team<G><<<(unsigned)gr.nthr, 32 * TEAM_WARPS, smem, ctx->st>>>(
+        ctx->U, Ut, ctx->N, ctx->SS, ctx->geo, alpha, gr, p);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    ctx->err = std::string("local gauge fixing: ") + cudaGetErrorString(e);
+    rc = NSPT_ERR_CUDA;
+  }
+  return true;
+}
+
 // stochastic_gauge_fixing (nspt.cc:660-862) with the context's thread
-// grid: one launch per barrier step, one group per reference thread.
+// grid: one launch per barrier step, a team or a group per reference thread.
 static int do_local_gf(nspt_ctx *ctx, double alpha) {
   long steps;
   const LgfGrid gr = thread_grid(ctx, steps);
@@ -583,6 +618,9 @@ static int do_local_gf(nspt_ctx *ctx, double alpha) {
   const double2 *Ut = ctx->snap_valid ? ctx->F : ctx->U;
   ctx->lg_current = false;
   int rc = NSPT_OK;
+  if (ordered(ctx) ? local_gf_team<ORDERED>(ctx, Ut, alpha, gr, steps, rc)
+                   : local_gf_team<32>(ctx, Ut, alpha, gr, steps, rc))
+    return rc;
   with_grid_form(ctx, gr.nthr, [&](auto G) {
     for (long p = 0; p < steps && !rc; p++)
       rc = wlaunch(ctx, G, k_local_gf<G.value>, lgf_slots<G.value>(), gr.nthr, "local gauge fixing", ctx->U, Ut,

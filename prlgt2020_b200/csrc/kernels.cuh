@@ -917,6 +917,8 @@ __global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
 // (twist_mu(exp(-alpha W)) = Omega W2 Omega^dag when x-mu wraps a twisted
 // face, nspt.cc:690-719).  alpha W is antihermitian, so exp(-alpha W) is the
 // dagger of exp(alpha W): one exponential and daggered products.
+constexpr int TEAM_WARPS = 8;
+
 template <int G>
 __host__ __device__ constexpr int lgf_slots() {
   return G == ORDERED ? 4 : 3;
@@ -1005,6 +1007,106 @@ __global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
     // the next site's copies read links written here
     __threadfence();
     gsync<G>();
+  }
+}
+
+// The same by a team: a CTA per reference thread, for barrier steps with few
+// threads, where the time is that of one site's chain.  The site's eight links
+// are staged at once, by all groups of the CTA (task t < 4: U_t(x), t >= 4:
+// U_{t-4}(x-mu)), the exponential is one group's (ORDERED: exp(alpha W) and
+// exp(-alpha W) two groups'), and the eight products are dealt to the groups from
+// the staged copies (no other thread writes those links between the barriers).
+// Slots: the eight links, four twisted copies, X and the exponential's.
+template <int G>
+__host__ __device__ constexpr int team_slots() {
+  return G == ORDERED ? 17 : 15;
+}
+
+template <int G>
+__global__ void __launch_bounds__(32 * TEAM_WARPS, G == ORDERED ? 1 : 2)
+    k_local_gf_team(double2 *U, const double2 *Ut, int N, int SS, Geo geo, double alpha,
+                    LgfGrid gr, long step) {
+  double2 *sm = wsm();
+  const int g = (threadIdx.x & 31) / glanes<G>(), per = 32 / glanes<G>();
+  const int workers = (blockDim.x >> 5) * per;
+  const int me = g < per ? (threadIdx.x >> 5) * per + g : workers;  // workers: a lane without
+  const int lane = glane<G>(), n = (int)link_rec(N), GS = group_stride(1, SS);
+  const int S = LEAD, Tw = S + 8 * GS, X = Tw + 4 * GS, Y = X + GS, E = Y + GS;
+  const double D3 = 1.0 / 3.0;
+  const LgfWalk walk(gr, blockIdx.x, step);
+#pragma unroll 1
+  for (long r = 0; r < gr.seg; r++) {
+    int x[4];
+    walk.site(gr, geo, r, x);
+    const int site = x[0] * geo.s0 + x[1] * geo.s1 + x[2] * geo.s2 + x[3];
+    for (int t = me; t < 8; t += workers) {
+      const int mu = t & 3;
+      const Nb bn = neighbour(geo, x, mu, -1);
+      wstage<G>(S + t * GS, U + link_at(mu, t < 4 ? site : bn.site, N), n);
+      // a back link read across a twisted face, as the step's start field has it
+      if (t >= 4 && Ut != U && (bn.bwd & geo.twist))
+        wstage<G>(Tw + mu * GS, Ut + link_at(mu, bn.site, N), n);
+    }
+    cp_commit();
+    cp_wait0();
+    __syncthreads();
+    // alpha Trless(W - W^dag), W = sum_mu U_mu(x) - U_mu(x-mu), a thread per order
+    for (int k = 1 + threadIdx.x; k <= N; k += blockDim.x) {
+      double2 w[9], b[9];
+#pragma unroll
+      for (int mu = 0; mu < 4; mu++) {
+        const unsigned tb = neighbour(geo, x, mu, -1).bwd & geo.twist;
+        const double2 *f = sm + S + mu * GS + 9 * k - 8;
+        const double2 *q = sm + (tb && Ut != U ? Tw + mu * GS : S + (4 + mu) * GS) + 9 * k - 8;
+        double2 m[9];
+#pragma unroll
+        for (int e = 0; e < 9; e++) m[e] = q[e];
+        if (tb) twist3(m, tb, 0u);
+#pragma unroll
+        for (int e = 0; e < 9; e++) w[e] = cadd(mu == 0 ? cz() : w[e], csub(f[e], m[e]));
+      }
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int q = 0; q < 3; q++) b[3 * i + q] = csub(w[3 * i + q], cconj(w[3 * q + i]));
+      const double2 tr = cadd(cadd(b[0], b[4]), b[8]);
+      const double2 z = make_double2(D3 * tr.x, D3 * tr.y);
+      b[0] = csub(b[0], z);
+      b[4] = csub(b[4], z);
+      b[8] = csub(b[8], z);
+      double2 *o = sm + X + 9 * k - 8;
+#pragma unroll
+      for (int e = 0; e < 9; e++) o[e] = cscale(b[e], alpha);
+    }
+    if (threadIdx.x == 0) sm[X] = cz();
+    __syncthreads();
+    int P = X, M = X;
+    if constexpr (G == ORDERED) {
+      P = E;
+      M = E + 2 * GS;
+      if (me == 0) ser_exp_horner<G, true>(X, Y, P, N);
+      if (me == 1) ser_exp_horner<G, true>(X, E + GS, M, N, -1.0);
+    } else {
+      if (me == 0) ser_exp<G, true>(X, Y, E, N);
+    }
+    __syncthreads();
+    for (int t = me; t < 8; t += workers) {
+      const int mu = t & 3, A = S + t * GS;
+      const bool fwd = t < 4;
+      const Nb back = neighbour(geo, x, mu, -1);
+      int R = M;
+      if (!fwd && ((back.bwd & geo.twist) >> mu & 1u)) {
+        R = Tw + mu * GS;
+        for (int e = lane; e < n; e += glanes<G>()) sm[R + e] = sm[M + e];
+        gsync<G>();
+        wtwist<G>(R, 0u, 1u << mu, N);
+      }
+      ser_mul<G>(A, fwd ? P : A, fwd ? A : R, N, fwd || G == ORDERED ? MUL_DAG : MUL_DB);
+      wstore<G>(U + link_at(mu, fwd ? site : back.site, N), A, n);
+    }
+    // the next site's copies read links written here
+    __threadfence();
+    __syncthreads();
   }
 }
 

@@ -95,6 +95,24 @@ def test_logarithms_across_the_ordered_form(engine_mod, oracle_mod, N):
     assert np.all(rel <= np.maximum(1e-12, 1e-16 * 4.0 ** np.arange(1, N + 1))), rel
 
 
+@pytest.mark.parametrize("zero_modes,N", [(False, 1), (False, 9), (False, 19), (True, 15)],
+                         ids=["n1", "n9", "n19", "ordered"])
+def test_local_gf_teams(engine_mod, oracle_mod, zero_modes, N):
+    """Local gauge fixing by a team and by a group per reference thread, three
+    sites to a thread (odd t), across a twisted face (zero modes: periodic)."""
+    L, twist = (4, 2, 4, 3), "" if zero_modes else "z"
+    for form in ("team", "group"):
+        o = oracle_mod.Oracle(L, N, twist_mask=TWIST.get(twist, 0))
+        o.random_start(7, 0.5)
+        e = engine_mod.NsptEngine(L, N, twist=twist, zero_modes=zero_modes)
+        e.set_gf_grid((2, 1, 2, 1))
+        e.set_local_gf_form(form)
+        e.upload(o.links)
+        e.stochastic_gauge_fixing(-0.05)
+        o.local_gauge_fix(-0.05, grid=(2, 1, 2, 1))
+        assert per_order_rel(e.download(), o.links, N).max() <= 1e-12, form
+
+
 def test_large_fields_cross_the_bus_whole(engine_mod):
     """Upload and download of a field that goes through the pinned buffers
     (28.7 MB: 14 chunks and a part of one), and of part of its orders."""
