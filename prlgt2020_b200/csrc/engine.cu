@@ -272,12 +272,49 @@ static LgfGrid thread_grid(const nspt_ctx *ctx, long &steps) {
   return gr;
 }
 
+// Whether the on-the-fly sweep takes a site's staples ahead of its links
+// (k_otf_parts): periodic fields, whose F is free (a twisted one holds the step's
+// start field there) and large enough, with no extent of 1 (no link of the site
+// is then its own neighbour).  The ORDERED form keeps its order of sums.  Steps
+// of many threads at low orders have warps enough to hide a link's chain, and the
+// parts' way through memory costs more: in one launch and in parts, 16^4 (4096
+// threads) N=6 4.5 and 5.1 ms, N=9 7.1 and 6.5, 24^4 (20736) N=8 19.6 and 20.5,
+// N=10 32.4 and 31.6; 12^4 (1296) N=8 3.03 and 2.16, 16*14^3 (2744) N=4 5.4 and
+// 3.4, 8^4 (256) N=11 3.9 and 2.1.
+static bool otf_in_parts(const nspt_ctx *ctx, const LgfGrid &gr) {
+  for (int d = 0; d < 4; d++)
+    if (ctx->L[d] < 2) return false;
+  return ctx->c1 == 0.0 && !ctx->geo.twist && !ordered(ctx) &&
+         (gr.nthr < 24L * ctx->nsm || ctx->N > BLK) && (long)OTF_PARTS * gr.nthr <= 4L * ctx->V;
+}
+
 // gauge_wilson on the fly (UPDATE_ONTHEFLY, nspt.cc:355-460): one launch per
-// barrier step of the thread grid, one group per reference thread.
+// barrier step of the thread grid, or two per site of its walk; one group per
+// reference thread.
 static int launch_sweep_otf(nspt_ctx *ctx, const SweepArgs &a) {
   long steps;
   const LgfGrid gr = thread_grid(ctx, steps);
   int rc = NSPT_OK;
+  if (otf_in_parts(ctx, gr)) {
+    const long parts = (long)OTF_PARTS * gr.nthr;
+    // all of a link's operands at once where every group then still has its place
+    const bool wide = gr.nthr * (long)(group_stride(OTF_LINK_SLOTS_WIDE, ctx->SS) * sizeof(double2)) <=
+                      ctx->nsm * 200L * 1024;
+    for (long p = 0; p < steps; p++)
+      for (long r = 0; r < gr.seg && !rc; r++) {
+        with_form(ctx, parts, [&](auto G) {
+          rc = wlaunch(ctx, G, k_otf_parts<G.value>, 3, parts, "on-the-fly sweep, staples", a, gr, p,
+                       r, ctx->F);
+        });
+        if (rc) break;
+        with_grid_form(ctx, gr.nthr, [&](auto G) {
+          rc = wlaunch(ctx, G, k_otf_links<G.value>,
+                       wide ? OTF_LINK_SLOTS_WIDE : OTF_LINK_SLOTS, gr.nthr,
+                       "on-the-fly sweep, links", a, gr, p, r, (const double2 *)ctx->F, wide);
+        });
+      }
+    return rc;
+  }
   with_grid_form(ctx, gr.nthr, [&](auto G) {
     for (long p = 0; p < steps && !rc; p++)
       rc = ctx->c1 != 0.0 ? wlaunch(ctx, G, k_sweep_imp_otf<G.value>, IMP_SLOTS, gr.nthr,

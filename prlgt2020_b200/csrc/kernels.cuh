@@ -562,6 +562,103 @@ __global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_otf(Swee
   }
 }
 
+// The on-the-fly update of a periodic field in two launches per site of the walk.
+// What a site's four links need of other sites' links does not change while they
+// are updated one after the other: the 12 lower staples (two products each) and
+// the 6 corners U_mu(x+nu)^dag after U_nu(x+mu), each of which serves the upper
+// staples of both its links.  k_otf_parts forms them, all independent (unit
+// t * nthr + thread: the groups of a warp mostly do the same part), and
+// k_otf_links is left with 5 products and an exponential per link in a row
+// instead of 13.  12^4 N=8 (16 steps of 1296 threads): a step took 190 us in one
+// launch and takes 45 and 90; bound by the latency of the links' chains, 9 warps
+// on an SM (otf_in_parts has the other sizes).
+constexpr int OTF_PARTS = 18, OTF_LINK_SLOTS = 3, OTF_LINK_SLOTS_WIDE = 8;
+
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_otf_parts(SweepArgs a, LgfGrid gr, long step, long r, double2 *parts, int gpc) {
+  const Grp<G> w(3, a.SS, gpc, (long)OTF_PARTS * gr.nthr);
+  if (!w.ok) return;
+  const int T = w.slot, Y = T + a.SS, Z = Y + a.SS, N = a.N;
+  const int t = (int)(w.id / gr.nthr), thr = (int)(w.id - (long)t * gr.nthr);
+  int x[4], mu, nu;
+  LgfWalk(gr, thr, step).site(gr, a.g, r, x);
+  const bool corner = t >= 12;
+  if (corner) {
+    plane_dirs(t - 12, mu, nu);
+  } else {
+    mu = t / 3;
+    nu = t - 3 * mu;
+    nu += nu >= mu ? 1 : 0;
+  }
+  const Nb l0 = corner ? neighbour(a.g, x, mu, 1) : neighbour(a.g, x, nu, -1, mu, 1);
+  const Nb l1 = neighbour(a.g, x, nu, corner ? 1 : -1);
+  stage_link<G>(T, a.U, nu, l0, N);
+  stage_link<G>(Y, a.U, mu, l1, N);
+  if (!corner) stage_link<G>(Z, a.U, nu, l1, N);
+  wstage_wait<G>();
+  ser_mul<G>(T, T, Y, N, corner ? MUL_DB : MUL_DA | MUL_DB);
+  if (!corner) ser_mul<G>(T, T, Z, N, MUL_DAG);
+  wstore<G>(parts + (size_t)w.id * link_rec(N), T, (int)link_rec(N));
+}
+
+template <int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>())
+    k_otf_links(SweepArgs a, LgfGrid gr, long step, long r, const double2 *parts, bool wide, int gpc) {
+  const Grp<G> w(wide ? OTF_LINK_SLOTS_WIDE : OTF_LINK_SLOTS, a.SS, gpc, gr.nthr);
+  if (!w.ok) return;
+  double2 *sm = wsm();
+  const int N = a.N, n = (int)link_rec(N), lane = glane<G>();
+  // sum, corners, the site's links: wide, a slot for each of the three and of the four
+  const int step_slot = wide ? a.SS : 0;
+  const int W = w.slot, T = W + a.SS, S = T + a.SS + 2 * step_slot;
+  const size_t part = (size_t)gr.nthr * n;
+  parts += (size_t)w.id * n;
+  int x[4];
+  LgfWalk(gr, w.id, step).site(gr, a.g, r, x);
+  const int site = x[0] * a.g.s0 + x[1] * a.g.s1 + x[2] * a.g.s2 + x[3];
+#pragma unroll 1
+  for (int mu = 0; mu < 4; mu++) {
+    auto stage = [&](int q) {
+      const int nu = q + (q >= mu ? 1 : 0);
+      wstage<G>(T + q * step_slot, parts + (12 + plane_of(min(mu, nu), max(mu, nu))) * part, n);
+      wstage<G>(S + nu * step_slot, a.U + link_at(nu, site, N), n);
+    };
+    const int Y = S + mu * step_slot;
+    if (wide) {
+      for (int q = 0; q < 3; q++) stage(q);
+      wstage<G>(Y, a.U + link_at(mu, site, N), n);
+    } else {
+      stage(0);
+    }
+    const double2 *low = parts + 3 * mu * part;
+    for (int e = lane; e < n; e += glanes<G>())
+      sm[W + e] = cadd(cadd(low[e], low[part + e]), low[2 * part + e]);
+    wstage_wait<G>();
+#pragma unroll 1
+    for (int q = 0; q < 3; q++) {
+      const int nu = q + (q >= mu ? 1 : 0);
+      ser_mul<G>(W, T + q * step_slot, S + nu * step_slot, N,
+                 (mu < nu ? MUL_DB : MUL_DA | MUL_DB) | MUL_ACC);
+      if (!wide) {
+        if (q < 2)
+          stage(q + 1);
+        else
+          wstage<G>(Y, a.U + link_at(mu, site, N), n);
+        wstage_wait<G>();
+      }
+    }
+    link_obs<G>(a, Y, (size_t)site * 4 + mu);
+    ser_mul<G>(W, Y, W, N, MUL_DAG);
+    link_trace<G>(a.obs_tr + ((size_t)site * 4 + mu) * 2 * (N + 1), W, N);
+    gsync<G>();
+    update_link<G, true>(a, T, Y, W, mu, site);
+    // the next link's copies read what this one wrote
+    __threadfence();
+    gsync<G>();
+  }
+}
+
 // ---------------- improved gauge actions ----------------
 
 // Sweep with an improved gauge action (TLSYM, IWA, DBW2; periodic boundaries):

@@ -113,6 +113,30 @@ def test_local_gf_teams(engine_mod, oracle_mod, zero_modes, N):
         assert per_order_rel(e.download(), o.links, N).max() <= 1e-12, form
 
 
+@pytest.mark.parametrize("N", [3, 9, 15], ids=["one_launch", "parts_nine_lanes", "parts_warp"])
+def test_onthefly_many_threads(engine_mod, oracle_mod, N):
+    """The on-the-fly sweep with 4096 reference threads: a 4^4 field and noise,
+    repeated over 16^4, stay repeated (blocks of 2 sites a side divide both)."""
+    P, O = engine_mod, oracle_mod
+    o = O.Oracle((4, 4, 4, 4), N)
+    o.random_start(13, 0.5)
+    nz = O.Rand55(17).gauss(o.V * 32)
+
+    def tiled(v):
+        v = np.asarray(v).reshape(4, 4, 4, 4, -1)
+        return np.ascontiguousarray(np.tile(v, (4, 4, 4, 4, 1)))
+
+    shape = (-1,) + o.links.shape[1:]
+    with P.NsptEngine((16, 16, 16, 16), N, update="onthefly") as e:
+        e.set_gf_grid((8, 8, 8, 8))
+        e.upload(tiled(o.links).reshape(shape))
+        e.set_noise(tiled(nz).ravel())
+        e.gauge_wilson(0.01)
+        got = e.download()
+    o.sweep(0.01, nz, onthefly=True, grid=(2, 2, 2, 2))
+    assert per_order_rel(got, tiled(o.links).reshape(shape), N).max() <= 1e-12
+
+
 def test_large_fields_cross_the_bus_whole(engine_mod):
     """Upload and download of a field that goes through the pinned buffers
     (28.7 MB: 14 chunks and a part of one), and of part of its orders."""
