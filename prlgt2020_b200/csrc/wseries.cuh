@@ -205,8 +205,8 @@ __device__ __forceinline__ void ordered_block(typename Acc::T (&acc)[BLK], const
   for (int t = 0; t < BLK - 1; t++)
 #pragma unroll
     for (int l = 0; l < 3; l++) {
-      T a = Acc::zero();
-      if (kb + t >= 0) a = Acc::in(wconj(left[9 * (kb + 1 + t) + la * l], sa), aux, kb + 1 + t);
+      if (kb + t < 0) continue;
+      const T a = Acc::in(wconj(left[9 * (kb + 1 + t) + la * l], sa), aux, kb + 1 + t);
 #pragma unroll
       for (int q = t + 1; q < BLK; q++) Acc::mac(acc[q], a, w[l][q - t]);
     }
