@@ -120,7 +120,7 @@ def dist_setup():
 
 
 def read_profile_value(key: str, path: str = "profiles/sweep_32x4_n24_traffic.txt"):
-    """A per-launch figure of the sweep kernel from a committed ncu summary
+    """A per-sweep figure of the sweep's kernels from a committed ncu summary
     (`key: value` lines)."""
     try:
         for line in open(os.path.join(ROOT, path)):
@@ -132,26 +132,33 @@ def read_profile_value(key: str, path: str = "profiles/sweep_32x4_n24_traffic.tx
 
 
 def read_profile_traffic():
-    """DRAM bytes (read + write) of one 32^4 x 24 sweep-kernel launch, from
-    the committed ncu summary (a 16^4 capture scaled by the link count)."""
-    return read_profile_value("traffic_bytes_per_launch")
+    """DRAM bytes (read + write) of one 32^4 x 24 sweep, from the committed ncu
+    summary (a 16*16*16*8 capture scaled by the link count)."""
+    return read_profile_value("traffic_bytes_per_sweep")
+
+
+def sweep_launches(L):
+    """Kernel launches of one Jacobi Wilson sweep: k_plaq and k_update per slab
+    of direction 0 (at least 4096 sites), the last plane's plaquettes ahead when
+    there are several, four k_colsum, k_inc (the Philox step counter)."""
+    plane = L[1] * L[2] * L[3]
+    slab = min(L[0], -(-4096 // plane))
+    return 2 * -(-L[0] // slab) + (slab < L[0]) + 5
 
 
 def executed_fraction(N: int, V: int, kernel_ms: float, peak: float):
-    """The FP64 rate the sweep kernel executes (not the canonical count):
-    DFMA thread instructions per link from the committed ncu summary of the
-    benchmark kernel (profiles/k_sweep_16x16x16x8_n24_full.md, key
-    dfma_thread_inst_per_link) x 2 flops x the 4V links of this sweep, over
+    """The FP64 rate the sweep's kernels execute (not the canonical count):
+    DFMA thread instructions per link from the committed ncu summary
+    (profiles/sweep_32x4_n24_traffic.txt, key dfma_thread_inst_per_link) x 2 flops x the 4V links of this sweep, over
     the kernel time measured here.  Only for the 24-order benchmark shape."""
-    per_link = read_profile_value("dfma_thread_inst_per_link",
-                                  "profiles/k_sweep_16x16x16x8_n24_full.md")
+    per_link = read_profile_value("dfma_thread_inst_per_link")
     if per_link is None or N != 24:
         return None
     tflops = per_link * 2.0 * 4 * V / (kernel_ms * 1e-3) / 1e12
     return {"achieved": tflops, "frac": tflops / peak, "unit": "TFLOP/s",
             "source": "DFMA thread instructions per link: ncu smsp__sass_thread_inst_executed_"
-                      "op_dfma_pred_on.sum of one launch at 16x16x16x8 x 24 orders "
-                      "(profiles/k_sweep_16x16x16x8_n24_full.md)"}
+                      "op_dfma_pred_on.sum of one sweep at 16x16x16x8 x 24 orders "
+                      "(profiles/sweep_32x4_n24_traffic.txt)"}
 
 
 def host_cpu() -> dict:
@@ -390,9 +397,9 @@ def run_ours(args, world, rank, local):
             "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak, "traffic": read_profile_traffic(),
                          "traffic_source": "profiles/sweep_32x4_n24_traffic.txt: ncu dram__bytes_read.sum "
-                                           "+ dram__bytes_write.sum of one k_sweep launch at 16^4 x 24, "
-                                           "scaled x16 (links) to 32^4; not measured in this run",
-                         "kernel": "k_sweep", "kernel_ms": kernel_ms,
+                                           "+ dram__bytes_write.sum of one sweep at 16*16*16*8 x 24, "
+                                           "scaled x32 (links) to 32^4; not measured in this run",
+                         "kernel": "k_plaq + k_update", "kernel_ms": kernel_ms,
                          "peak_source": "FP64 FMA microbenchmark on this GPU "
                                         "(nspt_measure_fp64_peak); MEASURED_PEAKS.json has no FP64 entry",
                          "flops_per_sweep": flops,
@@ -402,9 +409,8 @@ def run_ours(args, world, rank, local):
             "clocks": clocks,
             "e2e": e2e,
             "with_gf": with_gf,
-            # per sweep: k_sweep, three k_rowsum reductions, k_inc (the
-            # Philox step counter) -- the launch list in profiles/
-            "gpu_launches": 5 * args.steps,
+            "gpu_launches": sweep_launches(L) * args.steps if args.update == "jacobi" else
+                            (16 + 5) * args.steps,  # a k_sweep_otf per barrier step
             "cpu_baseline": cpu,
         }
         print(json.dumps(line), flush=True)

@@ -218,7 +218,7 @@ extern "C" int nspt_batch_observables(nspt_batch *b, double *plaq) {
   return NSPT_OK;
 }
 
-// Autotuner over the tile shape of the series kernels: orders a lane
+// Autotuner over the launch shape of the series kernels: orders a lane
 // accumulates per pass (MO: the block chosen by N, or MO_LOW where N <= 3
 // MO_LOW) and warps per CTA (one link per warp).  Every candidate is
 // captured and timed on the batch itself; the fastest is kept.  The trial

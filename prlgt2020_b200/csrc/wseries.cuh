@@ -278,8 +278,8 @@ __device__ __noinline__ void ser_mul_any(int out, int A, int Bs, int N, unsigned
           };
 #pragma unroll 1
           // by twos: a longer body has fewer moves of the window, but the SM's
-          // instruction cache pays for it.  12^4 N=12 sweep 2.05 ms by twos, 2.25 by
-          // fours, 2.40 with eights, 2.06 by ones; 16*16*16*8 N=24 8.2, 8.6, 9.1, 8.6
+          // instruction cache pays for it.  12^4 N=12 sweep 2.09 ms by twos, 2.25 by
+          // fours, 2.09 by ones; 16*16*16*8 N=24 8.39, 8.45 and 8.69
           if (n & 1) steps(std::integral_constant<int, 1>());
 #pragma unroll 1
           while (n) steps(std::integral_constant<int, 2>());
