@@ -288,6 +288,19 @@ static bool otf_in_parts(const nspt_ctx *ctx, const LgfGrid &gr) {
          (gr.nthr < 24L * ctx->nsm || ctx->N > BLK) && (long)OTF_PARTS * gr.nthr <= 4L * ctx->V;
 }
 
+// The order in which an ORDERED on-the-fly sweep adds up a link's six staples:
+// plane by plane where a barrier step has one site per thread and few threads,
+// else one by one.  The engine's first kernels gave such a step a group of lanes
+// per plane, on grids that filled 8 warps an SM at most (11 at 16 orders, of 3 x 3
+// slots each, would fit), unless told to take a group per thread; a run with
+// logarithms at high order keeps what it was begun with (ordered).
+static bool otf_by_planes(const nspt_ctx *ctx, const LgfGrid &gr) {
+  if (!ordered(ctx) || gr.seg != 1 || ctx->gf_form == NSPT_LGF_GROUP) return false;
+  if (ctx->gf_form == NSPT_LGF_TEAM) return true;
+  const long slot = ((long)link_rec(ctx->N) + 4) / 8 * 8 + 3;  // 3 (mod 8)
+  return gr.nthr <= std::min<long>(228 * 1024 / (9 * slot * (long)sizeof(double2)), 8) * ctx->nsm;
+}
+
 // gauge_wilson on the fly (UPDATE_ONTHEFLY, nspt.cc:355-460): one launch per
 // barrier step of the thread grid, or two per site of its walk; one group per
 // reference thread.
@@ -315,12 +328,13 @@ static int launch_sweep_otf(nspt_ctx *ctx, const SweepArgs &a) {
       }
     return rc;
   }
+  const bool planes = otf_by_planes(ctx, gr);
   with_grid_form(ctx, gr.nthr, [&](auto G) {
     for (long p = 0; p < steps && !rc; p++)
       rc = ctx->c1 != 0.0 ? wlaunch(ctx, G, k_sweep_imp_otf<G.value>, IMP_SLOTS, gr.nthr,
                                     "on-the-fly sweep", a, gr, p)
-                          : wlaunch(ctx, G, k_sweep_otf<G.value>, LINK_SLOTS, gr.nthr,
-                                    "on-the-fly sweep", a, gr, p);
+                          : wlaunch(ctx, G, k_sweep_otf<G.value>, LINK_SLOTS + (planes ? 1 : 0), gr.nthr,
+                                    "on-the-fly sweep", a, gr, p, planes);
   });
   return rc;
 }

@@ -496,10 +496,14 @@ __device__ __forceinline__ void chain_stage(const SweepArgs &a, int slot, int d,
 //   lower U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_nu(x-nu)    (QCDenvNODEpt_test.h:556)
 // For the on-the-fly update, whose links must be visited in order, and for
 // fields with flags other than 1 across twisted faces.
+//
+// The six are added up one by one in W; with a slot Z (ORDERED, see
+// otf_by_planes) a plane's two first, then the planes: (p0 + p1) + p2.
 template <bool FF, int G>
 __device__ __forceinline__ void link_one(const SweepArgs &a, int T, int Y, int W, int mu,
-                                         int site) {
+                                         int site, int Z = -1) {
   const int N = a.N, ffe = FF ? *a.ff_scale : 0;
+  const bool planes = G == ORDERED && Z >= 0;
   int x[4];
   coords(a.g, site, x);
   const Nb self = nb_self(site);
@@ -519,7 +523,14 @@ __device__ __forceinline__ void link_one(const SweepArgs &a, int T, int Y, int W
     chain_stage<G>(a, Y, nu, l2);
     wstage_wait<G>();
     twist_link<G>(Y, l2, a.g, N);
-    ser_mul_x<FF, G>(W, T, Y, N, ffe, (up ? MUL_DB : MUL_DAG) | (h ? MUL_ACC : 0));
+    ser_mul_x<FF, G>(planes && q ? Z : W, T, Y, N, ffe,
+                     (up ? MUL_DB : MUL_DAG) | ((planes ? !up : h > 0) ? MUL_ACC : 0));
+    if (planes && q && !up) {
+      double2 *sm = wsm();
+      for (int e = glane<G>(); e < (int)link_rec(N); e += glanes<G>())
+        sm[W + e] = cadd(sm[W + e], sm[Z + e]);
+      gsync<G>();
+    }
   }
   chain_stage<G>(a, Y, mu, self);
   wstage_wait<G>();
@@ -546,8 +557,8 @@ __global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_link(Swe
 // in place, mu = 0..3, each seeing the links updated before it; the threads of
 // one barrier step touch disjoint links.
 template <int G>
-__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_otf(SweepArgs a, LgfGrid gr, long step, int gpc) {
-  const Grp<G> w(LINK_SLOTS, a.SS, gpc, gr.nthr);
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_otf(SweepArgs a, LgfGrid gr, long step, bool planes, int gpc) {
+  const Grp<G> w(LINK_SLOTS + (planes ? 1 : 0), a.SS, gpc, gr.nthr);
   if (!w.ok) return;
   const LgfWalk walk(gr, w.id, step);
 #pragma unroll 1
@@ -555,7 +566,8 @@ __global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_sweep_otf(Swee
     int x[4];
     walk.site(gr, a.g, r >> 2, x);
     const int site = x[0] * a.g.s0 + x[1] * a.g.s1 + x[2] * a.g.s2 + x[3];
-    link_one<false, G>(a, w.slot, w.slot + a.SS, w.slot + 2 * a.SS, (int)(r & 3), site);
+    link_one<false, G>(a, w.slot, w.slot + a.SS, w.slot + 2 * a.SS, (int)(r & 3), site,
+                       planes ? w.slot + 3 * a.SS : -1);
     // the next link's copies read what this one wrote
     __threadfence();
     gsync<G>();

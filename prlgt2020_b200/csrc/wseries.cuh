@@ -27,7 +27,7 @@
 //           term by term in the order i, l (three windows, 240 registers).  The
 //           sums are then bit for bit those of a plain loop over i of 3x3
 //           products, which every field of a run with logarithms at high order
-//           has been made with: there rounding is amplified by some 4 per order
+//           has been made with: there rounding is amplified by some 3 per order
 //           (order 20 of a field of size 1: 1e-16 becomes 3e-7), so that a
 //           different order of summation is another field.
 //
