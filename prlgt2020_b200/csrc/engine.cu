@@ -281,7 +281,16 @@ static LgfGrid thread_grid(const nspt_ctx *ctx, long &steps) {
 // threads) N=6 4.5 and 5.1 ms, N=9 7.1 and 6.5, 24^4 (20736) N=8 19.6 and 20.5,
 // N=10 32.4 and 31.6; 12^4 (1296) N=8 3.03 and 2.16, 16*14^3 (2744) N=4 5.4 and
 // 3.4, 8^4 (256) N=11 3.9 and 2.1.
+// Two launches per site of the walk are also bounded: a call returns at its time
+// limit (nspt_set_timeout) only if its launches fit the stream's queue, some 1000,
+// and a graph of the step holds a node for each.  So a walk of several sites is
+// taken in parts up to OTF_WALK sites in a sweep, although a longer one is twice
+// as fast that way (5^4 N=8, one thread: 88 ms in one launch, 50 in 1250; 9^4 925
+// and 524, but with a limit of 20 ms the call came back after 503); steps of one
+// site each took four launches in the engine's first kernels and take two.
+constexpr long OTF_WALK = 256;
 static bool otf_in_parts(const nspt_ctx *ctx, const LgfGrid &gr) {
+  if (gr.seg > 1 && ctx->V > OTF_WALK * gr.nthr) return false;
   for (int d = 0; d < 4; d++)
     if (ctx->L[d] < 2) return false;
   return ctx->c1 == 0.0 && !ctx->geo.twist && !ordered(ctx) &&
