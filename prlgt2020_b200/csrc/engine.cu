@@ -389,7 +389,11 @@ static int launch_sweep(nspt_ctx *ctx, const SweepArgs &a) {
     constexpr int g = G.value;
     if constexpr (g != ORDERED) {
       if (ctx->tr_rows == 6) {
-        rc = ff ? launch_sweep_plaq<true, g>(ctx, a) : launch_sweep_plaq<false, g>(ctx, a);
+        if (ctx->plaq[0])
+          rc = ff ? launch_sweep_plaq<true, g>(ctx, a) : launch_sweep_plaq<false, g>(ctx, a);
+        else
+          rc = ff ? wlaunch(ctx, G, k_update_alone<true, g>, ALONE_SLOTS, nl, "sweep", a)
+                  : wlaunch(ctx, G, k_update_alone<false, g>, ALONE_SLOTS, nl, "sweep", a);
         return;
       }
     }
@@ -400,6 +404,15 @@ static int launch_sweep(nspt_ctx *ctx, const SweepArgs &a) {
               : wlaunch(ctx, G, k_sweep_link<false, g>, LINK_SLOTS, nl, "sweep", a);
   });
   return rc;
+}
+
+// Whether the sweep goes plaquette by plaquette: unless the order of the links is
+// fixed, the action has rectangles, the sums have an order to keep, or a flag
+// other than 1 meets a twisted face (where each link's staples see flags of their
+// own).
+static bool by_plaquettes(const nspt_ctx *ctx) {
+  return !(ctx->flags & NSPT_UPDATE_ONTHEFLY) && ctx->c1 == 0.0 && !ordered(ctx) &&
+         (ctx->unit_flags || !ctx->geo.twist);
 }
 
 static int do_sweep(nspt_ctx *ctx, double dt, bool use_noise) {
@@ -428,13 +441,7 @@ static int do_sweep(nspt_ctx *ctx, double dt, bool use_noise) {
   a.g = ctx->geo;
   a.Ut = ctx->U;
   const bool otf = (ctx->flags & NSPT_UPDATE_ONTHEFLY) != 0;
-  // plaquette by plaquette unless the order of the links is fixed, the action
-  // has rectangles, the sums have an order to keep, the records found no
-  // memory, or a flag other than 1 meets
-  // a twisted face (where each link's staples see flags of their own)
-  ctx->tr_rows = !otf && ctx->c1 == 0.0 && ctx->plaq[0] && !ordered(ctx) &&
-                         (ctx->unit_flags || !ctx->geo.twist)
-                     ? 6 : 4;
+  ctx->tr_rows = by_plaquettes(ctx) ? 6 : 4;
   if (otf) {
     // in place; with twisted boundaries F keeps the step's start field for
     // the reads across a twisted face (the reference's copy sites)
@@ -902,8 +909,8 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
          alloc((void **)&ctx->Gx, links / 4) && alloc((void **)&ctx->ftw, 4 * 128 * sizeof(double2));
   if (ok && !(flags & NSPT_UPDATE_ONTHEFLY) && ctx->c1 == 0.0 && !ordered(ctx)) {
     // Plaquette records of two slabs of at least SLAB_SITES sites, or of the
-    // whole lattice where that is no more.  Without the memory for them the
-    // sweep goes link by link.
+    // whole lattice where that is no more.  Without the memory for them each
+    // link forms its own (k_update_alone).
     const long plane = V / L[0];
     ctx->slab = (int)std::min<long>(L[0], (SLAB_SITES + plane - 1) / plane);
     if (2 * ctx->slab >= L[0]) ctx->slab = L[0];

@@ -431,6 +431,91 @@ __global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_update(SweepAr
   update_link<G, false>(a, T, Y, W, mu, site);
 }
 
+// The same sweep without the records, for contexts that found no memory for
+// them: a link forms its six plaquettes itself, with the products of k_plaq and
+// the sums of k_update in their order, so that the field has the same bits
+// whichever way a sweep went.  16 products per link instead of 8.5.
+constexpr int ALONE_SLOTS = 4;
+
+// Record q of plaquette (x, mu < nu) in S1 (q = 0, 1) or S2 (q = 2): see plaq_at
+template <bool FF, int G>
+__device__ __forceinline__ int plaq_part(const SweepArgs &a, int S0, int S1, int S2, int q, int mu,
+                                         int nu, int site, int ffe) {
+  const int N = a.N;
+  int x[4];
+  coords(a.g, site, x);
+  const Nb self = nb_self(site), um = neighbour(a.g, x, mu, 1), un = neighbour(a.g, x, nu, 1);
+  stage_link<G>(S2, a.U, nu, self, N);
+  if (q != 2) {
+    stage_link<G>(S0, a.U, mu, self, N);
+    stage_link<G>(S1, a.U, nu, um, N);
+    wstage_wait<G>();
+    twist_link<G>(S1, um, a.g, N);
+    ser_mul_x<FF, G>(S1, S0, S1, N, ffe, MUL_DAG);  // A
+  }
+  if (q == 1) {
+    ser_mul_x<FF, G>(S1, S1, S2, N, ffe, MUL_DA);
+    return S1;
+  }
+  stage_link<G>(S0, a.U, mu, un, N);
+  wstage_wait<G>();
+  twist_link<G>(S0, un, a.g, N);
+  ser_mul_x<FF, G>(S2, S2, S0, N, ffe, MUL_DAG);  // B
+  if (q == 0) {
+    ser_mul_x<FF, G>(S1, S1, S2, N, ffe, MUL_DB);
+    return S1;
+  }
+  stage_link<G>(S0, a.U, mu, self, N);
+  wstage_wait<G>();
+  ser_mul_x<FF, G>(S2, S2, S0, N, ffe, MUL_DA);
+  return S2;
+}
+
+template <bool FF, int G>
+__global__ void __launch_bounds__(32 * CTA_WARPS, sm_ctas<G>()) k_update_alone(SweepArgs a, int gpc) {
+  const Grp<G> w(ALONE_SLOTS, a.SS, gpc, 4L * a.g.V);
+  if (!w.ok) return;
+  double2 *sm = wsm();
+  const int N = a.N, n = (int)link_rec(N), ffe = FF ? *a.ff_scale : 0;
+  const int S0 = w.slot, S1 = S0 + a.SS, S2 = S1 + a.SS, W = S2 + a.SS;
+  const int site = (int)(w.id >> 2), mu = (int)(w.id & 3);
+  int x[4];
+  coords(a.g, site, x);
+  // t < 3: the lower staples into W; t >= 3: U_mu(x) W, then the plaquettes at x
+#pragma unroll 1
+  for (int t = 0; t < 6; t++) {
+    const int h = t % 3, nu = h + (h >= mu ? 1 : 0);
+    if (t == 3) {
+      stage_link<G>(S0, a.U, mu, nb_self(site), N);
+      wstage_wait<G>();
+      link_obs<G>(a, S0, (size_t)site * 4 + mu);
+      ser_mul_x<FF, G>(W, S0, W, N, ffe, 0);
+    }
+    const bool first = mu < nu;
+    const Nb d = neighbour(a.g, x, nu, -1);
+    const int S = plaq_part<FF, G>(a, S0, S1, S2, t >= 3 ? 0 : first ? 1 : 2, first ? mu : nu,
+                                   first ? nu : mu, t >= 3 ? site : d.site, ffe);
+    if (t < 3) {
+      if (d.bwd & a.g.twist) wtwist<G>(S, 1u << nu, 0u, N);
+      for (int e = w.lane; e < n; e += glanes<G>()) sm[W + e] = h ? cadd(sm[W + e], sm[S + e]) : sm[S + e];
+    } else {
+      for (int e = 1 + w.lane; e < n; e += glanes<G>()) {
+        const int k9 = (e - 1) / 9 * 9, m = e - 1 - k9, et = 1 + k9 + 3 * (m % 3) + m / 3;
+        sm[W + e] = cadd(sm[W + e], first ? sm[S + e] : cconj(sm[S + et]));
+      }
+      if (first) {
+        double *o = a.obs_tr + ((size_t)site * 6 + plane_of(mu, nu)) * (N + 1);
+        for (int k = w.lane; k <= N; k += glanes<G>()) {
+          const double2 *p = sm + S + 9 * k - 8;
+          o[k] = k ? p[0].x + p[4].x + p[8].x : 3. * sm[S].x;
+        }
+      }
+    }
+    gsync<G>();
+  }
+  update_link<G, false>(a, S0, S1, W, mu, site);
+}
+
 // ---------------- sweeps link by link ----------------
 
 // Thread grid of the reference's OpenMP build (choices.h:124-128): n[d]
