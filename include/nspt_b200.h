@@ -86,7 +86,10 @@ int nspt_destroy(nspt_ctx *ctx);
 const char *nspt_error_string(int code);
 const char *nspt_last_error(nspt_ctx *ctx);
 
-/* Device and memory footprint of a context (bytes). */
+/* Device memory of a context (bytes).  With a Jacobi update of the Wilson action
+ * it includes the records of plaquettes, which take half of the free memory at
+ * most; they go back when a context of the process finds no memory
+ * otherwise.  Without them a sweep takes longer and gives the same bits. */
 size_t nspt_device_bytes(const nspt_ctx *ctx);
 
 /* Replace ptGluon_fld::load / save (QCDenvNODEpt_test.h:342-374):

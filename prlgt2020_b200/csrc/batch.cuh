@@ -186,6 +186,12 @@ extern "C" int nspt_batch_step(nspt_batch *b, int nsteps, int gf_every) {
   if (!b || nsteps < 0 || gf_every < 0) return NSPT_ERR_ARG;
   const int P = graph_length(gf_every);
   if (nsteps % P) return NSPT_ERR_ARG;
+  // until the graph has run, no replica's records are taken back
+  std::vector<std::unique_lock<std::recursive_mutex>> in_use;
+  for (nspt_ctx *c : b->ctx) {
+    in_use.emplace_back(c->use);
+    take_records(c);
+  }
   for (nspt_ctx *c : b->ctx) {
     if (c->noise_pending) return NSPT_ERR_STATE;  // injected noise is for single steps
     if (cudaStreamSynchronize(c->st) != cudaSuccess) return NSPT_ERR_CUDA;

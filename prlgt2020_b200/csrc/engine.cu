@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -47,8 +48,12 @@ struct nspt_ctx {
   int SS;  // slot stride (double2)
   double2 *U, *F;    // link records (kernels.cuh)
   bool unit_flags;   // every link's flag is 1 (false after an upload that says otherwise)
-  double2 *plaq[2];  // plaquette records of two slabs of the Jacobi sweep
+  double2 *plaq[2];  // plaquette records of two slabs of the Jacobi sweep, or none
+  size_t plaq_bytes;
   int slab;          // planes of direction 0 per slab
+  // held by every call that launches sweeps or a graph of them: another context's
+  // creation may take the records back in between (release_records)
+  std::recursive_mutex use;
   double2 *Lg;       // per-link logs (zero modes, FA)
   bool snap_valid;   // on the fly, twisted: F holds the step's start field, which reads
                      // across a twisted face see until twist_boundary
@@ -85,8 +90,8 @@ struct nspt_ctx {
   // its kernels take by argument (seed, gauge-fixing grid, sweep shape,
   // float-float scale mode); a CUDA graph captured under another value is
   // stale (batch.cuh)
-  uint64_t launch_gen;
-  size_t bytes;
+  std::atomic<uint64_t> launch_gen;
+  std::atomic<size_t> bytes;
   std::string err;
 };
 
@@ -117,6 +122,51 @@ extern "C" const char *nspt_last_error(nspt_ctx *ctx) {
       return NSPT_ERR_CUDA;                                                   \
     }                                                                         \
   } while (0)
+
+// ---------------- memory ----------------
+
+// Every context of the process, so that one that cannot have the memory it needs
+// is given the plaquette records of the others, which they can do without.
+static struct Contexts {
+  std::mutex mu;
+  std::vector<nspt_ctx *> all;
+} g_ctx;
+
+static void free_records(nspt_ctx *ctx) {
+  for (double2 *&p : ctx->plaq) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  }
+  ctx->bytes -= ctx->plaq_bytes;
+  ctx->plaq_bytes = 0;
+}
+
+// The records of all contexts on a device that are in no call back to the driver.
+// Their next sweeps form each link's plaquettes anew or find memory again; a graph
+// that held the records is captured again (launch_gen).
+static bool release_records(int dev) {
+  bool any = false;
+  std::lock_guard<std::mutex> lock(g_ctx.mu);
+  for (nspt_ctx *c : g_ctx.all) {
+    std::unique_lock<std::recursive_mutex> use(c->use, std::try_to_lock);
+    if (!use || c->dev != dev || !c->plaq_bytes) continue;
+    cudaStreamSynchronize(c->st);  // what a call past its time limit left
+    free_records(c);
+    c->launch_gen++;
+    any = true;
+  }
+  return any;
+}
+
+// Device memory that a context cannot do without
+static cudaError_t dev_alloc(void **p, size_t n, int dev) {
+  cudaError_t e = cudaMalloc(p, n);
+  if (e == cudaErrorMemoryAllocation && release_records(dev)) {
+    cudaGetLastError();
+    e = cudaMalloc(p, n);
+  }
+  return e;
+}
 
 // ---------------- kernel shapes ----------------
 
@@ -413,6 +463,39 @@ static int launch_sweep(nspt_ctx *ctx, const SweepArgs &a) {
 static bool by_plaquettes(const nspt_ctx *ctx) {
   return !(ctx->flags & NSPT_UPDATE_ONTHEFLY) && ctx->c1 == 0.0 && !ordered(ctx) &&
          (ctx->unit_flags || !ctx->geo.twist);
+}
+
+// Plaquette records: of the whole lattice where that is two slabs of SLAB_SITES
+// sites or fewer, else of two such slabs, and of smaller ones where they would
+// leave less than half of the free memory to others.  Taken at the end of a
+// context's creation (0.5 to 0.9 ms, as much as a first sweep of a small lattice)
+// and, where they are not held, before a call's sweeps.  Without them each link
+// forms its own plaquettes (k_update_alone): 8^4 N=24 2.40 ms instead of 1.05, 12^4
+// N=8 2.19 and 1.02, in float-float 9.5 and 3.4.
+static void take_records(nspt_ctx *ctx) {
+  if (ctx->plaq_bytes || !by_plaquettes(ctx)) return;
+  size_t room = 0, total = 0;
+  if (cudaMemGetInfo(&room, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  const int L0 = ctx->L[0];
+  const long plane = ctx->V / L0;
+  const size_t rec = (size_t)plane * 18 * link_rec(ctx->N) * sizeof(double2);
+  int slab = (int)std::min<long>(L0, (SLAB_SITES + plane - 1) / plane);
+  if (2 * slab >= L0) slab = L0;
+  auto bytes = [&] { return rec * (slab < L0 ? 2 * slab : L0); };
+  while (slab > 1 && bytes() > room / 2) slab = std::min((slab + 1) / 2, L0 / 2);
+  if (bytes() > room / 2 || cudaMalloc(&ctx->plaq[0], rec * slab) != cudaSuccess ||
+      (slab < L0 && cudaMalloc(&ctx->plaq[1], rec * slab) != cudaSuccess)) {
+    cudaGetLastError();
+    free_records(ctx);
+    return;
+  }
+  ctx->slab = slab;
+  ctx->plaq_bytes = bytes();
+  ctx->bytes += ctx->plaq_bytes;
+  ctx->launch_gen++;
 }
 
 static int do_sweep(nspt_ctx *ctx, double dt, bool use_noise) {
@@ -809,6 +892,7 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
   ctx->V = V;
   ctx->U = ctx->F = ctx->Lg = ctx->Wg = ctx->Gx = nullptr;
   ctx->plaq[0] = ctx->plaq[1] = ctx->meas = nullptr;
+  ctx->plaq_bytes = 0;
   ctx->slab = L[0];
   ctx->unit_flags = true;
   ctx->tr_rows = 4;
@@ -886,7 +970,7 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
   const size_t nl = (size_t)4 * V;
   const size_t width = std::max<size_t>({12 * (size_t)N, 8 * (size_t)(N + 1), 8 * link_rec(N)});
   auto alloc = [&](void **p, size_t n) {
-    if (cudaMalloc(p, n) != cudaSuccess) return false;
+    if (dev_alloc(p, n, ctx->dev) != cudaSuccess) return false;
     ctx->bytes += n;
     return true;
   };
@@ -907,23 +991,6 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
   if (ok && (flags & NSPT_GF_FA))
     ok = alloc((void **)&ctx->Wg, (size_t)9 * N * V * sizeof(double2)) &&
          alloc((void **)&ctx->Gx, links / 4) && alloc((void **)&ctx->ftw, 4 * 128 * sizeof(double2));
-  if (ok && !(flags & NSPT_UPDATE_ONTHEFLY) && ctx->c1 == 0.0 && !ordered(ctx)) {
-    // Plaquette records of two slabs of at least SLAB_SITES sites, or of the
-    // whole lattice where that is no more.  Without the memory for them each
-    // link forms its own (k_update_alone).
-    const long plane = V / L[0];
-    ctx->slab = (int)std::min<long>(L[0], (SLAB_SITES + plane - 1) / plane);
-    if (2 * ctx->slab >= L[0]) ctx->slab = L[0];
-    const size_t n = (size_t)ctx->slab * plane * 18 * link_rec(N) * sizeof(double2);
-    if (cudaMalloc(&ctx->plaq[0], n) != cudaSuccess ||
-        (ctx->slab < L[0] && cudaMalloc(&ctx->plaq[1], n) != cudaSuccess)) {
-      cudaGetLastError();
-      if (ctx->plaq[0]) cudaFree(ctx->plaq[0]);
-      ctx->plaq[0] = ctx->plaq[1] = nullptr;
-    } else {
-      ctx->bytes += ctx->slab < L[0] ? 2 * n : n;
-    }
-  }
   if (!ok) {
     cudaGetLastError();
     cudaStreamDestroy(ctx->st);
@@ -936,12 +1003,24 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
     return fail(NSPT_ERR_CUDA);
   }
   stage_user(1);
+  {
+    std::lock_guard<std::mutex> lock(g_ctx.mu);
+    g_ctx.all.push_back(ctx);
+  }
+  {
+    std::lock_guard<std::recursive_mutex> in_use(ctx->use);
+    take_records(ctx);
+  }
   *out = ctx;
   return nspt_cold_start(ctx);
 }
 
 extern "C" int nspt_destroy(nspt_ctx *ctx) {
   if (!ctx) return NSPT_ERR_ARG;
+  {
+    std::lock_guard<std::mutex> lock(g_ctx.mu);
+    g_ctx.all.erase(std::find(g_ctx.all.begin(), g_ctx.all.end(), ctx));
+  }
   cudaStreamSynchronize(ctx->st);
   free_all(ctx);
   cudaEventDestroy(ctx->ev0);
@@ -953,7 +1032,7 @@ extern "C" int nspt_destroy(nspt_ctx *ctx) {
   return NSPT_OK;
 }
 
-extern "C" size_t nspt_device_bytes(const nspt_ctx *ctx) { return ctx ? ctx->bytes : 0; }
+extern "C" size_t nspt_device_bytes(const nspt_ctx *ctx) { return ctx ? ctx->bytes.load() : 0; }
 
 static void set_unit_flags(nspt_ctx *ctx, bool unit) {
   if (ctx->unit_flags != unit) ctx->launch_gen++;  // the sweep's route may change
@@ -1076,7 +1155,7 @@ extern "C" int nspt_upload_links(nspt_ctx *ctx, const void *aos, int A) {
     return field_copy(ctx, const_cast<void *>(aos), ctx->U, per_site * ctx->V, false);
   const int cs = (int)std::max<size_t>(1, std::min<size_t>(kChunkBytes / per_site, ctx->V));
   double2 *buf = nullptr;
-  CK(cudaMalloc(&buf, per_site * cs));
+  CK(dev_alloc((void **)&buf, per_site * cs, ctx->dev));
   int rc = NSPT_OK;
   for (long s0 = 0; s0 < ctx->V; s0 += cs) {
     const int n = (int)std::min<long>(cs, ctx->V - s0);
@@ -1104,7 +1183,7 @@ extern "C" int nspt_download_links(nspt_ctx *ctx, void *aos, int A) {
     return field_copy(ctx, aos, ctx->U, per_site * ctx->V, true);
   const int cs = (int)std::max<size_t>(1, std::min<size_t>(kChunkBytes / per_site, ctx->V));
   double2 *buf = nullptr;
-  CK(cudaMalloc(&buf, per_site * cs));
+  CK(dev_alloc((void **)&buf, per_site * cs, ctx->dev));
   int rc = NSPT_OK;
   for (long s0 = 0; s0 < ctx->V; s0 += cs) {
     const int n = (int)std::min<long>(cs, ctx->V - s0);
@@ -1128,7 +1207,7 @@ extern "C" int nspt_set_noise(nspt_ctx *ctx, const double *eta) {
   if (!ctx || !eta) return NSPT_ERR_ARG;
   const size_t n = (size_t)ctx->V * 4 * 8 * sizeof(double);
   if (!ctx->noise) {
-    if (cudaMalloc(&ctx->noise, n) != cudaSuccess) {
+    if (dev_alloc((void **)&ctx->noise, n, ctx->dev) != cudaSuccess) {
       cudaGetLastError();
       ctx->noise = nullptr;
       return NSPT_ERR_NOMEM;
@@ -1214,6 +1293,8 @@ static int timed_end(nspt_ctx *ctx) {
 
 extern "C" int nspt_gauge_wilson(nspt_ctx *ctx, double dt) {
   if (!ctx || !(dt >= 0.0)) return NSPT_ERR_ARG;
+  std::lock_guard<std::recursive_mutex> in_use(ctx->use);
+  take_records(ctx);
   int rc = timed_begin(ctx);
   if (rc) return rc;
   const bool use = ctx->noise_pending;
@@ -1253,7 +1334,7 @@ static int loop_sums(nspt_ctx *ctx, std::vector<double2> &h) {
     if (ctx->loop_part) cudaFree(ctx->loop_part);
     ctx->loop_part = nullptr;
     ctx->loop_part_n = 0;
-    if (cudaMalloc(&ctx->loop_part, need * sizeof(double2)) != cudaSuccess) {
+    if (dev_alloc((void **)&ctx->loop_part, need * sizeof(double2), ctx->dev) != cudaSuccess) {
       cudaGetLastError();
       return NSPT_ERR_NOMEM;
     }
@@ -1341,6 +1422,8 @@ extern "C" int nspt_set_local_gf_form(nspt_ctx *ctx, int form) {
 
 extern "C" int nspt_step(nspt_ctx *ctx, double dt, int nsteps, int gf_every) {
   if (!ctx || nsteps < 0 || !(dt >= 0.0) || gf_every < 0) return NSPT_ERR_ARG;
+  std::lock_guard<std::recursive_mutex> in_use(ctx->use);
+  take_records(ctx);
   int rc0 = timed_begin(ctx);
   if (rc0) return rc0;
   for (int s = 0; s < nsteps; s++) {
