@@ -17,7 +17,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <type_traits>
 #include <vector>
 
@@ -25,6 +24,7 @@
 #include "kernels.cuh"
 #include "fft.cuh"
 #include "loops.cuh"
+#include "hostcopy.cuh"
 
 using namespace nspt;
 
@@ -852,7 +852,7 @@ static void free_all(nspt_ctx *ctx) {
     if (p) cudaFree(p);
 }
 
-static void stage_user(int n);
+static HostStage g_stage;
 
 extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, nspt_ctx **out) {
   nspt_ctx *ctx = nullptr;
@@ -1002,7 +1002,7 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
     cudaStreamDestroy(ctx->st);
     return fail(NSPT_ERR_CUDA);
   }
-  stage_user(1);
+  g_stage.user(1);
   {
     std::lock_guard<std::mutex> lock(g_ctx.mu);
     g_ctx.all.push_back(ctx);
@@ -1028,7 +1028,7 @@ extern "C" int nspt_destroy(nspt_ctx *ctx) {
   for (int i = 0; i < 2 * nspt_ctx::KEV; i++) cudaEventDestroy(ctx->kev[i]);
   cudaStreamDestroy(ctx->st);
   delete ctx;
-  stage_user(-1);
+  g_stage.user(-1);
   return NSPT_OK;
 }
 
@@ -1052,90 +1052,9 @@ extern "C" int nspt_cold_start(nspt_ctx *ctx) {
 
 static const size_t kChunkBytes = 64u << 20;
 
-// Copies between a field in pageable host memory and the device.  One thread
-// moves a pageable copy through the driver's staging buffer, and faults the
-// pages of a fresh destination, at about 2.7 GB/s; here COPY_THREADS threads
-// each take a stretch of the field through a pinned buffer of their own.  One set
-// of buffers per process (16 MB), made with the first large copy and released
-// with the last context; a copy that finds them in use, made for another device,
-// or no memory for them goes the driver's way, as small ones and those in pinned
-// memory do.
-constexpr int COPY_THREADS = 8;
-constexpr size_t COPY_CHUNK = 2u << 20, COPY_LEAST = 16u << 20;
-static struct HostStage {
-  std::mutex mu;
-  int users = 0, dev = -1;
-  char *buf = nullptr;
-  cudaStream_t st[COPY_THREADS] = {};
-  void release() {  // with mu held
-    if (buf) cudaFreeHost(buf);
-    for (cudaStream_t &q : st)
-      if (q) cudaStreamDestroy(q), q = nullptr;
-    buf = nullptr;
-    dev = -1;
-  }
-  bool ready(int device) {  // with mu held
-    if (buf) return dev == device;
-    if (cudaHostAlloc((void **)&buf, COPY_THREADS * COPY_CHUNK, cudaHostAllocDefault) !=
-        cudaSuccess)
-      buf = nullptr;
-    for (cudaStream_t &q : st)
-      if (buf && cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess) {
-        q = nullptr;
-        release();
-      }
-    cudaGetLastError();
-    dev = buf ? device : -1;
-    return buf != nullptr;
-  }
-} g_stage;
-
-static void stage_user(int n) {
-  std::lock_guard<std::mutex> lock(g_stage.mu);
-  g_stage.users += n;
-  if (g_stage.users == 0) g_stage.release();
-}
-
 static int field_copy(nspt_ctx *ctx, void *host, void *dev, size_t bytes, bool to_host) {
   CK(cudaStreamSynchronize(ctx->st));
-  cudaPointerAttributes at;
-  const bool pinned = cudaPointerGetAttributes(&at, host) == cudaSuccess &&
-                      at.type != cudaMemoryTypeUnregistered;
-  cudaGetLastError();
-  std::unique_lock<std::mutex> lock(g_stage.mu, std::defer_lock);
-  if (!pinned && bytes >= COPY_LEAST && lock.try_lock() && g_stage.ready(ctx->dev)) {
-    cudaError_t err[COPY_THREADS] = {};
-    auto part = [&](int t) {
-      const size_t chunks = (bytes + COPY_CHUNK - 1) / COPY_CHUNK;
-      char *pin = g_stage.buf + t * COPY_CHUNK;
-      cudaStream_t st = g_stage.st[t];
-      err[t] = cudaSetDevice(ctx->dev);
-      for (size_t c = t * chunks / COPY_THREADS;
-           c < (t + 1) * chunks / COPY_THREADS && err[t] == cudaSuccess; c++) {
-        const size_t at = c * COPY_CHUNK, n = std::min(COPY_CHUNK, bytes - at);
-        char *h = (char *)host + at, *d = (char *)dev + at;
-        if (!to_host) memcpy(pin, h, n);
-        err[t] = to_host ? cudaMemcpyAsync(pin, d, n, cudaMemcpyDeviceToHost, st)
-                         : cudaMemcpyAsync(d, pin, n, cudaMemcpyHostToDevice, st);
-        if (err[t] == cudaSuccess) err[t] = cudaStreamSynchronize(st);
-        if (err[t] == cudaSuccess && to_host) memcpy(h, pin, n);
-      }
-    };
-    std::thread th[COPY_THREADS];
-    int n = 1;
-    try {
-      for (; n < COPY_THREADS; n++) th[n] = std::thread(part, n);
-    } catch (...) {  // no more threads: this one does the rest
-    }
-    part(0);
-    for (int t = n; t < COPY_THREADS; t++) part(t);
-    for (int t = 1; t < n; t++) th[t].join();
-    for (cudaError_t e : err) CK(e);
-    return NSPT_OK;
-  }
-  CK(cudaMemcpyAsync(to_host ? host : dev, to_host ? dev : host, bytes,
-                     to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
+  CK(g_stage.copy(ctx->st, ctx->dev, host, dev, bytes, to_host));
   return NSPT_OK;
 }
 
