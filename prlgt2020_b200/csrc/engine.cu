@@ -1058,20 +1058,27 @@ static int field_copy(nspt_ctx *ctx, void *host, void *dev, size_t bytes, bool t
   return NSPT_OK;
 }
 
+// What an upload leaves to find out: whether every link's flag is 1
+static int read_flags(nspt_ctx *ctx) {
+  int *other = (int *)ctx->meas, h = 0;
+  CK(cudaMemsetAsync(other, 0, sizeof(int), ctx->st));
+  k_other_flags<<<ctx->nsm * 8, 256, 0, ctx->st>>>(ctx->U, (size_t)4 * ctx->V, ctx->N, other);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(&h, other, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  set_unit_flags(ctx, h == 0);
+  return NSPT_OK;
+}
+
 extern "C" int nspt_upload_links(nspt_ctx *ctx, const void *aos, int A) {
   if (!ctx || !aos || A < ctx->N) return NSPT_ERR_ARG;
   ctx->lg_current = false;
   ctx->snap_valid = false;  // a new field: no stale twisted reads
-  const size_t rec = 1 + 9 * (size_t)A, per_site = 4 * rec * sizeof(double2);
-  {
-    const double *f = (const double *)aos;
-    bool unit = true;
-    for (size_t l = 0; l < (size_t)4 * ctx->V && unit; l++)
-      unit = f[2 * rec * l] == 1.0 && f[2 * rec * l + 1] == 0.0;
-    set_unit_flags(ctx, unit);
+  const size_t per_site = 4 * (1 + 9 * (size_t)A) * sizeof(double2);
+  if (A == ctx->N) {  // the device layout
+    const int rc = field_copy(ctx, const_cast<void *>(aos), ctx->U, per_site * ctx->V, false);
+    return rc ? rc : read_flags(ctx);
   }
-  if (A == ctx->N)  // the device layout
-    return field_copy(ctx, const_cast<void *>(aos), ctx->U, per_site * ctx->V, false);
   const int cs = (int)std::max<size_t>(1, std::min<size_t>(kChunkBytes / per_site, ctx->V));
   double2 *buf = nullptr;
   CK(dev_alloc((void **)&buf, per_site * cs, ctx->dev));
@@ -1092,7 +1099,7 @@ extern "C" int nspt_upload_links(nspt_ctx *ctx, const void *aos, int A) {
   }
   cudaStreamSynchronize(ctx->st);
   cudaFree(buf);
-  return rc;
+  return rc ? rc : read_flags(ctx);
 }
 
 extern "C" int nspt_download_links(nspt_ctx *ctx, void *aos, int A) {

@@ -1509,6 +1509,17 @@ __global__ void k_pack(double2 *__restrict__ aos, int A, int s0, int cs, const d
   }
 }
 
+// *other = 1 where a link's flag is not 1
+__global__ void k_other_flags(const double2 *__restrict__ U, size_t nlinks, int N, int *other) {
+  bool any = false;
+  for (size_t l = blockIdx.x * (size_t)blockDim.x + threadIdx.x; l < nlinks;
+       l += (size_t)gridDim.x * blockDim.x) {
+    const double2 f = U[l * link_rec(N)];
+    any |= !(f.x == 1.0 && f.y == 0.0);
+  }
+  if (any) *other = 1;
+}
+
 __global__ void k_cold(double2 *U, size_t nlinks, int N) {
   const size_t rec = link_rec(N), tot = nlinks * rec;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot;
