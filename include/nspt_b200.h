@@ -153,13 +153,15 @@ int nspt_twist_boundary(nspt_ctx *ctx);
  * NSPT_UPDATE_ONTHEFLY, whose rectangles reach two sites), else
  * NSPT_ERR_ARG. */
 int nspt_set_gf_grid(nspt_ctx *ctx, const int grid[4]);
-/* Which form of the kernels runs the work ordered by the thread grid -- the
- * local gauge fixing and the on-the-fly sweep; both visit the sites in the
- * grid's order and give the same links to rounding.  NSPT_LGF_GROUP: 9 lanes
- * per reference thread (orders below 18; above, as TEAM).  NSPT_LGF_TEAM: a
- * CTA per thread in the gauge fixing, a warp in the on-the-fly sweep: shorter
- * latency for grids with few threads.  NSPT_LGF_AUTO (the default): by the number of
- * threads and the order.  Anything else: NSPT_ERR_ARG. */
+/* Which kernels run the local gauge fixing ordered by the thread grid; both forms
+ * visit the sites in the grid's order and give the same links.  NSPT_LGF_GROUP: one
+ * group of lanes per reference thread.  NSPT_LGF_TEAM: a CTA per reference thread
+ * (shorter latency for grids with few threads), where a barrier step's teams take
+ * two waves on the GPU at most, else groups.  NSPT_LGF_AUTO (the default): as TEAM.
+ * In the on-the-fly sweep the form has an effect only above 14 orders with zero
+ * modes or Fourier-accelerated gauge fixing: there GROUP adds up a link's staples
+ * one by one and TEAM by planes, on grids with one site per thread and barrier
+ * step; AUTO by planes where there are few threads.  Anything else: NSPT_ERR_ARG. */
 #define NSPT_LGF_AUTO 0
 #define NSPT_LGF_GROUP 1
 #define NSPT_LGF_TEAM 2

@@ -286,10 +286,11 @@ class NsptEngine:
         self._check(load_library().nspt_set_gf_grid(self._h, g), "nspt_set_gf_grid")
 
     def set_local_gf_form(self, form: str):
-        """Form of the kernels that follow the thread grid: "group" (9 lanes
-        per reference thread), "team" (a CTA per thread in the gauge
-        fixing, a warp in the on-the-fly sweep) or "auto" (by the number of
-        threads and the order).  Both give the same links to rounding."""
+        """Kernels of the local gauge fixing: "group" (one group of lanes per
+        reference thread), "team" (a CTA per reference thread where a barrier
+        step has few of them) or "auto" (as "team").  All give the same links.
+        An on-the-fly sweep with logarithms above 14 orders adds up a link's
+        staples one by one with "group" and by planes with "team"."""
         code = {"auto": 0, "group": 1, "team": 2}.get(form)
         if code is None:
             raise ValueError(f"local gauge fixing form {form!r}: auto, group or team")

@@ -210,18 +210,6 @@ static void with_form(const nspt_ctx *ctx, long units, Fn fn) {
   else
     measure_form(ctx, units, fn);
 }
-// The kernels that follow the thread grid: as set by nspt_set_local_gf_form
-// (9 lanes serve orders below 18, see ser_exp).
-template <class Fn>
-static void with_grid_form(const nspt_ctx *ctx, long units, Fn fn) {
-  if (ordered(ctx) || ctx->gf_form == NSPT_LGF_AUTO)
-    with_form(ctx, units, fn);
-  else if (ctx->gf_form == NSPT_LGF_GROUP && ctx->N < 9 * EXP_LANE)
-    fn(std::integral_constant<int, 9>());
-  else
-    fn(std::integral_constant<int, 32>());
-}
-
 // Groups per CTA: as many as give an SM the most groups, with 228 KB of shared
 // memory per SM, 1 KB of it taken by each CTA, at most ctas_max CTAs per SM
 // (registers) of CTA_WARPS warps of 32 / lanes groups; among equals the
@@ -379,7 +367,7 @@ static int launch_sweep_otf(nspt_ctx *ctx, const SweepArgs &a) {
                        r, ctx->F);
         });
         if (rc) break;
-        with_grid_form(ctx, gr.nthr, [&](auto G) {
+        with_form(ctx, gr.nthr, [&](auto G) {
           rc = wlaunch(ctx, G, k_otf_links<G.value>,
                        wide ? OTF_LINK_SLOTS_WIDE : OTF_LINK_SLOTS, gr.nthr,
                        "on-the-fly sweep, links", a, gr, p, r, (const double2 *)ctx->F, wide);
@@ -388,7 +376,7 @@ static int launch_sweep_otf(nspt_ctx *ctx, const SweepArgs &a) {
     return rc;
   }
   const bool planes = otf_by_planes(ctx, gr);
-  with_grid_form(ctx, gr.nthr, [&](auto G) {
+  with_form(ctx, gr.nthr, [&](auto G) {
     for (long p = 0; p < steps && !rc; p++)
       rc = ctx->c1 != 0.0 ? wlaunch(ctx, G, k_sweep_imp_otf<G.value>, IMP_SLOTS, gr.nthr,
                                     "on-the-fly sweep", a, gr, p)
@@ -730,12 +718,13 @@ static int do_fa(nspt_ctx *ctx, double alpha) {
 // 0.505 and 0.53, 8^4 (256) 0.30 and 0.52, 6*8*8*9 N=11 (48 threads, 9 sites
 // each) 1.28 and 3.18.  So teams serve up to two waves of the CTAs that fit, and
 // the ORDERED form, with one team on an SM, one: 6*8*8*9 N=15 4.7 and 7.5 ms,
-// but 8^4 N=16 2.5 and 2.1.
+// but 8^4 N=16 2.5 and 2.1.  NSPT_LGF_TEAM asks for no more of them: 16^4 N=4 (4096
+// threads) takes 2.7 ms with teams and 0.72 with groups.  Teams and groups have the
+// same lanes per link and form every sum alike: the links are the same bit for bit.
 template <int G>
 static bool team_fits(const nspt_ctx *ctx, long nthr, size_t &smem) {
   smem = (LEAD + (size_t)team_slots<G>() * group_stride(1, ctx->SS)) * sizeof(double2);
   if (ctx->gf_form == NSPT_LGF_GROUP || smem > ctx->smem_optin) return false;
-  if (ctx->gf_form == NSPT_LGF_TEAM) return true;
   const long fit = std::min<long>(G == ORDERED ? 1 : 2, (long)(228 * 1024 / (smem + 1024)));
   return nthr <= (G == ORDERED ? 1 : 2) * fit * ctx->nsm;
 }
@@ -771,7 +760,7 @@ static int do_local_gf(nspt_ctx *ctx, double alpha) {
   if (ordered(ctx) ? local_gf_team<ORDERED>(ctx, Ut, alpha, gr, steps, rc)
                    : local_gf_team<32>(ctx, Ut, alpha, gr, steps, rc))
     return rc;
-  with_grid_form(ctx, gr.nthr, [&](auto G) {
+  with_form(ctx, gr.nthr, [&](auto G) {
     for (long p = 0; p < steps && !rc; p++)
       rc = wlaunch(ctx, G, k_local_gf<G.value>, lgf_slots<G.value>(), gr.nthr, "local gauge fixing", ctx->U, Ut,
                    ctx->N, ctx->SS, ctx->geo, alpha, gr, p);
