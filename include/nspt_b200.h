@@ -273,14 +273,13 @@ int nspt_batch_step(nspt_batch *b, int nsteps, int gf_every);
 double nspt_batch_last_step_ms(const nspt_batch *b);
 /* Plaquette series of every replica's last sweep: plaq[nrep][(N+1)*2]. */
 int nspt_batch_observables(nspt_batch *b, double *plaq);
-/* Autotuner over the launch shape of the series kernels: warps per CTA (1 to
- * 4, or as many as shared memory holds; more run as 4).  Every candidate is
- * timed on the batch step itself and the fastest kept: *warps_out, *mo_out;
- * ms_table (may be NULL) gets [2][8] times, column w-1 for w warps, 0 where a
- * candidate does not exist.  The two rows (*mo_out 8, or 4 where N <= 12) are
- * two timings of the same kernels, which accumulate 8 orders per lane whatever
- * the row.  The trial steps are undone (every replica back to a cold start with
- * its seed).  Call before stepping. */
+/* Autotuner over the launch shape of the series kernels: warps per CTA, 1 to 4.
+ * Every candidate is timed on the batch step itself and the fastest kept:
+ * *warps_out; *mo_out is 8, the orders that the kernels accumulate per lane.
+ * ms_table (may be NULL) gets [2][8] times, column w-1 for w warps; more than 4 run
+ * as 4 and have its time, and so has row 1 (up to 12 orders and 6 warps, 0
+ * otherwise), which older kernels of 4 orders per lane had.  The trial steps are
+ * undone (every replica back to a cold start with its seed).  Call before stepping. */
 int nspt_batch_tune_shape(nspt_batch *b, int gf_every, int *warps_out, int *mo_out,
                           float *ms_table);
 /* nspt_batch_tune_shape reporting the warps only. */

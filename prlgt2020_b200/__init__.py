@@ -429,9 +429,9 @@ class NsptBatch:
         return w.value
 
     def tune_shape(self, gf_every: int = 1):
-        """Autotune the launch shape: (warps per CTA, 8 or 4, table of step
-        times in ms [rows 8 / 4][warps 1..8], 0 = not tried); the rows are two
-        timings of the same kernels."""
+        """Autotune the launch shape: (warps per CTA, 8, table of step times in
+        ms [2][warps 1..8]; more than 4 warps, and row 1, repeat the times of what
+        runs there, 0 = not shown)."""
         w, mo = ctypes.c_int(), ctypes.c_int()
         table = (ctypes.c_float * 16)()
         check(load_library().nspt_batch_tune_shape(self._h, int(gf_every), ctypes.byref(w),

@@ -224,47 +224,38 @@ extern "C" int nspt_batch_observables(nspt_batch *b, double *plaq) {
   return NSPT_OK;
 }
 
-// Autotuner over the launch shape of the series kernels: orders a lane
-// accumulates per pass (MO: the block chosen by N, or MO_LOW where N <= 3
-// MO_LOW) and warps per CTA (one link per warp).  Every candidate is
-// captured and timed on the batch itself; the fastest is kept.  The trial
-// steps change the fields, so every replica is put back to a cold start
-// with its seed (counter 0) afterwards.  ms_table (may be NULL) receives
-// [2][8] times: row 0 the MO shape, row 1 MO_LOW, column w-1 for w warps,
-// 0 where the candidate does not exist.
+// Autotuner over the launch shape of the series kernels: warps per CTA, 1 to
+// CTA_WARPS (more run as CTA_WARPS).  Every candidate is captured and timed on the
+// batch itself; the fastest is kept.  The trial steps change the fields, so every
+// replica is put back to a cold start with its seed (counter 0) afterwards.
+// ms_table (may be NULL) receives [2][8] times, column w - 1 for w warps; row 1, and
+// columns past CTA_WARPS, repeat the time of the shape that runs there.
 extern "C" int nspt_batch_tune_shape(nspt_batch *b, int gf_every, int *warps_out, int *mo_out,
                                      float *ms_table) {
   if (!b) return NSPT_ERR_ARG;
   const int P = graph_length(gf_every);
-  if (ms_table)
-    for (int i = 0; i < 16; i++) ms_table[i] = 0.f;
-  float best = 0.f;
-  int best_w = 0, best_mo = 0;
-  for (int row = 0; row < 2; row++) {
-    const int mo = row == 0 ? MO : MO_LOW;
-    if (mo == MO_LOW && b->N > 3 * MO_LOW) continue;
-    const int wmax = mo == MO ? 8 : 6;
-    for (int w = 1; w <= wmax; w++) {
-      for (nspt_ctx *c : b->ctx) {
-        c->sweep_warps = w;
-        c->shape_mo = mo;
-        c->launch_gen++;
-      }
-      drop_graph(b);
-      int rc = nspt_batch_step(b, P, gf_every);  // capture + warm-up
-      if (!rc) rc = nspt_batch_step(b, 2 * P, gf_every);
-      if (rc) return rc;
-      if (ms_table) ms_table[row * 8 + (w - 1)] = b->last_ms;
-      if (!best_w || b->last_ms < best) {
-        best = b->last_ms;
-        best_w = w;
-        best_mo = mo;
-      }
+  float ms[CTA_WARPS];
+  int best_w = 1;
+  for (int w = 1; w <= CTA_WARPS; w++) {
+    for (nspt_ctx *c : b->ctx) {
+      c->sweep_warps = w;
+      c->launch_gen++;
     }
+    drop_graph(b);
+    int rc = nspt_batch_step(b, P, gf_every);  // capture + warm-up
+    if (!rc) rc = nspt_batch_step(b, 2 * P, gf_every);
+    if (rc) return rc;
+    ms[w - 1] = b->last_ms;
+    if (ms[w - 1] < ms[best_w - 1]) best_w = w;
   }
+  if (ms_table)
+    for (int i = 0; i < 16; i++) {
+      // row 1: up to 12 orders and 6 warps
+      const bool shown = i < 8 || (b->N <= 12 && i < 14);
+      ms_table[i] = shown ? ms[std::min(i % 8, CTA_WARPS - 1)] : 0.f;
+    }
   for (int r = 0; r < b->nrep; r++) {
     b->ctx[r]->sweep_warps = best_w;
-    b->ctx[r]->shape_mo = best_mo;
     b->ctx[r]->launch_gen++;
     int rc = nspt_cold_start(b->ctx[r]);
     if (!rc) rc = nspt_seed(b->ctx[r], b->seed[r], 0);
@@ -274,7 +265,7 @@ extern "C" int nspt_batch_tune_shape(nspt_batch *b, int gf_every, int *warps_out
   drop_graph(b);
   b->warps = best_w;
   if (warps_out) *warps_out = best_w;
-  if (mo_out) *mo_out = best_mo;
+  if (mo_out) *mo_out = BLK;
   return NSPT_OK;
 }
 

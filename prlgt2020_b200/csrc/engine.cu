@@ -71,8 +71,7 @@ struct nspt_ctx {
   int gf_grid[4]; // local gauge fixing: the reference's thread grid (ntt, ntx, nty, ntz)
   int gf_form;    // form of the grid-ordered kernels: NSPT_LGF_AUTO, _GROUP or _TEAM
   unsigned long long *dcounter;  // Philox step counter on the device (advanced by k_inc)
-  int sweep_warps;               // warps per CTA of the sweep, 0 = as many as fit
-  int shape_mo;                  // the tuner's row: see nspt_batch_tune_shape
+  int sweep_warps;               // warps per CTA at most, 0 = as many as fit (nspt_batch_tune_shape)
   double c1;                     // improved action weight (0: Wilson), c0 = 1 - 8 c1
   double *obs_tr2;               // rectangle traces (improved actions)
   int *ff_e;                     // float-float scale exponent used by the sweep (device)
@@ -176,8 +175,6 @@ constexpr int MEASURE_CTAS = 592;
 // the 2368 warps that the GPU holds
 constexpr long SLAB_SITES = 4096;
 
-constexpr int MO = 8, MO_LOW = 4;
-
 // Lanes of a link's group (wseries.cuh) in a launch of `units` groups: 9 where
 // the SMs then have enough warps, 32 where they have not -- because shared
 // memory holds few links (sweep of 16 x 16 x 16 x 8, ms with 9 / 32 lanes: 2.2 /
@@ -194,8 +191,8 @@ static int form_lanes(const nspt_ctx *ctx, long units) {
 static bool ordered(const nspt_ctx *ctx) {
   return ctx->N > 14 && (ctx->flags & (NSPT_ZEROMODE | NSPT_GF_FA));
 }
-// Run fn with the form as a constant: for what enters the field, and for
-// measurements, which have no order to keep.
+// Run fn with the form as a constant: for what enters the field, and (measure_form)
+// for what has no order to keep.
 template <class Fn>
 static void measure_form(const nspt_ctx *ctx, long units, Fn fn) {
   if (form_lanes(ctx, units) == 9)
@@ -362,12 +359,12 @@ static int launch_sweep_otf(nspt_ctx *ctx, const SweepArgs &a) {
                       ctx->nsm * 200L * 1024;
     for (long p = 0; p < steps; p++)
       for (long r = 0; r < gr.seg && !rc; r++) {
-        with_form(ctx, parts, [&](auto G) {
+        measure_form(ctx, parts, [&](auto G) {
           rc = wlaunch(ctx, G, k_otf_parts<G.value>, 3, parts, "on-the-fly sweep, staples", a, gr, p,
                        r, ctx->F);
         });
         if (rc) break;
-        with_form(ctx, gr.nthr, [&](auto G) {
+        measure_form(ctx, gr.nthr, [&](auto G) {
           rc = wlaunch(ctx, G, k_otf_links<G.value>,
                        wide ? OTF_LINK_SLOTS_WIDE : OTF_LINK_SLOTS, gr.nthr,
                        "on-the-fly sweep, links", a, gr, p, r, (const double2 *)ctx->F, wide);
@@ -889,7 +886,6 @@ extern "C" int nspt_create(const int L[4], int N, unsigned flags, double alpha, 
   ctx->ftw = nullptr;
   ctx->dcounter = nullptr;
   ctx->sweep_warps = 0;
-  ctx->shape_mo = 0;
   ctx->lg_current = false;
   ctx->snap_valid = false;
   ctx->launch_gen = 0;

@@ -276,7 +276,6 @@ __device__ __noinline__ void ser_mul_any(int out, int A, int Bs, int N, unsigned
             n -= U;
             i += U;
           };
-#pragma unroll 1
           // by twos: a longer body has fewer moves of the window, but the SM's
           // instruction cache pays for it.  12^4 N=12 sweep 2.09 ms by twos, 2.25 by
           // fours, 2.09 by ones; 16*16*16*8 N=24 8.39, 8.45 and 8.69
