@@ -11,7 +11,7 @@
 enum cudaError_t { cudaSuccess, cudaErrorInvalidValue, cudaErrorMemoryAllocation };
 enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
 enum { cudaMemoryTypeUnregistered, cudaMemoryTypeHost };
-enum { cudaEventDisableTiming = 2, cudaHostAllocPortable = 1 };
+enum { cudaEventDisableTiming = 2, cudaHostRegisterPortable = 1 };
 struct cudaPointerAttributes {
   int type;
 };
@@ -23,7 +23,7 @@ typedef int *cudaEvent_t;
 
 struct Fake {
   static inline thread_local int device = 0;
-  static inline std::atomic<int> copies{0}, wrong_device{0}, allocs{0}, frees{0}, events{0};
+  static inline std::atomic<int> copies{0}, wrong_device{0}, allocs{0}, events{0};
   static inline std::atomic<int> fail_copy{-1};  // this copy fails
   static inline std::atomic<bool> fail_alloc{false};
   static inline std::atomic<size_t> pinned_bytes{0};
@@ -40,25 +40,22 @@ inline cudaError_t cudaSetDevice(int d) {
   Fake::device = d;
   return cudaSuccess;
 }
-inline cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
+inline cudaError_t cudaHostRegister(void *p, size_t n, unsigned) {
   if (Fake::fail_alloc) return cudaErrorMemoryAllocation;
-  *p = malloc(n);
   std::lock_guard<std::mutex> lock(Fake::mu);
-  Fake::pinned.insert({(char *)*p, (char *)*p + n});
+  Fake::pinned.insert({(char *)p, (char *)p + n});
   Fake::allocs++;
   Fake::pinned_bytes = n;
   return cudaSuccess;
 }
-inline cudaError_t cudaFreeHost(void *p) {
+inline cudaError_t cudaHostUnregister(void *p) {
   std::lock_guard<std::mutex> lock(Fake::mu);
   for (auto it = Fake::pinned.begin(); it != Fake::pinned.end(); ++it)
     if (it->first == p) {
       Fake::pinned.erase(it);
-      break;
+      return cudaSuccess;
     }
-  free(p);
-  Fake::frees++;
-  return cudaSuccess;
+  return cudaErrorInvalidValue;
 }
 inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
   std::lock_guard<std::mutex> lock(Fake::mu);

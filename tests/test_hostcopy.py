@@ -1,7 +1,7 @@
 """Large copies between pageable host fields and the device (csrc/hostcopy.cuh) on
 the CPU, against a fake of the CUDA runtime calls that it makes: whole at every
 size, the caller's current device left alone, several threads and devices at
-once, errors returned, the pinned set small beside the copy and given back."""
+once, errors returned, the pinned set made when it pays and given back."""
 import os
 import subprocess
 
