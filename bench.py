@@ -132,18 +132,33 @@ def read_profile_value(key: str, path: str = "profiles/sweep_32x4_n24_traffic.tx
 
 
 def read_profile_traffic():
-    """DRAM bytes (read + write) of one 32^4 x 24 sweep, from the committed ncu
-    summary (a 16*16*16*8 capture scaled by the link count)."""
+    """DRAM bytes (read + write) of one 32^4 x 24 sweep, estimated from the
+    committed ncu summary (a 16*16*16*8 capture scaled by the link count: its slabs
+    are 256 MB, those of 32^4 2 GB, and less of them stays in L2)."""
     return read_profile_value("traffic_bytes_per_sweep")
 
 
 def sweep_launches(L):
     """Kernel launches of one Jacobi Wilson sweep: k_plaq and k_update per slab
-    of direction 0 (at least 4096 sites), the last plane's plaquettes ahead when
-    there are several, four k_colsum, k_inc (the Philox step counter)."""
+    of direction 0 (at least 4096 sites; the whole lattice where that is two slabs
+    or fewer), the last plane's plaquettes ahead when there are several, four
+    k_colsum, k_inc (the Philox step counter)."""
     plane = L[1] * L[2] * L[3]
     slab = min(L[0], -(-4096 // plane))
+    if 2 * slab >= L[0]:
+        slab = L[0]
     return 2 * -(-L[0] // slab) + (slab < L[0]) + 5
+
+
+def onthefly_launches(L):
+    """Kernel launches of one twisted on-the-fly sweep: a k_sweep_otf per barrier
+    step of the default thread grid (blocks of 2 along even extents, odd ones not
+    split; a step walks what lies behind the last split direction), and the sums."""
+    split = [d for d in range(4) if L[d] % 2 == 0]
+    steps = 1
+    for d in range(split[-1] + 1 if split else 0):
+        steps *= 2 if d in split else L[d]
+    return steps + 5
 
 
 def executed_fraction(N: int, V: int, kernel_ms: float, peak: float):
@@ -398,7 +413,8 @@ def run_ours(args, world, rank, local):
                          "frac": achieved / peak, "traffic": read_profile_traffic(),
                          "traffic_source": "profiles/sweep_32x4_n24_traffic.txt: ncu dram__bytes_read.sum "
                                            "+ dram__bytes_write.sum of one sweep at 16*16*16*8 x 24, "
-                                           "scaled x32 (links) to 32^4; not measured in this run",
+                                           "scaled x32 (links) to 32^4: an estimate, not measured at "
+                                           "32^4 nor in this run",
                          "kernel": "k_plaq + k_update", "kernel_ms": kernel_ms,
                          "peak_source": "FP64 FMA microbenchmark on this GPU "
                                         "(nspt_measure_fp64_peak); MEASURED_PEAKS.json has no FP64 entry",
@@ -410,7 +426,7 @@ def run_ours(args, world, rank, local):
             "e2e": e2e,
             "with_gf": with_gf,
             "gpu_launches": sweep_launches(L) * args.steps if args.update == "jacobi" else
-                            (16 + 5) * args.steps,  # a k_sweep_otf per barrier step
+                            onthefly_launches(L) * args.steps,
             "cpu_baseline": cpu,
         }
         print(json.dumps(line), flush=True)

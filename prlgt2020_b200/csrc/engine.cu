@@ -180,7 +180,9 @@ constexpr long SLAB_SITES = 4096;
 // memory holds few links (sweep of 16 x 16 x 16 x 8, ms with 9 / 32 lanes: 2.2 /
 // 2.9 at 8 orders, 5.3 / 5.6 at 14, 6.7 / 6.1 at 16, 13.7 / 11.2 at 24) or
 // because the launch is small (1296 links of an on-the-fly step of 12^4 x 8: 5.1
-// / 4.0 ms per sweep; 1024 links of 4^4: 67 / 51 us).
+// / 4.0 ms per sweep; 1024 links of 4^4: 67 / 51 us).  Float-float products follow
+// the same line; their own would lie lower (12^4, ms with 9 / 32 lanes: 1.44 / 1.83
+// at 4 orders, 3.36 / 3.06 at 8, 8.99 / 6.73 at 12).
 static int form_lanes(const nspt_ctx *ctx, long units) {
   return ctx->N > 14 || units < 24L * ctx->nsm ? 32 : 9;
 }
@@ -1476,7 +1478,7 @@ extern "C" int nspt_plaquette_measure(nspt_ctx *ctx, double *plaq) {
   std::vector<double2> r(N + 1);
   CK(cudaMemcpyAsync(r.data(), tmp, r.size() * sizeof(double2), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
-  ctx->have_obs = false;  // the trace buffer now holds the static measurement
+  ctx->have_obs = false;  // the last sweep's observables are to be read before a measurement
   for (int k = 0; k <= N; k++) {  // nspt.cc:1398-1404
     plaq[2 * k] = r[k].x / (double)(ctx->V * 72);
     plaq[2 * k + 1] = r[k].y / (double)(ctx->V * 72);

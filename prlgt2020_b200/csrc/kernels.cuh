@@ -13,7 +13,8 @@
 //
 // Every link update is done by a group of 9 lanes, three to a warp, or by a warp, with a few
 // shared-memory series slots (wseries.cuh); a group's work is independent of all
-// others, no kernel of the step has a block barrier.
+// others.  Only the teams of the local gauge fixing, the transpose of the FFT's
+// input and the sums have block barriers.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -24,7 +24,7 @@
 //           orders) or the launch has no more.
 //
 //   G = ORDERED: as G = 9, but all three convolutions of an entry advance together,
-//           term by term in the order i, l (three windows, 240 registers).  The
+//           term by term in the order i, l (three windows, 200 to 255 registers).  The
 //           sums are then bit for bit those of a plain loop over i of 3x3
 //           products, which every field of a run with logarithms at high order
 //           has been made with: there rounding is amplified by some 3 per order
@@ -449,7 +449,7 @@ __constant__ double c_invfact[52] = {
 // and upper triangle (X^2 is hermitian) and N^2/4 steps of scalar work instead of the 1 + N/2 products of Horner in X^2, whose small sizes
 // cost a product's fixed part each.  The error against exact arithmetic is that
 // of the Horner form (both 1e-16 to 6e-16 per order, up to 40 orders).
-// Lanes own orders: up to EXP_LANE each, so G = 9 serves N < 18.
+// Lanes own orders: up to EXP_LANE each, so G = 9 serves N < 18 (it is used to 14).
 constexpr int EXP_LANE = 2;
 template <int G, bool DAG>
 __device__ __noinline__ void ser_exp(int X, int X2, int Z, int N) {
