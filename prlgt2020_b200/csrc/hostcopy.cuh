@@ -6,18 +6,18 @@
 // ms and now 21, down 190 and 50).  All copies go through the caller's stream, one
 // stream does as well as eight.
 //
-// The buffers are one set per process (16 MB), released with the last context.  They
-// lie on huge pages, which are pinned in 2 ms (10 ms on 4 KB pages), and are made
-// once COPY_PAYS bytes have been asked for since the last release: a program that
-// opens one engine after another takes no longer for its copies than the driver's
-// way (97 MB up 9 ms, down 21).  A copy that finds the set in use, or no memory for
-// it, goes the driver's way, as small ones and those in pinned memory do.
+// The buffers are one set per process (16 MB), released with the last context.  The
+// driver takes 10 ms to make them, as long as it takes for 100 MB up or 45 MB down by
+// itself, so they are made once COPY_PAYS bytes have been asked for since the last
+// release: a program that opens one engine after another waits no longer for its
+// copies than with the driver's.  (Huge pages of our own are pinned in 2 ms, but
+// downloads through them are slower: 97 MB 4.4 ms and not 3.4, 155 MB 6.6 and 5.9.)
+// A copy that finds the set in use, or no memory for it, goes the driver's way, as
+// small ones and those in pinned memory do.
 #pragma once
 #include <cuda_runtime.h>
-#include <sys/mman.h>
 
 #include <algorithm>
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -25,7 +25,7 @@
 namespace nspt {
 
 constexpr int COPY_THREADS = 8;
-constexpr size_t COPY_LEAST = 16u << 20, COPY_PAYS = 48u << 20;
+constexpr size_t COPY_LEAST = 16u << 20, COPY_PAYS = 128u << 20;
 // a thread's buffer: 97 MB up in 2.7 ms with 2 MB, 3.9 with 512 KB, 4.6 with 256 KB
 constexpr size_t COPY_CHUNK = 2u << 20;
 
@@ -121,10 +121,7 @@ class HostStage {
     return p;
   }
   void release() {  // with mu_ held
-    if (buf_) {
-      cudaHostUnregister(buf_);
-      free(buf_);
-    }
+    if (buf_) cudaFreeHost(buf_);
     buf_ = nullptr;
     asked_ = 0;
   }
@@ -132,13 +129,10 @@ class HostStage {
     if (buf_) return true;
     asked_ += std::min(bytes, COPY_PAYS);
     if (asked_ < COPY_PAYS) return false;
-    const size_t n = COPY_THREADS * COPY_CHUNK;
-    char *p = (char *)aligned_alloc(COPY_CHUNK, n);
-    if (!p) return false;
-    madvise(p, n, MADV_HUGEPAGE);
-    if (cudaHostRegister(p, n, cudaHostRegisterPortable) != cudaSuccess) {
+    char *p = nullptr;
+    if (cudaHostAlloc((void **)&p, COPY_THREADS * COPY_CHUNK, cudaHostAllocPortable) !=
+        cudaSuccess) {
       cudaGetLastError();
-      free(p);
       return false;
     }
     buf_ = p;

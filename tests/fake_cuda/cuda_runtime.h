@@ -11,7 +11,7 @@
 enum cudaError_t { cudaSuccess, cudaErrorInvalidValue, cudaErrorMemoryAllocation };
 enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
 enum { cudaMemoryTypeUnregistered, cudaMemoryTypeHost };
-enum { cudaEventDisableTiming = 2, cudaHostRegisterPortable = 1 };
+enum { cudaEventDisableTiming = 2, cudaHostAllocPortable = 1 };
 struct cudaPointerAttributes {
   int type;
 };
@@ -40,19 +40,21 @@ inline cudaError_t cudaSetDevice(int d) {
   Fake::device = d;
   return cudaSuccess;
 }
-inline cudaError_t cudaHostRegister(void *p, size_t n, unsigned) {
+inline cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
   if (Fake::fail_alloc) return cudaErrorMemoryAllocation;
+  *p = malloc(n);
   std::lock_guard<std::mutex> lock(Fake::mu);
-  Fake::pinned.insert({(char *)p, (char *)p + n});
+  Fake::pinned.insert({(char *)*p, (char *)*p + n});
   Fake::allocs++;
   Fake::pinned_bytes = n;
   return cudaSuccess;
 }
-inline cudaError_t cudaHostUnregister(void *p) {
+inline cudaError_t cudaFreeHost(void *p) {
   std::lock_guard<std::mutex> lock(Fake::mu);
   for (auto it = Fake::pinned.begin(); it != Fake::pinned.end(); ++it)
     if (it->first == p) {
       Fake::pinned.erase(it);
+      free(p);
       return cudaSuccess;
     }
   return cudaErrorInvalidValue;

@@ -26,6 +26,7 @@ int main() {
   {  // whole, both ways, at sizes around the chunks; the caller's device stays
     HostStage h;
     h.user(1);
+    size_t asked = 0;
     for (size_t n : {(size_t)1, COPY_LEAST - 1, COPY_LEAST, COPY_LEAST + 1,
                      (size_t)28713984, (size_t)70000001, (size_t)300000007}) {
       const auto a = pattern(n, 1);
@@ -37,8 +38,9 @@ int main() {
       HOLDS(Fake::device == 0);
       HOLDS(d == a && b == a);
       HOLDS(Fake::wrong_device == 0 && Fake::events == 0);
-      // one set, once 48 MB have been asked for
-      HOLDS(Fake::pinned.size() == (n > COPY_LEAST) && Fake::allocs == (n > COPY_LEAST));
+      // one set, once 128 MB have been asked for
+      if (n >= COPY_LEAST) asked += 2 * n;
+      HOLDS(Fake::pinned.size() == (asked >= COPY_PAYS) && Fake::allocs == (asked >= COPY_PAYS));
     }
     HOLDS(Fake::pinned_bytes == (16u << 20));
     // a smaller copy uses the set that is there
@@ -60,9 +62,9 @@ int main() {
     for (int rep = 0; rep < 2; rep++) {
       h.user(1);
       const int allocs = Fake::allocs;
-      for (int i = 0; i < 4; i++) {
+      for (int i = 0; i < 9; i++) {
         HOLDS(h.copy(&s0, 0, (void *)a.data(), d.data(), a.size(), false) == cudaSuccess);
-        HOLDS(Fake::allocs == allocs + (i >= 2) && d == a);
+        HOLDS(Fake::allocs == allocs + (i >= 7) && d == a);
       }
       h.user(-1);
     }
@@ -95,10 +97,10 @@ int main() {
   {  // an error of any copy comes back, and the next copy is whole
     HostStage h;
     h.user(1);
-    const size_t n = 80000003;
+    const size_t n = 140000003;
     const auto a = pattern(n, 5);
     std::vector<char> d(n);
-    for (int at : {0, 5, 38}) {
+    for (int at : {0, 5, 66}) {
       Fake::copies = 0;
       Fake::fail_copy = at;
       HOLDS(h.copy(&s0, 0, (void *)a.data(), d.data(), n, false) == cudaErrorInvalidValue);
@@ -111,7 +113,7 @@ int main() {
   {  // no pinned memory: the driver's way, in one copy; pinned fields always go that way
     HostStage h;
     h.user(1);
-    const size_t n = 80000003;
+    const size_t n = 140000003;
     const auto a = pattern(n, 6);
     std::vector<char> d(n);
     Fake::fail_alloc = true;
@@ -119,14 +121,13 @@ int main() {
     HOLDS(h.copy(&s1, 1, (void *)a.data(), d.data(), n, false) == cudaSuccess && d == a);
     HOLDS(Fake::copies == 1);
     Fake::fail_alloc = false;
-    void *p = malloc(n);
-    cudaHostRegister(p, n, 0);
+    void *p;
+    cudaHostAlloc(&p, n, 0);
     memcpy(p, a.data(), n);
     Fake::copies = 0;
     HOLDS(h.copy(&s1, 1, p, d.data(), n, false) == cudaSuccess && d == a);
     HOLDS(Fake::copies == 1 && Fake::wrong_device == 0);
-    cudaHostUnregister(p);
-    free(p);
+    cudaFreeHost(p);
     h.user(-1);
   }
   printf("ok\n");
