@@ -157,8 +157,9 @@ static bool release_records(int dev) {
   return any;
 }
 
-// Device memory that a context cannot do without
+// Device memory that a context on `dev` cannot do without, whatever device is current
 static cudaError_t dev_alloc(void **p, size_t n, int dev) {
+  const OnDevice current(dev);
   cudaError_t e = cudaMalloc(p, n);
   if (e == cudaErrorMemoryAllocation && release_records(dev)) {
     cudaGetLastError();
@@ -461,6 +462,7 @@ static bool by_plaquettes(const nspt_ctx *ctx) {
 // N=8 2.19 and 1.02, in float-float 9.5 and 3.4.
 static void take_records(nspt_ctx *ctx) {
   if (ctx->plaq_bytes || !by_plaquettes(ctx)) return;
+  const OnDevice current(ctx->dev);
   size_t room = 0, total = 0;
   if (cudaMemGetInfo(&room, &total) != cudaSuccess) {
     cudaGetLastError();
